@@ -18,10 +18,14 @@
 // outlet column of a tile share a warp and the Zou-He arithmetic is issued once
 // per tile, not once per row; a row of a group is at least a 32-byte sector.
 //
-// Measured on GB300 (1024 x 2048, porosity 0.7): 1.05 ms per iteration, the
-// FP64 pipe 84% busy with 369 instructions per 32 fluid cells, against 2.3 ms
-// for one thread per pair of cells in the reference's operand order (solid
-// lanes idle, twelve divisions and the products by 0 and 1 evaluated).
+// Measured on GB300 (1024 x 2048, porosity 0.7), per iteration: 2.3 ms with one
+// thread per pair of cells in the reference's operand order (solid lanes idle,
+// twelve divisions, the products by 0 and 1 evaluated); 1.05 ms with full warps
+// and the rewritings of fd_exact_cell.h (369 FP64 instructions per 32 fluid
+// cells, the pipe 84% busy, one issue slot in ten used); 0.87 ms with the
+// products in integer arithmetic (250 FP64 instructions).  Five CTAs an SM (96
+// registers, some spilled) beat four by 6% on 400 x 400: warps in flight hide
+// the pipe's latency.
 //
 // Cells whose values leave the range that exact_cell() takes (a diverging run),
 // and the body-force variant, are evaluated in the reference's operand order by
@@ -34,6 +38,9 @@
 namespace fd {
 
 constexpr int kExactTX = 32;
+#ifndef FD_EXACT_MINB
+#define FD_EXACT_MINB 5
+#endif
 
 struct ExactArgs {
   FusedArgs<double> a;
@@ -42,15 +49,16 @@ struct ExactArgs {
 };
 
 // Pulled populations of one cell: stream with wrap-around, then bounce-back links.
+__device__ __forceinline__ double exact_pull_one(const double* __restrict__ planes, size_t P, int H, int W, int x,
+                                                 int y, unsigned bits, int i) {
+  size_t src = (size_t)i * P + (size_t)wrap(y - ey_of(i), H) * W + wrap(x - ex_of(i), W);
+  if (i > 0 && ((bits >> (i - 1)) & 1u)) src = (size_t)opp_of(i) * P + (size_t)y * W + x;
+  return __ldg(planes + src);
+}
 __device__ __forceinline__ void exact_pull(const double* __restrict__ planes, size_t P, int H, int W, int x, int y,
                                            unsigned bits, double (&v)[9]) {
-  const size_t q = (size_t)y * W + x;
 #pragma unroll
-  for (int i = 0; i < 9; ++i) {
-    size_t src = (size_t)i * P + (size_t)wrap(y - ey_of(i), H) * W + wrap(x - ex_of(i), W);
-    if (i > 0 && ((bits >> (i - 1)) & 1u)) src = (size_t)opp_of(i) * P + q;
-    v[i] = __ldg(planes + src);
-  }
+  for (int i = 0; i < 9; ++i) v[i] = exact_pull_one(planes, P, H, W, x, y, bits, i);
 }
 
 __device__ __forceinline__ void exact_store(const FusedArgs<double>& a, size_t P, size_t q, const double (&f)[9],
@@ -100,10 +108,11 @@ __device__ __noinline__ void exact_slow_cell(const FusedArgs<double>& a, int x, 
 }
 
 template <int TY, int NT>
-__global__ void __launch_bounds__(NT) k_exact_step(const __grid_constant__ ExactArgs ea) {
+__global__ void __launch_bounds__(NT, FD_EXACT_MINB) k_exact_step(const __grid_constant__ ExactArgs ea) {
   constexpr int CW = 32 / TY, CHUNKS = kExactTX / CW, PW = kExactTX + 2;
   static_assert(TY * CW == 32 && CHUNKS * CW == kExactTX, "a group of 32 cells is CW columns of the tile");
   __shared__ double psi[(TY + 2) * PW];
+  __shared__ double edge_g[2][TY][9];  // g of the inlet and outlet column's cells after Zou-He
   __shared__ unsigned need[CHUNKS];
   __shared__ uint16_t list[CHUNKS * 32];
   const FusedArgs<double>& a = ea.a;
@@ -118,7 +127,8 @@ __global__ void __launch_bounds__(NT) k_exact_step(const __grid_constant__ Exact
 
   // 1. psi of the tile and its surroundings; which cells need arithmetic
   for (int e = t; e < (TY + 2) * PW; e += NT) {
-    int x = x0 + e % PW - 1, y = y0 + e / PW - 1;
+    const int px = e % PW - 1, py = e / PW - 1;
+    int x = x0 + px, y = y0 + py;
     if (x > a.W || y > a.H) continue;  // past the ghost cells of a tile that the lattice ends in
     double v;
     if (walls && (y < 0 || y >= a.H)) {
@@ -129,13 +139,20 @@ __global__ void __launch_bounds__(NT) k_exact_step(const __grid_constant__ Exact
       x = wrap(x, a.W);
       y = wrap(y, a.H);
       const unsigned m = a.mask[(size_t)y * a.W + x];
-      if (m & SOLID) {
+      const bool edge = !xy && (x == 0 || x == a.W - 1);
+      if ((m & SOLID) && !edge) {
         v = a.c.psi_wall;
       } else {
         double g[9];
         exact_pull(a.src + 9 * P, P, a.H, a.W, x, y, m & 0xFFu, g);
-        if (x == 0 || x == a.W - 1) zou_he_g(a.c, a.variant, a.H, a.W, x, y, g);
-        v = sum9(g);
+        if (edge) {
+          zou_he_g(a.c, a.variant, a.H, a.W, x, y, g);
+          if (py >= 0 && py < TY && px >= 0 && px < kExactTX) {
+#pragma unroll
+            for (int i = 0; i < 9; ++i) edge_g[x == 0 ? 0 : 1][py][i] = g[i];
+          }
+        }
+        v = (m & SOLID) ? a.c.psi_wall : sum9(g);
       }
     }
     psi[e] = v;
@@ -190,22 +207,26 @@ __global__ void __launch_bounds__(NT) k_exact_step(const __grid_constant__ Exact
       exact_slow_cell(a, x, y, m & 0xFFu, ps, PW);
       continue;
     }
-    double f[9], g[9];
-    exact_pull(a.src, P, a.H, a.W, x, y, m & 0xFFu, f);
-    exact_pull(a.src + 9 * P, P, a.H, a.W, x, y, m & 0xFFu, g);
-    if (x == 0 || x == a.W - 1) {
-      zou_he_g(a.c, a.variant, a.H, a.W, x, y, g);
-      exact_boundary(a, P, x, y, ps, PW, f);
+    const unsigned bits = m & 0xFFu;
+    double f[9];
+    exact_pull(a.src, P, a.H, a.W, x, y, bits, f);
+    const bool edge = x == 0 || x == a.W - 1;
+    if (edge) exact_boundary(a, P, x, y, ps, PW, f);
+    auto load_g = [&](int i) {
+      return edge ? edge_g[x == 0 ? 0 : 1][ly][i] : exact_pull_one(a.src + 9 * P, P, a.H, a.W, x, y, bits, i);
+    };
+    auto store = [&](int i, double fn, double gn) {
+      a.dst[(size_t)i * P + q] = fn;
+      a.dst[(size_t)(9 + i) * P + q] = gn;
+    };
+    if (m & SOLID) {  // of the inlet or outlet column
+#pragma unroll
+      for (int i = 0; i < 9; ++i) store(i, f[i], edge_g[x == 0 ? 0 : 1][ly][i]);
+      continue;
     }
-    if (!(m & SOLID)) {
-      const ExactStencil st = exact_stencil(ea.k, ps[0], ps[1], ps[-1], ps[PW], ps[-PW], ps[PW + 1], ps[PW - 1],
-                                            ps[1 - PW], ps[-1 - PW]);
-      if (!exact_cell(ea.k, ps[0], st, f, g)) {
-        exact_slow_cell(a, x, y, m & 0xFFu, ps, PW);
-        continue;
-      }
-    }
-    exact_store(a, P, q, f, g);
+    const ExactStencil st = exact_stencil(ea.k, ps[0], ps[1], ps[-1], ps[PW], ps[-PW], ps[PW + 1], ps[PW - 1],
+                                          ps[1 - PW], ps[-1 - PW]);
+    if (!exact_cell(ea.k, ps[0], st, f, load_g, store)) exact_slow_cell(a, x, y, bits, ps, PW);
   }
 }
 

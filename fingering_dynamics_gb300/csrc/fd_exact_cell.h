@@ -1,7 +1,7 @@
 // One fluid cell of the FP64 step with fewer FP64 operations and the same
 // bits, plain C++ so that it can be checked without a GPU.
 //
-// The FP64 pipe of sm_103a retires two results per clock and SM (an FP32 one
+// The FP64 pipe of sm_103a retires two results per clock and SM (the FP32 one
 // 128), so the FP64 step's time is its count of FP64 operations.  Every
 // rewriting below returns exactly what the reference's operand order
 // (fd_physics.cuh) returns:
@@ -31,8 +31,10 @@
 
 #ifdef __CUDACC__
 #define FD_CELL __host__ __device__ __forceinline__
+#define FD_CELL_CALL static __host__ __device__ __noinline__
 #else
 #define FD_CELL inline
+#define FD_CELL_CALL inline
 #endif
 
 namespace fd {
@@ -78,7 +80,72 @@ FD_CELL bool cell_in_range(double v) {
 #endif
   const uint32_t h = (uint32_t)(b >> 32) & 0x7fffffffu, l = (uint32_t)b;
   constexpr uint32_t lo = (uint32_t)(1023 - E) << 20, hi = (uint32_t)(1023 + E) << 20;
-  return (h - lo) < (hi - lo) || (h | l) == 0u;
+  return ((h - lo) < (hi - lo)) | ((h | l) == 0u);
+}
+
+FD_CELL uint64_t cell_bits(double v) {
+#ifdef __CUDA_ARCH__
+  return (uint64_t)__double_as_longlong(v);
+#else
+  uint64_t b;
+  std::memcpy(&b, &v, 8);
+  return b;
+#endif
+}
+FD_CELL double cell_double(uint32_t hi, uint32_t lo) {
+#ifdef __CUDA_ARCH__
+  return __hiloint2double((int)hi, (int)lo);
+#else
+  const uint64_t b = ((uint64_t)hi << 32) | lo;
+  double v;
+  std::memcpy(&v, &b, 8);
+  return v;
+#endif
+}
+
+// a * b rounded to nearest even in integer arithmetic (the product of the two
+// 53-bit significands, its top 53 bits, the rest as the rounding bits).  A zero
+// operand gives a signed zero.  Operands and result must be zero or have
+// exponents within +-800: `ok` is cleared where the result has not (operands
+// are results that were checked before, or sums of them).
+FD_CELL double cell_mul_int(double a, double b, bool& ok) {
+  const uint64_t A = cell_bits(a), B = cell_bits(b);
+  const uint32_t ah = (uint32_t)(A >> 32), al = (uint32_t)A, bh = (uint32_t)(B >> 32), bl = (uint32_t)B;
+  const uint32_t Ah = ((ah << 11) | (al >> 21)) | 0x80000000u, Al = al << 11;
+  const uint32_t Bh = ((bh << 11) | (bl >> 21)) | 0x80000000u, Bl = bl << 11;
+  const uint64_t t = (uint64_t)Al * Bl;
+  const uint64_t u = (uint64_t)Al * Bh + (t >> 32);
+  const uint64_t v = (uint64_t)Ah * Bl + (uint32_t)u;
+  const uint64_t h = (uint64_t)Ah * Bh + (u >> 32) + (v >> 32);  // significands' product / 2^64: bit 63 or 62 is set
+  const uint32_t top = (uint32_t)(h >> 63), sh = 10u + top;
+  const uint32_t rem = ((uint32_t)h << (32u - sh)) | (((uint32_t)v | (uint32_t)t) != 0u ? 1u : 0u);
+  uint64_t m = h >> sh;
+  m += (rem + ((uint32_t)m & 1u)) > 0x80000000u ? 1u : 0u;
+  const uint32_t ea = ah & 0x7ff00000u, eb = bh & 0x7ff00000u;
+  // the exponent field, one less because the leading bit of m adds one
+  const uint32_t e = ea + eb + (top << 20) - (1024u << 20);
+  const bool zero = (ea == 0u) | (eb == 0u);
+  ok = ok & (zero | (e - (223u << 20) < (1600u << 20)));
+  const uint32_t sign = (ah ^ bh) & 0x80000000u;
+  return cell_double((zero ? 0u : (uint32_t)(m >> 32) + e) | sign, zero ? 0u : (uint32_t)m);
+}
+
+// N 2^X a rounded to nearest even in integer arithmetic (N = 3 or 9)
+template <int N, int X>
+FD_CELL double cell_scale_int(double a) {
+  constexpr uint32_t L = N == 3 ? 1 : 3;  // floor(log2 N)
+  static_assert(N == 3 || N == 9, "multipliers of the equilibria");
+  const uint64_t A = cell_bits(a);
+  const uint32_t ah = (uint32_t)(A >> 32);
+  const uint64_t p = ((A & 0xfffffffffffffull) | 0x10000000000000ull) * (uint64_t)N;
+  const uint32_t top = (uint32_t)(p >> (53 + L)), sh = L + top;
+  const uint32_t rem = (uint32_t)p << (32u - sh);
+  uint64_t m = p >> sh;
+  m += (rem + ((uint32_t)m & 1u)) > 0x80000000u ? 1u : 0u;
+  const uint32_t ea = ah & 0x7ff00000u;
+  const uint32_t hi = (uint32_t)(m >> 32) + ea + ((top + L - 1u + (uint32_t)X) << 20);
+  const bool zero = ea == 0u;
+  return cell_double((zero ? 0u : hi) | (ah & 0x80000000u), zero ? 0u : (uint32_t)m);
 }
 
 // a / b rounded to nearest for a constant b, y = 1 / b (see above)
@@ -117,75 +184,148 @@ FD_CELL ExactStencil exact_stencil(const ExactConst& k, double C, double E, doub
   return s;
 }
 
-// Macroscopic fields and collision of one fluid cell (fingering_periodic.py:
-// 455-460, 470-479) from its pulled populations f, g, its psi and psi's
-// derivatives.  On success f and g are the new populations; on failure (false)
-// they are untouched.
-FD_CELL bool exact_cell(const ExactConst& k, double psi, const ExactStencil& st, double (&f)[9], double (&g)[9]) {
-  double rho = f[0];
-#pragma unroll
-  for (int i = 1; i < 9; ++i) rho = rho + f[i];
+// How many of a cell's products are formed in integer arithmetic (0: none, 58:
+// all), in the order of their numbers below.  An integer product is about 40
+// instructions, which the four schedulers issue in 10 clocks beside the FP64
+// pipe, against the pipe's 16.  Ten iterations of 1024 x 2048: 11.6 ms with
+// none, 10.7 with those of cell_relax (7), 10.2 with all; 25 of 400 x 400:
+// 3.16, 2.96, 2.57 ms.
+#ifndef FD_EXACT_INT_PRODUCTS
+#define FD_EXACT_INT_PRODUCTS 58
+#endif
+
+template <int K>
+FD_CELL double cell_mul(double a, double b, bool& ok) {
+  if constexpr (K < FD_EXACT_INT_PRODUCTS) return cell_mul_int(a, b, ok);
+  else return a * b;
+}
+template <int K, int N, int X>
+FD_CELL double cell_scale(double a) {
+  if constexpr (K < FD_EXACT_INT_PRODUCTS) return cell_scale_int<N, X>(a);
+  else return (X < 0 ? 0.5 * N : (double)N) * a;
+}
+
+// New f (x) and g (y) of one direction: w (A + rho q), w (B + psi q) are the
+// equilibria, SF P S the forcing.  f is NaN where a value left the range.  A
+// function of its own on the GPU: nine copies of its integer products do not
+// fit the instruction cache.
+struct CellPair {
+  double x, y;
+};
+FD_CELL_CALL CellPair cell_relax(double w, double A, double B, double rho, double psi, double q, double SF, double P,
+                                 double S, double inv_t, double tau_inv, double f, double g) {
+  bool ok = cell_in_range<100>(g);
+  const double fe = cell_mul<0>(w, A + cell_mul<1>(rho, q, ok), ok);
+  const double ge = cell_mul<2>(w, B + cell_mul<3>(psi, q, ok), ok);
+  const double fn = cell_fma(SF, cell_mul<4>(P, S, ok), f - cell_mul<5>(inv_t, f - fe, ok));
+  return CellPair{ok ? fn : cell_double(0x7ff80000u, 0u), g - cell_mul<6>(tau_inv, g - ge, ok)};
+}
+
+// Macroscopic fields of one fluid cell (fingering_periodic.py:470-479) from its
+// density, pulled f, psi and psi's derivatives.
+struct ExactMacro {
+  double rho, ux, uy, p, mu, tau, psi, gx, gy;
+  bool ok;  // every value in range
+};
+
+FD_CELL ExactMacro exact_macros(const ExactConst& k, double rho, double psi, const ExactStencil& st,
+                                const double (&f)[9]) {
+  ExactMacro m;
   const double mx = ((((f[1] - f[3]) + f[5]) - f[6]) - f[7]) + f[8];
   const double my = ((((f[2] - f[4]) + f[5]) + f[6]) - f[7]) - f[8];
-  const double gx = st.gx, gy = st.gy;
-  const double mu = ((k.a * psi) * (1.0 - psi * psi)) - k.kappa * st.lap;
-  const double mgx = mu * gx, mgy = mu * gy;
+  bool ok = st.ok & cell_in_range<100>(rho) & (rho != 0.0) & cell_in_range<100>(psi);
+  const double mu = cell_mul<7>(k.a * psi, 1.0 - cell_mul<8>(psi, psi, ok), ok) - cell_mul<9>(k.kappa, st.lap, ok);
+  const double mgx = cell_mul<10>(mu, st.gx, ok), mgy = cell_mul<11>(mu, st.gy, ok);
   const double jx = cell_fma(0.5, mgx, mx), jy = cell_fma(0.5, mgy, my);
   const double y = cell_rcp(rho);
-  const double ux = cell_div_shared(jx, rho, y), uy = cell_div_shared(jy, rho, y);
-  const double p = k.one_third * rho + psi * mu;
+  m.ux = cell_div_shared(jx, rho, y);
+  m.uy = cell_div_shared(jy, rho, y);
+  m.p = cell_mul<12>(k.one_third, rho, ok) + cell_mul<13>(psi, mu, ok);
   const double v1 = cell_div_shared(k.eta_n, rho, y), v2 = cell_div_shared(k.eta_n_M, rho, y);
-  const double vv = v1 * v2;
-  const double mv = vv / ((v1 * (1.0 - psi)) + (v2 * (1.0 + psi)));  // half of the mixed viscosity
-  const double inv_t = cell_rcp(cell_fma(2.0, 3.0 * mv, 0.5));
-  const double pref = cell_fma(-0.5, inv_t, 1.0);                     // 1 - 1 / (2 tau)
-  const double na = rho - k.c_a0 * p, nb = psi - k.c_b0 * mu;
-  const bool ok = st.ok & cell_in_range<100>(rho) & (rho != 0.0) & cell_in_range<800>(jx) & cell_in_range<800>(jy) &
-                  cell_in_range<800>(k.eta_n) & cell_in_range<800>(k.eta_n_M) & cell_in_range<800>(vv) &
-                  cell_in_range<800>(mgx) & cell_in_range<800>(mgy) & cell_in_range<800>(mu) & cell_in_range<800>(na) &
-                  cell_in_range<800>(nb) & cell_in_range<100>(ux) & cell_in_range<100>(uy) & cell_in_range<100>(inv_t);
-  if (!ok) return false;
-  const double A0 = cell_div_const(na, k.w0, k.yw0), A = 3.0 * p;
-  const double B0 = cell_div_const(nb, k.w0, k.yw0), B = k.c_b18 * mu;
-  const double P = (mu * k.w1) * pref;  // forcing prefactor of w_1; 4 P and P / 4 are those of w_0 and w_5
-  const double xx = ux * ux, yy = uy * uy;
-  const double u15 = 1.5 * (xx + yy);
-  // relaxation of one direction: SF = w_1's multiple of the forcing weight
-#define FD_CELL_RELAX(I, WQ, AQ, BQ, Q, SF, S)                      \
-  {                                                                 \
-    const double q_ = (Q);                                          \
-    const double fe = (WQ) * ((AQ) + rho * q_);                     \
-    const double ge = (WQ) * ((BQ) + psi * q_);                     \
-    f[I] = cell_fma(SF, P * (S), f[I] - inv_t * (f[I] - fe));       \
-    g[I] = g[I] - k.tau_inv * (g[I] - ge);                          \
-  }
-  const double x3 = 3.0 * ux, y3 = 3.0 * uy;
-  const double wx = x3 * gx, wy = y3 * gy;
-  FD_CELL_RELAX(0, k.w0, A0, B0, -u15, 4.0, -(wx + wy));
-  const double xp = (1.0 - ux) * 3.0, xm = (-1.0 - ux) * 3.0, yp = (1.0 - uy) * 3.0, ym = (-1.0 - uy) * 3.0;
+  const double vv = cell_mul<14>(v1, v2, ok);
+  // half of the mixed viscosity
+  const double mv = vv / (cell_mul<15>(v1, 1.0 - psi, ok) + cell_mul<16>(v2, 1.0 + psi, ok));
+  m.tau = cell_fma(2.0, 3.0 * mv, 0.5);
+  m.rho = rho;
+  m.mu = mu;
+  m.psi = psi;
+  m.gx = st.gx;
+  m.gy = st.gy;
+  m.ok = ok & cell_in_range<800>(jx) & cell_in_range<800>(jy) & cell_in_range<800>(k.eta_n) &
+         cell_in_range<800>(k.eta_n_M) & cell_in_range<800>(vv) & cell_in_range<800>(mgx) & cell_in_range<800>(mgy);
+  return m;
+}
+
+// Collision of one fluid cell (fingering_periodic.py:455-460) from its
+// macroscopic fields and f; g_i comes from load_g(i) and the new populations go
+// to store(i, f, g).  False: what was stored must not be used, the caller
+// evaluates the cell otherwise.
+template <typename LoadG, typename Store>
+FD_CELL bool exact_collide(const ExactConst& k, const ExactMacro& m, const double (&f)[9], LoadG load_g, Store store) {
+  const double rho = m.rho, ux = m.ux, uy = m.uy, p = m.p, mu = m.mu, psi = m.psi, gx = m.gx, gy = m.gy;
+  bool ok = m.ok;
+  const double inv_t = cell_rcp(m.tau);
+  const double pref = cell_fma(-0.5, inv_t, 1.0);  // 1 - 1 / (2 tau)
+  const double na = rho - cell_mul<17>(k.c_a0, p, ok), nb = psi - cell_mul<18>(k.c_b0, mu, ok);
+  ok = ok & cell_in_range<800>(mu) & cell_in_range<800>(na) & cell_in_range<800>(nb) & cell_in_range<100>(ux) &
+       cell_in_range<100>(uy) & cell_in_range<100>(inv_t);
+  const double A0 = cell_div_const(na, k.w0, k.yw0), A = cell_scale<40, 3, 0>(p);
+  const double B0 = cell_div_const(nb, k.w0, k.yw0), B = cell_mul<19>(k.c_b18, mu, ok);
+  // forcing prefactor of w_1; 4 P and P / 4 are those of w_0 and w_5
+  const double P = cell_mul<20>(cell_mul<21>(mu, k.w1, ok), pref, ok);
+  const double xx = cell_mul<22>(ux, ux, ok), yy = cell_mul<23>(uy, uy, ok);
+  const double u15 = cell_scale<41, 3, -1>(xx + yy);
+  const double x3 = cell_scale<42, 3, 0>(ux), y3 = cell_scale<43, 3, 0>(uy);
+  const double wx = cell_mul<24>(x3, gx, ok), wy = cell_mul<25>(y3, gy, ok);
+  // one direction: weight, constant parts of its equilibria, q, scale of its forcing, S
+  auto relax = [&](int i, double w, double Aq, double Bq, double q, double SF, double S) {
+    const CellPair r = cell_relax(w, Aq, Bq, rho, psi, q, SF, P, S, inv_t, k.tau_inv, f[i], load_g(i));
+    ok &= ((uint32_t)(cell_bits(r.x) >> 32) & 0x7ff00000u) != 0x7ff00000u;
+    store(i, r.x, r.y);
+  };
+  relax(0, k.w0, A0, B0, -u15, 4.0, -(wx + wy));
+  const double xp = cell_scale<44, 3, 0>(1.0 - ux), xm = cell_scale<45, 3, 0>(-1.0 - ux);
+  const double yp = cell_scale<46, 3, 0>(1.0 - uy), ym = cell_scale<47, 3, 0>(-1.0 - uy);
   {
-    const double s = 4.5 * xx, n = 9.0 * ux;
-    FD_CELL_RELAX(1, k.w1, A, B, (x3 + s) - u15, 1.0, (xp + n) * gx - wy);
-    FD_CELL_RELAX(3, k.w1, A, B, (s - x3) - u15, 1.0, (xm + n) * gx - wy);
+    const double s = cell_scale<48, 9, -1>(xx), n = cell_scale<49, 9, 0>(ux);
+    const double S1 = cell_mul<26>(xp + n, gx, ok) - wy, S3 = cell_mul<27>(xm + n, gx, ok) - wy;
+    relax(1, k.w1, A, B, (x3 + s) - u15, 1.0, S1);
+    relax(3, k.w1, A, B, (s - x3) - u15, 1.0, S3);
   }
   {
-    const double s = 4.5 * yy, n = 9.0 * uy;
-    FD_CELL_RELAX(2, k.w1, A, B, (y3 + s) - u15, 1.0, (yp + n) * gy - wx);
-    FD_CELL_RELAX(4, k.w1, A, B, (s - y3) - u15, 1.0, (ym + n) * gy - wx);
+    const double s = cell_scale<50, 9, -1>(yy), n = cell_scale<51, 9, 0>(uy);
+    const double S2 = cell_mul<28>(yp + n, gy, ok) - wx, S4 = cell_mul<29>(ym + n, gy, ok) - wx;
+    relax(2, k.w1, A, B, (y3 + s) - u15, 1.0, S2);
+    relax(4, k.w1, A, B, (s - y3) - u15, 1.0, S4);
   }
   const double w5 = 0.25 * k.w1;
   {
-    const double e = ux + uy, t = 3.0 * e, s = 4.5 * (e * e), n = 9.0 * e;
-    FD_CELL_RELAX(5, w5, A, B, (t + s) - u15, 0.25, (xp + n) * gx + (yp + n) * gy);
-    FD_CELL_RELAX(7, w5, A, B, (s - t) - u15, 0.25, (xm + n) * gx + (ym + n) * gy);
+    const double e = ux + uy, t = cell_scale<52, 3, 0>(e), s = cell_scale<53, 9, -1>(cell_mul<30>(e, e, ok));
+    const double n = cell_scale<54, 9, 0>(e);
+    const double S5 = cell_mul<31>(xp + n, gx, ok) + cell_mul<32>(yp + n, gy, ok);
+    const double S7 = cell_mul<33>(xm + n, gx, ok) + cell_mul<34>(ym + n, gy, ok);
+    relax(5, w5, A, B, (t + s) - u15, 0.25, S5);
+    relax(7, w5, A, B, (s - t) - u15, 0.25, S7);
   }
   {
-    const double e = uy - ux, t = 3.0 * e, s = 4.5 * (e * e), n = 9.0 * e;
-    FD_CELL_RELAX(6, w5, A, B, (t + s) - u15, 0.25, (xm - n) * gx + (yp + n) * gy);
-    FD_CELL_RELAX(8, w5, A, B, (s - t) - u15, 0.25, (xp - n) * gx + (ym + n) * gy);
+    const double e = uy - ux, t = cell_scale<55, 3, 0>(e), s = cell_scale<56, 9, -1>(cell_mul<35>(e, e, ok));
+    const double n = cell_scale<57, 9, 0>(e);
+    const double S6 = cell_mul<36>(xm - n, gx, ok) + cell_mul<37>(yp + n, gy, ok);
+    const double S8 = cell_mul<38>(xp - n, gx, ok) + cell_mul<39>(ym + n, gy, ok);
+    relax(6, w5, A, B, (t + s) - u15, 0.25, S6);
+    relax(8, w5, A, B, (s - t) - u15, 0.25, S8);
   }
-#undef FD_CELL_RELAX
-  return true;
+  return ok;
+}
+
+// Both, for the fused step.
+template <typename LoadG, typename Store>
+FD_CELL bool exact_cell(const ExactConst& k, double psi, const ExactStencil& st, const double (&f)[9], LoadG load_g,
+                        Store store) {
+  double rho = f[0];
+#pragma unroll
+  for (int i = 1; i < 9; ++i) rho = rho + f[i];
+  return exact_collide(k, exact_macros(k, rho, psi, st, f), f, load_g, store);
 }
 
 }  // namespace fd

@@ -1,6 +1,6 @@
 """The FP64 step's cell arithmetic (csrc/fd_exact_cell.h), compiled for the
 host, against the oracle's operand order: every bit of the macroscopic fields'
-collision must agree, and values outside its range must be refused untouched."""
+collision must agree, and values outside its range must be refused."""
 import ctypes as C
 import os
 import shutil
@@ -18,25 +18,26 @@ using namespace fd;
 extern "C" void cells(const double* c, long n, const double* nb, double* f, double* g, unsigned char* ok) {
   const ExactConst k = make_exact_const(c[0], c[1], c[2], c[3], c[4], c[5], c[6], c[7], c[8], c[9], c[10]);
   for (long j = 0; j < n; ++j) {
-    double v[9], fc[9], gc[9];
-    for (int i = 0; i < 9; ++i) { v[i] = nb[i * n + j]; fc[i] = f[i * n + j]; gc[i] = g[i * n + j]; }
+    double v[9], fc[9], fo[9], go[9];
+    for (int i = 0; i < 9; ++i) { v[i] = nb[i * n + j]; fc[i] = f[i * n + j]; }
     const ExactStencil s = exact_stencil(k, v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8]);
-    ok[j] = exact_cell(k, v[0], s, fc, gc);
-    for (int i = 0; i < 9; ++i) { f[i * n + j] = fc[i]; g[i * n + j] = gc[i]; }
+    ok[j] = exact_cell(k, v[0], s, fc, [&](int i) { return g[i * n + j]; },
+                       [&](int i, double a, double b) { fo[i] = a; go[i] = b; });
+    if (ok[j]) for (int i = 0; i < 9; ++i) { f[i * n + j] = fo[i]; g[i * n + j] = go[i]; }
   }
 }
 """
 
 
-@pytest.fixture(scope="module")
-def cells(tmp_path_factory):
+@pytest.fixture(scope="module", params=[0, 58])  # products in integer arithmetic: none, all
+def cells(tmp_path_factory, request):
     cxx = shutil.which("g++")
     if cxx is None:
         pytest.skip("no host compiler")
     d = tmp_path_factory.mktemp("exact_cell")
     (d / "cell.cpp").write_text(SRC)
     lib = str(d / "cell.so")
-    subprocess.run([cxx, "-O2", "-std=c++17", "-ffp-contract=off", "-fPIC", "-shared", "-I",
+    subprocess.run([cxx, "-O2", f"-DFD_EXACT_INT_PRODUCTS={request.param}", "-std=c++17", "-ffp-contract=off", "-fPIC", "-shared", "-I",
                     os.path.join(REPO, "fingering_dynamics_gb300", "csrc"), str(d / "cell.cpp"), "-o", lib], check=True)
     return C.CDLL(lib).cells
 
