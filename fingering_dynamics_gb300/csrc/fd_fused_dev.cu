@@ -1,11 +1,10 @@
 // Packed-storage fused step (deviation form, FP32 arithmetic) and the
 // pack / unpack conversions, with their C ABI.
-#include "fd_fused_dev.cuh"
-#include "fd_host.h"
+#include "fd_tile.cuh"
 
 namespace fd {
 // This unit's copy of the device status word (fd_fused_dev.cuh), which the
-// register kernel latches; fd_device_status() combines it with the others.
+// tile kernel latches; fd_device_status() combines it with the others.
 int dev_device_error(unsigned* out, bool clear) { return device_error_word(out, clear); }
 int fused_tma(const fd_params& p, const fd_storage& st, const DevCoef& c, const uint16_t* mask,
               const double* inlet_ux, void* pa, void* pb, void* sa, void* sb, int nsteps, int R, cudaStream_t s);
@@ -31,14 +30,41 @@ size_t packed_bytes(int H, int W, int dtype) {
   }
 }
 
-int auto_rows_dev(int H, int W) {
-  const long long chunks = ((long long)(W / FD_DEV_VEC) + kDevLanes - 1) / kDevLanes;
-  long long R = (long long)H * chunks / (152LL * 64);
-  if (R < 4) R = 4;
-  if (R > 64) R = 64;
-  if (R > H) R = H;
-  return (int)R;
+// The tile kernel with the arithmetic of the width (fd_tile.cuh).
+template <typename SF, bool RING>
+int tile_sf(const fd_params& p, const fd_storage& st, const DevCoef& c, const uint16_t* mask, const double* inlet_ux,
+            char* pa, char* pb, float* sa, float* sb, int nsteps, cudaStream_t s) {
+  const bool sr = st.rounding == FD_ROUND_STOCHASTIC;
+  if constexpr (std::is_same_v<SF, float>) {
+    return launch_tile<float, RING, false, false>(p, c, mask, inlet_ux, pa, pb, sa, sb, nsteps, 0, s);
+  } else {
+    if (RING && (st.f_scale_log2 != 0 || st.g_scale_log2 != 0)) {
+      return sr ? launch_tile<SF, RING, RING, true>(p, c, mask, inlet_ux, pa, pb, sa, sb, nsteps, st.seed, s)
+                : launch_tile<SF, RING, RING, false>(p, c, mask, inlet_ux, pa, pb, sa, sb, nsteps, 0, s);
+    }
+    return sr ? launch_tile<SF, RING, false, true>(p, c, mask, inlet_ux, pa, pb, sa, sb, nsteps, st.seed, s)
+              : launch_tile<SF, RING, false, false>(p, c, mask, inlet_ux, pa, pb, sa, sb, nsteps, 0, s);
+  }
 }
+
+template <bool RING>
+int tile(const fd_params& p, const fd_storage& st, const DevCoef& c, const uint16_t* mask, const double* inlet_ux,
+         void* pa, void* pb, void* sa, void* sb, int nsteps, cudaStream_t s) {
+  char *a = (char*)pa, *b = (char*)pb;
+  float *x = (float*)sa, *y = (float*)sb;
+  switch (st.dtype) {
+    case FD_F16: return tile_sf<__half, RING>(p, st, c, mask, inlet_ux, a, b, x, y, nsteps, s);
+    case FD_BF16: return tile_sf<__nv_bfloat16, RING>(p, st, c, mask, inlet_ux, a, b, x, y, nsteps, s);
+    default: return tile_sf<float, RING>(p, st, c, mask, inlet_ux, a, b, x, y, nsteps, s);
+  }
+}
+
+// Cells up to which the tile kernel is taken where the staged kernel could run.
+// Per step, tile / staged, us: FP32 64 x 128 3.5 / 30, 512 x 512 9.7 / 29, 1024 x
+// 2048 64 / 72, 2048 x 2048 123 / 118; FP16 512 x 1024 15.7 / 26.9, 1024 x 1024
+// 29.5 / 34.0, 1024 x 2048 57 / 50.  The staged kernel's time does not fall with
+// the lattice (a strip is at least 16 rows, a microsecond or more each).
+constexpr long long tile_cells(int dtype) { return dtype == FD_F32 ? 3000000 : 1500000; }
 
 }  // namespace
 }  // namespace fd
@@ -103,40 +129,23 @@ int fd_fused_step_packed(const fd_params* prm, const fd_storage* st, const uint1
   FD_REQUIRE(mask && inlet_ux && pop_a && pop_b && side_a && side_b, FD_ERR_ARG, "fd_fused_step_packed: NULL pointer");
   FD_REQUIRE(pop_a != pop_b && side_a != side_b, FD_ERR_ARG, "fd_fused_step_packed: ping-pong buffers must differ");
   FD_REQUIRE(nsteps >= 0, FD_ERR_ARG, "fd_fused_step_packed: negative step count");
-  const int vec = FD_DEV_VEC;
-  FD_REQUIRE(prm->W % 4 == 0 && prm->W >= 2 * vec && prm->H >= 3, FD_ERR_SHAPE,
-             "fd_fused_step_packed: W must be a multiple of 4 and >= %d, H >= 3 (got %dx%d)", 2 * vec, prm->H, prm->W);
+  FD_REQUIRE(prm->W % 4 == 0 && prm->W >= 4 && prm->H >= 3, FD_ERR_SHAPE,
+             "fd_fused_step_packed: W must be a multiple of 4 and >= 4, H >= 3 (got %dx%d)", prm->H, prm->W);
   FD_REQUIRE(((uintptr_t)pop_a | (uintptr_t)pop_b) % 256 == 0 && (uintptr_t)mask % 16 == 0, FD_ERR_ARG,
              "fd_fused_step_packed: population buffers must be 256-byte aligned");
   if (nsteps == 0) return FD_OK;
   const DevCoef c = make_dev_coef(*prm, st->f_scale_log2, st->g_scale_log2);
   cudaStream_t s = as_stream(stream);
-  // shared-memory staged kernel: needs 16-byte aligned rows of every plane
-  if (prm->W % 8 == 0) {
-    const int r = fused_tma(*prm, *st, c, mask, inlet_ux, pop_a, pop_b, side_a, side_b, nsteps, rows_per_warp, s);
-    return r == FD_OK ? FD_OK : check_launch("fd_fused_step_packed");
-  }
-  const int R = rows_per_warp > 0 ? rows_per_warp : auto_rows_dev(prm->H, prm->W);
-  float* sa = (float*)side_a;
-  float* sb = (float*)side_b;
-  const bool sr = st->rounding == FD_ROUND_STOCHASTIC;
-  char* pa = (char*)pop_a;
-  char* pb = (char*)pop_b;
+  // The staged kernel needs 16-byte aligned rows of every plane (W a multiple of
+  // 8) and enough strips to fill the GPU; other lattices take the tile kernel,
+  // unless the caller asks for a strip height.
   int r;
-  switch (st->dtype) {
-    case FD_F16:
-      r = sr ? launch_fused_dev<__half, FD_DEV_VEC, true>(*prm, c, mask, inlet_ux, pa, pb, sa, sb, nsteps, R, st->seed, s)
-             : launch_fused_dev<__half, FD_DEV_VEC, false>(*prm, c, mask, inlet_ux, pa, pb, sa, sb, nsteps, R, 0, s);
-      break;
-    case FD_BF16:
-      r = sr ? launch_fused_dev<__nv_bfloat16, FD_DEV_VEC, true>(*prm, c, mask, inlet_ux, pa, pb, sa, sb, nsteps, R,
-                                                                 st->seed, s)
-             : launch_fused_dev<__nv_bfloat16, FD_DEV_VEC, false>(*prm, c, mask, inlet_ux, pa, pb, sa, sb, nsteps, R, 0,
-                                                                  s);
-      break;
-    default:
-      r = launch_fused_dev<float, FD_DEV_VEC, false>(*prm, c, mask, inlet_ux, pa, pb, sa, sb, nsteps, R, 0, s);
-  }
+  if (prm->W % 8 != 0)
+    r = tile<false>(*prm, *st, c, mask, inlet_ux, pop_a, pop_b, side_a, side_b, nsteps, s);
+  else if (rows_per_warp <= 0 && (long long)prm->H * prm->W <= tile_cells(st->dtype))
+    r = tile<true>(*prm, *st, c, mask, inlet_ux, pop_a, pop_b, side_a, side_b, nsteps, s);
+  else
+    r = fused_tma(*prm, *st, c, mask, inlet_ux, pop_a, pop_b, side_a, side_b, nsteps, rows_per_warp, s);
   return r == FD_OK ? FD_OK : check_launch("fd_fused_step_packed");
 }
 
