@@ -93,6 +93,8 @@ SIGNATURES = {
     "fd_pack": [_P, _I, _VP, _S, _VP, _VP],
     "fd_unpack": [_P, _S, _VP, _I, _VP, _VP],
     "fd_fused_step_packed": [_P, _S, _VP, _VP, _VP, _VP, _VP, _VP, _I, _I, _VP],
+    "fd_enter": [_P, _VP, _F, _VP, _S, _VP, _VP],
+    "fd_finish": [_P, _I, _VP, _S, _VP, _VP, _VP, _F, _VP],
     "fd_device_status": [C.POINTER(C.c_uint), _I],
     "fd_selftest_wait_timeout": [C.c_uint, _I, _VP],
     "fd_fused_step_packed_noalloc": [_P, _S, _VP, _VP, _VP, _VP, _VP, _I, _I, _VP],

@@ -39,6 +39,7 @@ UNITS = {
     "fd_fused_f32.cu": [],
     "fd_fused_dev.cu": [],
     "fd_fused_tma.cu": [],
+    "fd_finish.cu": ["-fmad=false"],
     "fd_noalloc.cu": [],
     "fd_diag.cu": [],
     "fd_batch.cu": [],

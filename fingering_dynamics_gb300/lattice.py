@@ -174,20 +174,28 @@ class Lattice:
     # ------------------------------------------------------------------
     # fused path
     # ------------------------------------------------------------------
+    def _finish_fused(self):
+        """_finish_from of the fused state into the other population buffer, in one kernel."""
+        L.call("fd_finish", C.byref(self.prm), self.fd_dtype, _ptr(self.mask),
+               None if self.storage is None else C.byref(self.storage), _ptr(self.current_buffer()),
+               _ptr(self.side[self.scur]), _ptr(self.inlet_ux), C.byref(self.fields(self.pop[1 - self.cur])),
+               self._stream())
+
     def enter_fused(self):
         """Collide the current iteration and keep the result as fused state."""
         if self.mode == "fused":
             return
-        self.boundary_fields(self.side[self.scur])
-        self.collide()
-        if self.storage is not None:
+        if self.storage is None:
+            self.boundary_fields(self.side[self.scur])
+            self.collide()
+        else:
             if self.ppop is None:
                 nbytes = L.lib().fd_packed_bytes(self.H, self.W, C.byref(self.storage))
                 if not nbytes:
                     raise L.FDError(-1, "fd_packed_bytes", "invalid storage")
                 self.ppop = [torch.empty(nbytes, dtype=torch.uint8, device=self.device) for _ in range(2)]
-            L.call("fd_pack", C.byref(self.prm), self.fd_dtype, _ptr(self.pop[self.cur]), C.byref(self.storage),
-                   _ptr(self.ppop[self.pcur]), self._stream())
+            L.call("fd_enter", C.byref(self.prm), _ptr(self.mask), C.byref(self.fields()), _ptr(self.side[self.scur]),
+                   C.byref(self.storage), _ptr(self.ppop[self.pcur]), self._stream())
         self.mode = "fused"
 
     def advance(self, n: int, rows_per_warp: int = 0):
@@ -248,16 +256,14 @@ class Lattice:
     def peek(self):
         """Fields of the next iteration (psi, rho, ux, uy, ... in the field
         tensors) without leaving fused mode: the pending packed state is
-        unpacked into the reference-layout buffers, which the fused state does
-        not use, and finished there.  The state itself is not touched, so a
+        finished into a reference-layout buffer, which the fused state does
+        not use.  The state itself is not touched, so a
         lattice that is a member of an ensemble can be read between batched
         steps."""
         self._require("fused")
         if self.storage is None:
             raise ValueError("peek needs packed storage (dtype f32, f16 or bf16)")
-        L.call("fd_unpack", C.byref(self.prm), C.byref(self.storage), _ptr(self.ppop[self.pcur]), self.fd_dtype,
-               _ptr(self.pop[self.cur]), self._stream())
-        self._finish_from(self.pop[self.cur], self.side[self.scur], self.pop[1 - self.cur])
+        self._finish_fused()
 
     def restart_from_fields(self, psi, ux, uy, rho=None, iteration: int | None = None,
                             regularised: bool = False):
@@ -323,11 +329,7 @@ class Lattice:
         """Finish the pending iteration; the fields become current."""
         if self.mode == "reference":
             return
-        if self.storage is not None:
-            L.call("fd_unpack", C.byref(self.prm), C.byref(self.storage), _ptr(self.ppop[self.pcur]), self.fd_dtype,
-                   _ptr(self.pop[self.cur]), self._stream())
-        src, dst = self.pop[self.cur], self.pop[1 - self.cur]
-        self._finish_from(src, self.side[self.scur], dst)
+        self._finish_fused()
         self.cur = 1 - self.cur
         self.mode = "reference"
         self.iteration += 1

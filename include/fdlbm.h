@@ -259,6 +259,22 @@ int fd_pack(const fd_params* prm, int src_dtype, const void* src, const fd_stora
 /* Packed -> reference layout (18 planes of dst_dtype). */
 int fd_unpack(const fd_params* prm, const fd_storage* st, const void* src, int dst_dtype, void* dst, void* stream);
 
+/* fd_boundary_fields (into `side`), fd_collide (in place) and fd_pack (into
+ * `dst`, fd_packed_bytes()) of an FP32 state in one pass: the start of a fused
+ * run.  The same bits as the three calls. */
+int fd_enter(const fd_params* prm, const uint16_t* mask, const fd_fields* fields, void* side, const fd_storage* st,
+             void* dst, void* stream);
+
+/* The pending part of an iteration of a fused state (fingering_periodic.py:
+ * 461-479): stream, bounce-back, Zou-He, rho and psi, macroscopic fields, from
+ * `src` (packed as `st` says, or with st NULL 18 planes of dtype) and its
+ * boundary values `side` into `out`, whose f and g are 9 planes each and must
+ * not overlap src.  The same bits as fd_unpack, fd_stream, fd_bounce_back,
+ * fd_zou_he_inlet, fd_zou_he_outlet, fd_update_rho_psi and fd_update_macros one
+ * after the other. */
+int fd_finish(const fd_params* prm, int dtype, const uint16_t* mask, const fd_storage* st, const void* src,
+              const void* side, const double* inlet_ux, const fd_fields* out, void* stream);
+
 /* fd_fused_step on packed buffers (the same loop body, fingering_periodic.py:454-479
  * / fingering.py:558-585, computed in FP32 in deviation form).  pop_a/pop_b:
  * fd_packed_bytes() each, 256-byte aligned; side_a/side_b: 6*H floats.
