@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "fd_batch_plan.h"
 #include "fd_fused_tma.cuh"
 #include "fd_host.h"
 
@@ -17,7 +18,8 @@ struct fd_batch {
   std::vector<fd_instance> inst;
   void* d_inst = nullptr;  // BatchInst<SF>[n]
   int4* d_tiles = nullptr;
-  int ntiles = 0;
+  int ntiles = 0;  // tiles of the shape asked for (fd_batch_tiles)
+  int nwork = 0;   // tiles of the table, whose strips may be shorter (fd_batch_plan.h)
   int grid = 0;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -68,7 +70,14 @@ int prepare(fd_batch* b) {
   auto kern = k_fused_tma_batch<SF, NT, tma_ring_depth<SF>(), false, STOCH>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, M::ALLOC) != cudaSuccess)
     return check_launch("fd_batch: shared-memory attribute");
+  int per_sm = 1, dev = 0, sms = 1;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, M::ALLOC);
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  b->grid = per_sm * sms;
   std::vector<BatchInst<SF>> hi(b->n);
+  BatchShape shape;
+  b->ntiles = 0;
   std::vector<int4> tiles;
   // members already flagged non-finite are not stepped any more: leave their
   // tiles out, so that the live members' tiles share the persistent grid
@@ -81,20 +90,21 @@ int prepare(fd_batch* b) {
     hi[i].args[1] = instance_args<SF>(b->inst[i], b->st, b->rows, true, b->d_status + i);
     if (int r = tma_maps<SF, NT>(hi[i].args[0], (const char*)b->inst[i].pop_a, hi[i].maps[0])) return r;
     if (int r = tma_maps<SF, NT>(hi[i].args[1], (const char*)b->inst[i].pop_b, hi[i].maps[1])) return r;
-    const int nb = (b->inst[i].prm.W + NT - 1) / NT, ns = hi[i].args[0].nstrips;
-    if (flagged[(size_t)i] != 0u) continue;
-    for (int s = 0; s < ns; ++s)
-      for (int bb = 0; bb < nb; ++bb) tiles.push_back(make_int4(i, bb, s, 0));
+    const int nb = flagged[(size_t)i] != 0u ? 0 : (b->inst[i].prm.W + NT - 1) / NT;
+    b->ntiles += nb * hi[i].args[0].nstrips;
+    shape.height.push_back(b->inst[i].prm.H);
+    shape.bands.push_back(nb);
+  }
+  const std::vector<int> strips = plan_strips(shape, b->rows, b->grid);
+  for (int i = 0; i < b->n; ++i) {
+    const int H = shape.height[(size_t)i], R = strip_rows(H, strips[(size_t)i]);
+    for (int y = 0; y < H; y += R)
+      for (int bb = 0; bb < shape.bands[(size_t)i]; ++bb) tiles.push_back(make_int4(i, bb, y, std::min(y + R, H)));
   }
   // largest first (rows of the tile's strip), ties in table order: the
   // kernel's counter then hands them out greedily
-  auto strip_rows = [&](const int4& t) {
-    const DevArgs<SF>& a = hi[t.x].args[0];
-    const int y0 = t.z * a.R;
-    return (y0 + a.R < a.H ? y0 + a.R : a.H) - y0;
-  };
   std::stable_sort(tiles.begin(), tiles.end(),
-                   [&](const int4& u, const int4& v) { return strip_rows(u) > strip_rows(v); });
+                   [](const int4& u, const int4& v) { return u.w - u.z > v.w - v.z; });
   cudaFree(b->d_inst);
   cudaFree(b->d_tiles);
   b->d_inst = nullptr;
@@ -106,13 +116,8 @@ int prepare(fd_batch* b) {
       (!tiles.empty() &&
        cudaMemcpy(b->d_tiles, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice) != cudaSuccess))
     return check_launch("fd_batch: table upload");
-  b->ntiles = (int)tiles.size();
-  int per_sm = 1, dev = 0, sms = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, M::ALLOC);
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  b->grid = per_sm * sms;
-  if (b->grid > b->ntiles) b->grid = b->ntiles;
+  b->nwork = (int)tiles.size();
+  if (b->grid > b->nwork) b->grid = b->nwork;
   if (b->grid < 1) b->grid = 1;
   return FD_OK;
 }
@@ -121,7 +126,7 @@ template <typename SF, int NT, bool STOCH>
 void launch_one(const fd_batch* b, int parity, cudaStream_t st) {
   using M = TmaSmem<SF, NT, tma_ring_depth<SF>()>;
   k_fused_tma_batch<SF, NT, tma_ring_depth<SF>(), false, STOCH><<<b->grid, NT, M::ALLOC, st>>>(
-      (const BatchInst<SF>*)b->d_inst, b->d_tiles, b->ntiles, parity, b->d_ctl);
+      (const BatchInst<SF>*)b->d_inst, b->d_tiles, b->nwork, parity, b->d_ctl);
 }
 
 template <typename SF, bool STOCH>

@@ -424,13 +424,13 @@ __device__ __forceinline__ DevStencil ring_stencil(const PsiRing<SF, NT, NS>& ri
   }
 }
 
-// One strip of one band: the body shared by the single-lattice kernel and the
+// One strip of one band (rows y0 .. y1 - 1): the body shared by the single-lattice kernel and the
 // batched persistent kernel.  The mbarriers must be initialised; `phase`
 // (per-slot parity of the next fill to wait for) and `ok` carry over from
 // strip to strip.  Ends with a CTA barrier, so the ring can be refilled.
 template <typename SF, int NT, int NS, bool SCALED, bool STOCH>
-__device__ __forceinline__ void tma_strip_ring(const DevArgs<SF>& a, const TmaMaps* tm, int band, int strip, char* smem,
-                                               unsigned& phase, bool& ok) {
+__device__ __forceinline__ void tma_strip_ring(const DevArgs<SF>& a, const TmaMaps* tm, int band, int y0, int y1,
+                                               char* smem, unsigned& phase, bool& ok) {
   static_assert(NS >= 5, "rows y-2 .. y+2 must be resident while row y is computed");
   using L = SlotLayout<SF, NT>;
   using M = TmaSmem<SF, NT, NS>;
@@ -440,7 +440,6 @@ __device__ __forceinline__ void tma_strip_ring(const DevArgs<SF>& a, const TmaMa
 
   const int t = threadIdx.x;
   const int x0 = band * NT;
-  const int y0 = strip * a.R, y1 = min(y0 + a.R, a.H);
   const int x = x0 + t;
   const bool owned = x < a.W;
   const bool walls = a.variant == FD_VARIANT_WALLS;
@@ -620,7 +619,7 @@ __device__ __forceinline__ float inlet_corner_drho(const DevArgs<SF>& a, int yn)
 // share a boundary then read its halo rows at about the same time (both at
 // their start, or both at their end) and the second read finds them in L2.
 template <typename SF, int NT, bool SCALED, bool STOCH>
-__device__ __forceinline__ void tma_strip_split(const DevArgs<SF>& a, const TmaMaps* tm, int band, int strip,
+__device__ __forceinline__ void tma_strip_split(const DevArgs<SF>& a, const TmaMaps* tm, int band, int y0, int y1,
                                                 bool down, char* smem, unsigned& phase, bool& ok) {
   using L = SlotLayout<SF, NT>;
   using M = TmaSmem<SF, NT, 4>;
@@ -630,7 +629,6 @@ __device__ __forceinline__ void tma_strip_split(const DevArgs<SF>& a, const TmaM
 
   const int t = threadIdx.x;
   const int x0 = band * NT;
-  const int y0 = strip * a.R, y1 = min(y0 + a.R, a.H);
   const int n = y1 - y0;  // local rows -2 .. n+1: g halves -2 .. n+1, f halves -1 .. n
   const int x = x0 + t;
   const bool owned = x < a.W;
@@ -770,10 +768,10 @@ __device__ __forceinline__ void tma_strip_split(const DevArgs<SF>& a, const TmaM
 // `down`: walk the strip from its top row (the split ring only; the
 // whole-row ring always walks up).
 template <typename SF, int NT, int NS, bool SCALED, bool STOCH>
-__device__ __forceinline__ void tma_strip(const DevArgs<SF>& a, const TmaMaps* tm, int band, int strip, bool down,
-                                          char* smem, unsigned& phase, bool& ok) {
-  if constexpr (NS == 4) tma_strip_split<SF, NT, SCALED, STOCH>(a, tm, band, strip, down, smem, phase, ok);
-  else tma_strip_ring<SF, NT, NS, SCALED, STOCH>(a, tm, band, strip, smem, phase, ok);
+__device__ __forceinline__ void tma_strip(const DevArgs<SF>& a, const TmaMaps* tm, int band, int y0, int y1,
+                                          bool down, char* smem, unsigned& phase, bool& ok) {
+  if constexpr (NS == 4) tma_strip_split<SF, NT, SCALED, STOCH>(a, tm, band, y0, y1, down, smem, phase, ok);
+  else tma_strip_ring<SF, NT, NS, SCALED, STOCH>(a, tm, band, y0, y1, smem, phase, ok);
 }
 
 template <typename SF, int NT, int NS>
@@ -812,8 +810,9 @@ __global__ void __launch_bounds__(NT) k_fused_tma(const __grid_constant__ DevArg
   unsigned phase = 0;
   bool ok = true;
   const int strip = strip0 + (int)blockIdx.x / nbands;
-  tma_strip<SF, NT, NS, SCALED, STOCH>(a, &tm, (int)blockIdx.x % nbands, strip, FD_TMA_WALK_DOWN && (strip & 1),
-                                       smem, phase, ok);
+  const int y0 = strip * a.R;
+  tma_strip<SF, NT, NS, SCALED, STOCH>(a, &tm, (int)blockIdx.x % nbands, y0, min(y0 + a.R, a.H),
+                                       FD_TMA_WALK_DOWN && (strip & 1), smem, phase, ok);
 }
 
 // One lattice of a batch: its arguments and the tensor maps of its source
@@ -824,7 +823,7 @@ struct BatchInst {
   TmaMaps maps[2];
 };
 
-// Persistent kernel over a tile table of (instance, band, strip) entries,
+// Persistent kernel over a tile table of (instance, band, first row, end row) entries,
 // largest tiles first: each CTA takes the next untaken tile from a counter
 // until none is left (greedy largest-first balancing of uneven tiles).  Every
 // instance advances one iteration.
@@ -876,7 +875,7 @@ __global__ void __launch_bounds__(NT, (NS == 4 ? tma_resident_ctas<SF, NT, NS>()
       continue;
     }
     const int4 tl = tiles[k];
-    tma_strip<SF, NT, NS, SCALED, STOCH>(sa, stm, tl.y, tl.z, false, smem, phase, ok);
+    tma_strip<SF, NT, NS, SCALED, STOCH>(sa, stm, tl.y, tl.z, tl.w, false, smem, phase, ok);
   }
 }
 

@@ -353,7 +353,8 @@ typedef struct fd_batch fd_batch;
  * Every iteration is one persistent launch of the staged kernel over a table
  * of (member, band, strip) tiles: bands of band_width cells (64, 128, 256) and
  * strips of at most rows_per_strip rows (a member's strips are of equal
- * height within one row).  Allocates the (small) device tables. */
+ * height within one row; they are cut shorter where that fills the persistent
+ * grid's rounds better).  Allocates the (small) device tables. */
 int fd_batch_create(const fd_instance* inst, int n, const fd_storage* st, int rows_per_strip, int band_width,
                     fd_batch** out);
 
@@ -381,7 +382,7 @@ int fd_batch_parity(const fd_batch* b);
  * Returns FD_ERR_NONFINITE if any member is flagged, FD_OK otherwise. */
 int fd_batch_member_status(fd_batch* b, uint32_t* out, int clear);
 
-/* Number of tiles per iteration. */
+/* Number of tiles per iteration in strips as tall as rows_per_strip allows. */
 int fd_batch_tiles(const fd_batch* b);
 
 /* CTAs of the persistent launch (resident CTAs per SM x SMs, at most the tile
