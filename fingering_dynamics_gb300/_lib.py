@@ -88,6 +88,8 @@ SIGNATURES = {
     "fd_update_rho_psi": [_P, _I, _VP, _F, _VP],
     "fd_update_macros": [_P, _I, _VP, _F, _VP],
     "fd_field": [_P, _I, _I, _VP, _F, _VP, _VP],
+    "fd_collision_term_fluid": [_P, _I, _I, _I, _VP, C.c_int64, _F, _VP, _VP],
+    "fd_field_fluid": [_P, _I, _I, _VP, C.c_int64, _F, _VP, _VP],
     "fd_fused_step": [_P, _I, _VP, _VP, _VP, _VP, _VP, _VP, _I, _I, _VP],
     "fd_packed_bytes": [_I, _I, _S],
     "fd_pack": [_P, _I, _VP, _S, _VP, _VP],

@@ -68,8 +68,9 @@ class ComputeBase:
         if self.mask.shape != (H, W):
             raise ValueError(f"mask shape {self.mask.shape} does not match H, W = {H}, {W}")
         self.block_mask = np.logical_not(self.mask)
-        self._mask_t = torch.from_numpy(self.mask).to(self._dev)
         self._n_fluid = int(self.mask.sum())
+        self._cells = torch.from_numpy(np.flatnonzero(self.mask)).to(self._dev)  # fluid cells, row-major
+        self._inlet = None  # (u0, inlet profile on the device)
         word = np.where(self.block_mask, SOLID_BIT, 0).astype(np.uint16)
         self._word = torch.from_numpy(word.view(np.int16)).to(self._dev)
         self.gamma = float(gl["gamma"])
@@ -118,13 +119,13 @@ class ComputeBase:
                 raise ValueError("Compute arrays must stay contiguous tensors of the lattice's dtype and device")
 
     def _masked_get(self, name):
-        return self._full[name][self._mask_t]
+        return torch.index_select(self._full[name].view(-1), 0, self._cells)
 
     def _masked_set(self, name, value):
         v = torch.as_tensor(value, dtype=self._dtype, device=self._dev)
         if v.shape != (self._n_fluid,):
             raise ValueError(f"{name} must have shape ({self._n_fluid},)")
-        self._full[name][self._mask_t] = v
+        self._full[name].view(-1).index_copy_(0, self._cells, v)
 
     rho = property(lambda s: s._masked_get("rho"), lambda s, v: s._masked_set("rho", v))
     ux = property(lambda s: s._masked_get("ux"), lambda s, v: s._masked_set("ux", v))
@@ -135,17 +136,22 @@ class ComputeBase:
 
     def _field(self, name, masked=True):
         self._check_layout()
+        if masked:
+            out = torch.empty(self._n_fluid, dtype=self._dtype, device=self._dev)
+            L.call("fd_field_fluid", C.byref(self._prm), self._fd, L.FIELDS[name], _vp(self._cells), self._n_fluid,
+                   C.byref(self._fields()), _vp(out), _stream())
+            return out
         out = torch.zeros((self.H, self.W), dtype=self._dtype, device=self._dev)
         L.call("fd_field", C.byref(self._prm), self._fd, L.FIELDS[name], _vp(self._word), C.byref(self._fields()),
                _vp(out), _stream())
-        return out[self._mask_t] if masked else out
+        return out
 
     def _term(self, term, j):
         self._check_layout()
-        out = torch.zeros((self.H, self.W), dtype=self._dtype, device=self._dev)
-        L.call("fd_collision_term", C.byref(self._prm), self._fd, L.TERMS[term], int(j), _vp(self._word),
-               C.byref(self._fields()), _vp(out), _stream())
-        return out[self._mask_t]
+        out = torch.empty(self._n_fluid, dtype=self._dtype, device=self._dev)
+        L.call("fd_collision_term_fluid", C.byref(self._prm), self._fd, L.TERMS[term], int(j), _vp(self._cells),
+               self._n_fluid, C.byref(self._fields()), _vp(out), _stream())
+        return out
 
     # -- the reference's methods -------------------------------------------------
     def getP(self):            # fingering_periodic.py:123-124
@@ -205,7 +211,10 @@ class ComputeBase:
     def _zou_he(self, fn):
         self._check_layout()
         side = torch.empty((6, self.H), dtype=self._dtype, device=self._dev)
-        ux = torch.from_numpy(self._inlet_ux()).to(self._dev)
+        u0 = float(self._globals()["u0"])
+        if self._inlet is None or self._inlet[0] != u0:
+            self._inlet = (u0, torch.from_numpy(self._inlet_ux()).to(self._dev))
+        ux = self._inlet[1]
         L.call("fd_boundary_fields", C.byref(self._prm), self._fd, _vp(self._word), _vp(self.psi),
                _vp(self.nabla_psi2), _vp(side), _stream())
         L.call(fn, C.byref(self._prm), self._fd, _vp(self.f), _vp(self.g), _vp(side), _vp(ux), _stream())

@@ -154,6 +154,12 @@ int fd_collide(const fd_params* prm, int dtype, const uint16_t* mask, const fd_f
 int fd_collision_term(const fd_params* prm, int dtype, int term, int j, const uint16_t* mask,
                       const fd_fields* fields, void* out, void* stream);
 
+/* fd_collision_term on n listed cells (row-major indices below H*W of fluid
+ * cells, device int64), densely packed into out[0..n-1]: the array the
+ * reference's getter returns (its arrays hold fluid cells only). */
+int fd_collision_term_fluid(const fd_params* prm, int dtype, int term, int j, const int64_t* cells, int64_t n,
+                            const fd_fields* fields, void* out, void* stream);
+
 /* stream(f, g) (fingering_periodic.py:327-343): dst = src shifted by e_i,
  * periodic in x and y, every cell.  src and dst must not overlap. */
 int fd_stream(const fd_params* prm, int dtype, const void* src_f, const void* src_g, void* dst_f,
@@ -203,6 +209,11 @@ int fd_update_macros(const fd_params* prm, int dtype, const uint16_t* mask, cons
  * fields into `out` ((H,W)). */
 int fd_field(const fd_params* prm, int dtype, int field_id, const uint16_t* mask, const fd_fields* fields,
              void* out, void* stream);
+
+/* fd_field for rho, mu, ux, uy, p and mix_tau on n listed fluid cells, densely
+ * packed as fd_collision_term_fluid does. */
+int fd_field_fluid(const fd_params* prm, int dtype, int field_id, const int64_t* cells, int64_t n,
+                   const fd_fields* fields, void* out, void* stream);
 
 /* ---- fused step --------------------------------------------------------- */
 
