@@ -45,7 +45,9 @@ UNITS = {
     "fd_batch.cu": [],
     "fd_host_step.cu": [],
     "sg_kernels.cu": [],
+    "sg_conv.cu": [],
     "sg_tcgen05.cu": [],
+    "sg_wgrad.cu": [],
 }
 
 

@@ -1,0 +1,349 @@
+// 3x3 convolution (forward and data gradient) of the learned surrogate at widths
+// that are multiples of 128, on tcgen05 (sg_conv3x3_tma, sg_conv3x3_tma_ws).
+//
+// Implicit GEMM, M = pixels, N = output channels, K = 9 x input channels.  A
+// persistent CTA walks tiles of R image rows x 128 pixels x BN output channels
+// (R accumulators of BN tensor-memory columns, two buffers of them):
+//   warp 8  (one thread) issues the boxes.  A: per chunk of CH input channels one
+//           box of the input's halo, (R + 2) rows x 130 pixels x CH channels,
+//           swizzled over the pixel's 32 or 64 bytes; pixels outside the image
+//           read as zero, the convolution's padding.  B: per chunk nine boxes of
+//           BN output channels x CH, one per tap.  Where the weights of all chunks
+//           fit beside the ring they are loaded once per CTA and stay;
+//   warp 9  issues the MMAs of a stage: each tap's A operand is the window that
+//           starts at row r + ky and pixel kx of the halo (the swizzle follows the
+//           address, so a window may start on any pixel).  The descriptors are a
+//           base and constants, in uniform registers;
+//   warps 0..7 finish tile j (bias, GELU, stores) while tile j + 1 is multiplied.
+// K advances 16 channels at a time, the nine taps of a slice back to back, so the
+// FP32 sums run in one order whatever the chunk and tile.
+//
+// What it replaced: boxes of 8 channels (16-byte pieces, four to eight times as
+// many), the weights streamed anew for every tile, two descriptors built per MMA
+// by the thread that also issued the boxes.  Measured at batch 32, us, before ->
+// here: 16 -> 32 (256 x 512, GELU) 271 -> 169, 32 -> 32 354 -> 191, 96 -> 32 855 ->
+// 340, 32 -> 96 (no activation) 924 -> 302, 64 -> 64 (128 x 256) 250 -> 126, 192 ->
+// 64 507 -> 204, 128 -> 128 (64 x 128) 207 -> 83, 384 -> 128 397 -> 160 (1448
+// TFLOP/s).  The thin layers with GELU are bound by the epilogue's tanhf and the
+// writes of z and y (537 MB, 79 us), the wide ones by the tensor pipe.
+#include "sg_tc.cuh"
+
+namespace sg {
+namespace {
+
+constexpr int kCvEpiWarps = 8;
+constexpr int kCvThreads = 32 * (kCvEpiWarps + 2);
+
+template <int BN, int R, int CH>
+struct CvCfg {
+  static constexpr int ROW = CH * 2;                                        // bytes of a pixel or output channel
+  static constexpr int A_TX = (R + 2) * kHaloPx * ROW;
+  static constexpr int A_BYTES = (A_TX + 1023) / 1024 * 1024;
+  static constexpr int TAP = BN * ROW, B_BYTES = (9 * TAP + 1023) / 1024 * 1024;  // one tap's and one chunk's weights
+  static constexpr int NCOL = 2 * R * BN;                                   // two accumulator buffers
+  static constexpr int COLS = NCOL <= 32 ? 32 : (NCOL <= 64 ? 64 : (NCOL <= 128 ? 128 : (NCOL <= 256 ? 256 : 512)));
+  static constexpr int S_MAX = 6;
+  static constexpr int TAIL = (2 * S_MAX + 5) * 8 + BN * 4 + 16 + 1024;       // barriers, bias, TMEM address, alignment
+  static_assert(NCOL <= 512 && TAP % (8 * ROW) == 0, "tile");
+};
+
+struct CvShape {
+  int N, H, W, Cin, Cout, act;
+  int nk, S;       // chunks, ring stages
+  int resident;    // the weights of all chunks stay in shared memory
+};
+
+template <int BN, int R, int CH>
+__global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_rows(const __grid_constant__ ConvMaps maps, const CvShape sh,
+                                                               const float* __restrict__ bias, bf16* __restrict__ z,
+                                                               bf16* __restrict__ y) {
+  using C = CvCfg<BN, R, CH>;
+  extern __shared__ char smem_raw[];
+  char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  const int S = sh.S, nk = sh.nk, stage = C::A_BYTES + (sh.resident ? 0 : C::B_BYTES);
+  char* wres = smem + S * stage;  // resident weights
+  char* tail = wres + (sh.resident ? nk * C::B_BYTES : 0);
+  uint64_t* full = reinterpret_cast<uint64_t*>(tail);
+  uint64_t *empty = full + C::S_MAX, *accf = empty + C::S_MAX, *acce = accf + 2, *wfull = acce + 2;
+  float* sbias = reinterpret_cast<float*>(wfull + 1);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sbias + BN);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tiles_x = sh.W / kTcBM, nco = sh.Cout / BN;
+  const int ntiles = sh.N * (sh.H / R) * tiles_x * nco;
+  const int mine = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;  // this CTA's tiles
+  // the grid is a multiple of the output-channel tiles, so a CTA keeps one of them
+  const int co0 = ((int)blockIdx.x % nco) * BN;
+
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(C::COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (tid == 0) {
+    for (int i = 0; i < 2 * C::S_MAX + 2; ++i) mbar_init(&full[i]);
+    mbar_init(wfull);
+    for (int i = 0; i < 2; ++i)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&acce[i])), "n"(kCvEpiWarps) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  for (int i = tid; i < BN; i += kCvThreads) sbias[i] = bias ? bias[co0 + i] : 0.0f;
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+
+  // tile j of this CTA -> (first output row n H + yy, x0)
+  auto tile_of = [&](int j, int& row, int& x0) {
+    const int pt = ((int)blockIdx.x + j * (int)gridDim.x) / nco;
+    x0 = (pt % tiles_x) * kTcBM;
+    row = (pt / tiles_x) * R;
+  };
+
+  if (warp == kCvEpiWarps) {
+    if (lane == 0 && mine > 0) {
+      auto load_b = [&](char* dst, int kc, uint64_t* bar) {
+#pragma unroll
+        for (int tap = 0; tap < 9; ++tap) tma_load_3d(dst + tap * C::TAP, &maps.w, kc * CH, tap, co0, bar);
+      };
+      if (sh.resident) {
+        mbar_expect_tx(wfull, (unsigned)(nk * 9 * C::TAP));
+        for (int kc = 0; kc < nk; ++kc) load_b(wres + kc * C::B_BYTES, kc, wfull);
+      }
+      const unsigned tx = (unsigned)(C::A_TX + (sh.resident ? 0 : 9 * C::TAP));
+      int c = 0;  // chunks issued
+      bool ok = true;
+      for (int j = 0; j < mine && ok; ++j) {
+        int row, x0;
+        tile_of(j, row, x0);
+        const int n = row / sh.H, yy = row % sh.H;
+        for (int kc = 0; kc < nk; ++kc, ++c) {
+          const int st = c % S;
+          if (c >= S) ok = mbar_wait_ok(&empty[st], (unsigned)(c / S - 1) & 1u, true);
+          if (!ok) break;
+          char* a = smem + st * stage;
+          mbar_expect_tx(&full[st], tx);
+          tma_load_4d(a, &maps.x, kc * CH, x0 - 1, yy - 1, n, &full[st]);
+          if (!sh.resident) load_b(a + C::A_BYTES, kc, &full[st]);
+        }
+      }
+      // everything issued has landed before the CTA gives its shared memory up
+      if (sh.resident) mbar_wait_ok(wfull, 0u, false);
+      for (int i = 0; i < S && i < c; ++i)
+        mbar_wait_ok(&full[i], (unsigned)((c - 1 - ((c - 1 - i) % S)) / S) & 1u, false);
+    }
+    __syncwarp();
+  } else if (warp == kCvEpiWarps + 1) {
+    uint32_t leader;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(leader));
+    constexpr uint32_t idesc = instr_desc<kTcBM, BN>();
+    const uint64_t a0 = smem_desc_sw<C::ROW>(smem_u32(smem), 16, 8 * C::ROW);
+    const uint64_t w0 = smem_desc_sw<C::ROW>(smem_u32(sh.resident ? wres : smem + C::A_BYTES), 16, 8 * C::ROW);
+    bool ok = mine > 0 && (!sh.resident || mbar_wait_ok(wfull, 0u, true));
+    int c = 0;
+    for (int j = 0; j < mine && ok; ++j) {
+      const int b = j & 1;
+      if (j >= 2) ok = mbar_wait_ok(&acce[b], (unsigned)((j - 2) >> 1) & 1u, true);  // tile j - 2 has been read
+      const uint32_t d0 = tmem + (uint32_t)(b * R * BN);
+      for (int kc = 0; kc < nk && ok; ++kc, ++c) {
+        const int st = c % S;
+        ok = mbar_wait_ok(&full[st], (unsigned)(c / S) & 1u, true);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        // an address step of 16 bytes is 1 in the descriptors' low bits
+        const uint64_t as = a0 + (uint64_t)(st * stage / 16);
+        const uint64_t bs = w0 + (uint64_t)((sh.resident ? kc * C::B_BYTES : st * stage) / 16);
+        if (leader) {
+#pragma unroll
+          for (int s = 0; s < CH / 16; ++s) {
+#pragma unroll
+            for (int tap = 0; tap < 9; ++tap) {
+              const int ky = tap / 3, kx = tap % 3;
+              const uint32_t acc = (s > 0 || tap > 0) ? 1u : (kc > 0 ? 1u : 0u);
+#pragma unroll
+              for (int r = 0; r < R; ++r)
+                tc_mma(d0 + (uint32_t)(r * BN), as + (uint64_t)((((r + ky) * kHaloPx + kx) * C::ROW + s * 32) / 16),
+                       bs + (uint64_t)((tap * C::TAP + s * 32) / 16), idesc, acc);
+            }
+          }
+          tc_commit(&empty[st]);
+          if (kc == nk - 1) tc_commit(&accf[b]);  // tile j's accumulators are complete
+        }
+        __syncwarp();
+      }
+    }
+    // the MMAs issued have completed before tensor and shared memory are given up
+    for (int i = 0; i < S && i < c; ++i)
+      mbar_wait_ok(&empty[i], (unsigned)((c - 1 - ((c - 1 - i) % S)) / S) & 1u, false);
+  } else {
+    // epilogue: warp w reads TMEM lanes 32 q .. 32 q + 31 (pixels x0 + 32 q + lane of each row, q = w % 4) of every
+    // second group of 16 columns (w / 4)
+    const int q = warp & 3, h = warp >> 2;
+    for (int j = 0; j < mine; ++j) {
+      const int b = j & 1;
+      int row, x0;
+      tile_of(j, row, x0);
+      mbar_wait_ok(&accf[b], (unsigned)(j >> 1) & 1u, true);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+      for (int i = h; i < R * (BN / 16); i += 2) {
+        const int r = i / (BN / 16), c0 = (i % (BN / 16)) * 16;
+        float v[16];
+        tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * R * BN + i * 16), v);
+        const size_t o = ((size_t)(row + r) * sh.W + x0 + q * 32 + lane) * sh.Cout + co0 + c0;
+        uint32_t zw[8], yw[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          float t0 = v[2 * k] + sbias[c0 + 2 * k], t1 = v[2 * k + 1] + sbias[c0 + 2 * k + 1];
+          const __nv_bfloat162 zp = __floats2bfloat162_rn(t0, t1);
+          zw[k] = *reinterpret_cast<const uint32_t*>(&zp);
+          if (sh.act == SG_ACT_GELU) {
+            t0 = gelu_f(t0);
+            t1 = gelu_f(t1);
+          }
+          const __nv_bfloat162 yp = __floats2bfloat162_rn(t0, t1);
+          yw[k] = *reinterpret_cast<const uint32_t*>(&yp);
+        }
+        if (z) {
+          reinterpret_cast<uint4*>(z + o)[0] = make_uint4(zw[0], zw[1], zw[2], zw[3]);
+          reinterpret_cast<uint4*>(z + o)[1] = make_uint4(zw[4], zw[5], zw[6], zw[7]);
+        }
+        if (y) {
+          reinterpret_cast<uint4*>(y + o)[0] = make_uint4(yw[0], yw[1], yw[2], yw[3]);
+          reinterpret_cast<uint4*>(y + o)[1] = make_uint4(yw[4], yw[5], yw[6], yw[7]);
+        }
+      }
+      // this warp's reads of buffer b are complete (tcgen05.wait::ld in tmem_ld16)
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acce[b])) : "memory");
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C::COLS) : "memory");
+  }
+}
+
+// Tensor maps of one call: x as (C, W, H, N) with boxes of CH channels x 130
+// pixels x R + 2 rows, the weights [co][tap][ci] as (Cin, 9, Cout) with boxes of
+// CH channels x 1 tap x BN output channels.
+inline int encode_conv_maps(ConvMaps& m, const bf16* x, int N, int H, int W, int Cin, const bf16* w, int Cout,
+                            int R, int BN, int CH) {
+  const fd::EncodeTiledFn fn = fd::encode_tiled_fn();
+  FD_REQUIRE(fn != nullptr, FD_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  const CUtensorMapSwizzle sw = CH == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
+  const cuuint64_t es = 2;
+  const cuuint64_t xd[4] = {(cuuint64_t)Cin, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
+  const cuuint64_t xs[3] = {Cin * es, (cuuint64_t)W * Cin * es, (cuuint64_t)H * W * Cin * es};
+  const cuuint32_t xb[4] = {(cuuint32_t)CH, (cuuint32_t)kHaloPx, (cuuint32_t)(R + 2), 1u};
+  const cuuint32_t e4[4] = {1u, 1u, 1u, 1u};
+  CUresult r = fn(&m.x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(x), xd, xs, xb, e4,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  FD_REQUIRE(r == CUDA_SUCCESS, FD_ERR_CUDA, "sg_conv3x3_tma: input tensor map (%d)", (int)r);
+  const cuuint64_t wd[3] = {(cuuint64_t)Cin, 9u, (cuuint64_t)Cout};
+  const cuuint64_t ws[2] = {Cin * es, 9u * Cin * es};
+  const cuuint32_t wb[3] = {(cuuint32_t)CH, 1u, (cuuint32_t)BN};
+  r = fn(&m.w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(w), wd, ws, wb, e4,
+         CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  FD_REQUIRE(r == CUDA_SUCCESS, FD_ERR_CUDA, "sg_conv3x3_tma: weight tensor map (%d)", (int)r);
+  return FD_OK;
+}
+
+struct CvCall {
+  const bf16* x;
+  int N, H, W, Cin;
+  const bf16* w;
+  const float* b;
+  int Cout, act;
+  bf16 *z, *y;
+  cudaStream_t s;
+  int sms;
+};
+
+template <int BN, int R, int CH>
+int launch_rows(const CvCall& c) {
+  using C = CvCfg<BN, R, CH>;
+  auto kern = k_conv3x3_rows<BN, R, CH>;
+  static std::atomic<unsigned long long> attr_done{0};
+  if (fd::ensure_smem_attr(kern, 227 * 1024, attr_done) != cudaSuccess)
+    return fd::check_launch("sg_conv3x3_tma: shared-memory attribute");
+  constexpr int kRoom = 227 * 1024 - C::TAIL;
+  CvShape sh{c.N, c.H, c.W, c.Cin, c.Cout, c.act, c.Cin / CH, 0, 0};
+  // the weights stay where two stages of the ring fit beside them (or all the chunks there are)
+  const int need = sh.nk < 2 ? 1 : 2;
+  sh.resident = sh.nk * C::B_BYTES + need * C::A_BYTES <= kRoom;
+  const int stage = C::A_BYTES + (sh.resident ? 0 : C::B_BYTES);
+  sh.S = std::min<int>(C::S_MAX, (kRoom - (sh.resident ? sh.nk * C::B_BYTES : 0)) / stage);
+  if (sh.S < 1) {
+    fd::set_error("sg_conv3x3_tma: no stage fits");
+    return FD_ERR_SHAPE;
+  }
+  const int nco = c.Cout / BN;
+  const long long ntiles = (long long)c.N * (c.H / R) * (c.W / kTcBM) * nco;
+  const long long grid = std::min<long long>(ntiles, std::max(1, c.sms / nco) * (long long)nco);
+  ConvMaps maps;
+  if (int r = encode_conv_maps(maps, c.x, c.N, c.H, c.W, c.Cin, c.w, c.Cout, R, BN, CH)) return r;
+  kern<<<(unsigned)grid, kCvThreads, 227 * 1024, c.s>>>(maps, sh, c.b, c.z, c.y);
+  return fd::check_launch("sg_conv3x3_tma");
+}
+
+// Rows per tile: the most of 4, 2, 1 that divide H with two buffers of R x BN
+// accumulator columns in the tensor memory, and fewer where there would be less
+// than two tiles per SM (a batch of one: 256 x 512 has 256 tiles of four rows).
+constexpr long long kCvTiles = 2;
+template <int BN, int CH>
+int rows_r(const CvCall& c) {
+  const long long per_row = (long long)c.N * c.H * (c.W / kTcBM) * (c.Cout / BN), want = kCvTiles * c.sms;
+  if constexpr (BN <= 64) {
+    if (c.H % 4 == 0 && per_row / 4 >= want) return launch_rows<BN, 4, CH>(c);
+  }
+  if (c.H % 2 == 0 && per_row / 2 >= want) return launch_rows<BN, 2, CH>(c);
+  return launch_rows<BN, 1, CH>(c);
+}
+
+template <int CH>
+int rows_n(const CvCall& c) {
+  if (c.Cout % 128 == 0) return rows_r<128, CH>(c);
+  if (c.Cout % 96 == 0 && c.Cout % 64 != 0) return rows_r<96, CH>(c);
+  if (c.Cout % 64 == 0) return rows_r<64, CH>(c);
+  if (c.Cout % 32 == 0) return rows_r<32, CH>(c);
+  return rows_r<16, CH>(c);
+}
+
+int conv_rows(const void* x, int N, int H, int W, int Cin, const void* w, const float* bias, int Cout, int act, void* z,
+              void* y, void* stream, const char* what) {
+  FD_REQUIRE(x && w && (z || y) && N > 0 && H > 0 && W > 0, FD_ERR_ARG, "%s: bad arguments", what);
+  FD_REQUIRE(W % kTcBM == 0 && Cin % 16 == 0 && Cout % 16 == 0 && Cin > 0 && Cout > 0, FD_ERR_SHAPE,
+             "%s: needs W a multiple of 128 and channel counts multiples of 16 (got W=%d, %d -> %d)", what, W, Cin, Cout);
+  FD_REQUIRE(act == SG_ACT_NONE || act == SG_ACT_GELU, FD_ERR_ARG, "%s: activation %d", what, act);
+  FD_REQUIRE(((uintptr_t)x | (uintptr_t)w | (uintptr_t)z | (uintptr_t)y) % 16 == 0, FD_ERR_ARG,
+             "%s: tensors must be 16-byte aligned", what);
+  int dev = 0, sms = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const CvCall c{(const bf16*)x, N, H, W, Cin, (const bf16*)w, bias, Cout, act, (bf16*)z, (bf16*)y, fd::as_stream(stream), sms};
+  return Cin % 32 == 0 ? rows_n<32>(c) : rows_n<16>(c);
+}
+
+}  // namespace
+
+int conv_error_word(unsigned* out, bool clear) { return tc_error_word(out, clear); }
+
+}  // namespace sg
+
+extern "C" {
+
+int sg_conv3x3_tma(const void* x, int N, int H, int W, int Cin, const void* w, const float* bias, int Cout,
+                   int act, void* z, void* y, void* stream) {
+  return sg::conv_rows(x, N, H, W, Cin, w, bias, Cout, act, z, y, stream, "sg_conv3x3_tma");
+}
+
+int sg_conv3x3_tma_ws(const void* x, int N, int H, int W, int Cin, const void* w, const float* bias, int Cout,
+                      int act, void* z, void* y, void* stream) {
+  return sg::conv_rows(x, N, H, W, Cin, w, bias, Cout, act, z, y, stream, "sg_conv3x3_tma_ws");
+}
+
+}  // extern "C"

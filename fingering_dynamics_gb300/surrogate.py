@@ -87,10 +87,10 @@ class UNet:
                  conv: str = "auto"):
         """``conv`` selects the forward and data-gradient convolution kernel:
         "tcgen05" (fifth-generation tensor cores, accumulator in tensor
-        memory), "tma" (the same fed by tensor-map boxes from one thread;
-        images whose width is a multiple of 128, the others fall back to
-        "tcgen05"), "tma_ws" (its persistent warp-specialised form, same
-        shapes), "mma" (warp-level tensor-core instructions) or "auto" (all
+        memory), "tma" (the same as a persistent kernel fed by tensor-map
+        boxes; images whose width is a multiple of 128, the others fall back to
+        "tcgen05"), "tma_ws" (the same kernel),
+        "mma" (warp-level tensor-core instructions) or "auto" (all
         that take the shape timed once per convolution shape at first use, the
         fastest kept).  The weight gradient runs on the tcgen05 kernel at widths
         that are multiples of 128 for every choice but "mma" ("auto": the faster
@@ -183,6 +183,7 @@ class UNet:
 
     _KERNELS = {"mma": "sg_conv3x3", "tcgen05": "sg_conv3x3_tc", "tma": "sg_conv3x3_tma",
                 "tma_ws": "sg_conv3x3_tma_ws"}
+    _TIMED = ("mma", "tcgen05", "tma")  # "auto" times these ("tma_ws" names the kernel of "tma")
 
     @staticmethod
     def _takes(kernel, w, ci, co):
@@ -201,7 +202,8 @@ class UNet:
             fn = self.conv_choice[key]
         else:  # time each kernel that takes the shape once on the real operands; the last call's result stands
             best = None
-            for k, fn in self._KERNELS.items():
+            for k in self._TIMED:
+                fn = self._KERNELS[k]
                 if not self._takes(k, w, ci, co):
                     continue
                 L.call(fn, *args)

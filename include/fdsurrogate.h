@@ -39,18 +39,16 @@ int sg_conv3x3_tc(const void* x, int N, int H, int W, int Cin, const void* w, co
                   void* z, void* y, void* stream);
 int sg_tc_status(unsigned* out, int clear);
 
-/* sg_conv3x3_tc fed by the tensor memory accelerator: one thread loads the
- * operands as tensor-map boxes (zero fill outside the image = the padding) into
- * a ring of stages and issues the MMAs as each lands.  Same arguments and
- * results; needs W a multiple of 128 and Cin, Cout multiples of 16
- * (FD_ERR_SHAPE otherwise).  Its waits share sg_tc_status's error word. */
+/* sg_conv3x3_tc as a persistent kernel fed by the tensor memory accelerator:
+ * one warp loads the operands as swizzled tensor-map boxes (zero fill outside
+ * the image = the padding) into a ring of stages, one issues the MMAs as each
+ * lands into one of two accumulator buffers, eight finish the previous tile.
+ * Same arguments and results; needs W a multiple of 128 and Cin, Cout multiples
+ * of 16 (FD_ERR_SHAPE otherwise).  Its waits share sg_tc_status's error word. */
 int sg_conv3x3_tma(const void* x, int N, int H, int W, int Cin, const void* w, const float* bias, int Cout, int act,
                    void* z, void* y, void* stream);
 
-/* sg_conv3x3_tma as a persistent kernel with warp-specialised roles: one
- * thread issues the boxes and MMAs of the CTA's tiles through one ring, two
- * accumulator buffers in tensor memory let four epilogue warps finish a tile
- * while the next one is multiplied.  Same arguments, results and shape rule. */
+/* The same kernel under the name of what was its persistent form. */
 int sg_conv3x3_tma_ws(const void* x, int N, int H, int W, int Cin, const void* w, const float* bias, int Cout,
                       int act, void* z, void* y, void* stream);
 
