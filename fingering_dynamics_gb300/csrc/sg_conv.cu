@@ -34,6 +34,32 @@ namespace {
 constexpr int kCvEpiWarps = 8;
 constexpr int kCvThreads = 32 * (kCvEpiWarps + 2);
 
+// Bias, activation and stores of 16 output channels of one pixel (element offset o).
+__device__ __forceinline__ void cv_store16(const float (&v)[16], const float* sbias, int act, bf16* __restrict__ z,
+                                           bf16* __restrict__ y, size_t o) {
+  uint32_t zw[8], yw[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    float t0 = v[2 * k] + sbias[2 * k], t1 = v[2 * k + 1] + sbias[2 * k + 1];
+    const __nv_bfloat162 zp = __floats2bfloat162_rn(t0, t1);
+    zw[k] = *reinterpret_cast<const uint32_t*>(&zp);
+    if (act == SG_ACT_GELU) {
+      t0 = gelu_f(t0);
+      t1 = gelu_f(t1);
+    }
+    const __nv_bfloat162 yp = __floats2bfloat162_rn(t0, t1);
+    yw[k] = *reinterpret_cast<const uint32_t*>(&yp);
+  }
+  if (z) {
+    reinterpret_cast<uint4*>(z + o)[0] = make_uint4(zw[0], zw[1], zw[2], zw[3]);
+    reinterpret_cast<uint4*>(z + o)[1] = make_uint4(zw[4], zw[5], zw[6], zw[7]);
+  }
+  if (y) {
+    reinterpret_cast<uint4*>(y + o)[0] = make_uint4(yw[0], yw[1], yw[2], yw[3]);
+    reinterpret_cast<uint4*>(y + o)[1] = make_uint4(yw[4], yw[5], yw[6], yw[7]);
+  }
+}
+
 template <int BN, int R, int CH>
 struct CvCfg {
   static constexpr int ROW = CH * 2;                                        // bytes of a pixel or output channel
@@ -191,27 +217,7 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_rows(const __grid_con
         float v[16];
         tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * R * BN + i * 16), v);
         const size_t o = ((size_t)(row + r) * sh.W + x0 + q * 32 + lane) * sh.Cout + co0 + c0;
-        uint32_t zw[8], yw[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          float t0 = v[2 * k] + sbias[c0 + 2 * k], t1 = v[2 * k + 1] + sbias[c0 + 2 * k + 1];
-          const __nv_bfloat162 zp = __floats2bfloat162_rn(t0, t1);
-          zw[k] = *reinterpret_cast<const uint32_t*>(&zp);
-          if (sh.act == SG_ACT_GELU) {
-            t0 = gelu_f(t0);
-            t1 = gelu_f(t1);
-          }
-          const __nv_bfloat162 yp = __floats2bfloat162_rn(t0, t1);
-          yw[k] = *reinterpret_cast<const uint32_t*>(&yp);
-        }
-        if (z) {
-          reinterpret_cast<uint4*>(z + o)[0] = make_uint4(zw[0], zw[1], zw[2], zw[3]);
-          reinterpret_cast<uint4*>(z + o)[1] = make_uint4(zw[4], zw[5], zw[6], zw[7]);
-        }
-        if (y) {
-          reinterpret_cast<uint4*>(y + o)[0] = make_uint4(yw[0], yw[1], yw[2], yw[3]);
-          reinterpret_cast<uint4*>(y + o)[1] = make_uint4(yw[4], yw[5], yw[6], yw[7]);
-        }
+        cv_store16(v, sbias + c0, sh.act, z, y, o);
       }
       // this warp's reads of buffer b are complete (tcgen05.wait::ld in tmem_ld16)
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -226,18 +232,166 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_rows(const __grid_con
   }
 }
 
-// Tensor maps of one call: x as (C, W, H, N) with boxes of CH channels x 130
-// pixels x R + 2 rows, the weights [co][tap][ci] as (Cin, 9, Cout) with boxes of
+// ---------------------------------------------------------------------------
+// Narrow images (widths 8, 16, 32 and 64; sg_conv3x3_tc): a tile is 128 pixels,
+// 128 / W rows of one image.  A halo would not be 128 evenly spaced operand rows,
+// so a stage is one tap of a chunk of BK channels: a box of the tile's pixels
+// shifted by the tap (zeros outside the image), 128 rows of BK channels, and the
+// tap's weights.  K advances chunk by chunk, the nine taps of a chunk back to
+// back, 16 channels at a time within a tap, as in k_conv3x3_tc, which all threads
+// fed by 16-byte copies: at 32 x 32 x 64, us, 128 -> 256 channels 247 -> 50, 256 ->
+// 256 445 -> 71, 256 -> 128 255 -> 38 (the warp-level kernel 157, 283, 143); one image,
+// 256 -> 256, 48 -> 14.5 (25).
+// Same roles as k_conv3x3_rows.
+// ---------------------------------------------------------------------------
+template <int BN, int BK>
+struct CnCfg {
+  static constexpr int ROW = BK * 2;
+  static constexpr int A_BYTES = kTcBM * ROW, B_BYTES = (BN * ROW + 1023) / 1024 * 1024, STAGE = A_BYTES + B_BYTES;
+  static constexpr uint32_t TX = (uint32_t)(A_BYTES + BN * ROW);
+  static constexpr int COLS = 2 * BN < 32 ? 32 : 2 * BN;
+  static constexpr int S = 220 * 1024 / STAGE > 8 ? 8 : 220 * 1024 / STAGE;
+  static constexpr int OFF_BAR = S * STAGE;
+  static constexpr int SMEM = OFF_BAR + (2 * S + 4) * 8 + BN * 4 + 16 + 1024;
+  static_assert(A_BYTES % 1024 == 0 && SMEM <= 227 * 1024 && COLS <= 512, "tile");
+};
+
+template <int BN, int BK>
+__global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_narrow(const __grid_constant__ ConvMaps maps, const CvShape sh,
+                                                                 const float* __restrict__ bias, bf16* __restrict__ z,
+                                                                 bf16* __restrict__ y) {
+  using C = CnCfg<BN, BK>;
+  constexpr int S = C::S;
+  extern __shared__ char smem_raw[];
+  char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
+  uint64_t *empty = full + S, *accf = empty + S, *acce = accf + 2;
+  float* sbias = reinterpret_cast<float*>(acce + 2);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sbias + BN);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rows = kTcBM / sh.W, tiles_y = (sh.H + rows - 1) / rows, nco = sh.Cout / BN;
+  const int ntiles = sh.N * tiles_y * nco, nst = sh.nk * 9;  // stages of a tile
+  const int mine = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  const int co0 = ((int)blockIdx.x % nco) * BN;  // the grid is a multiple of the output-channel tiles
+
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(C::COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (tid == 0) {
+    for (int i = 0; i < 2 * S + 2; ++i) mbar_init(&full[i]);
+    for (int i = 0; i < 2; ++i)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&acce[i])), "n"(kCvEpiWarps) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  for (int i = tid; i < BN; i += kCvThreads) sbias[i] = bias ? bias[co0 + i] : 0.0f;
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  // tile j of this CTA -> image n, first row y0
+  auto tile_of = [&](int j, int& n, int& y0) {
+    const int pt = ((int)blockIdx.x + j * (int)gridDim.x) / nco;
+    n = pt / tiles_y;
+    y0 = (pt % tiles_y) * rows;
+  };
+
+  if (warp == kCvEpiWarps) {
+    if (lane == 0 && mine > 0) {
+      int c = 0;
+      bool ok = true;
+      for (int j = 0; j < mine && ok; ++j) {
+        int n, y0;
+        tile_of(j, n, y0);
+        for (int k = 0; k < nst; ++k, ++c) {
+          const int st = c % S, kc = k / 9, tap = k % 9;
+          if (c >= S) ok = mbar_wait_ok(&empty[st], (unsigned)(c / S - 1) & 1u, true);
+          if (!ok) break;
+          char* a = smem + st * C::STAGE;
+          mbar_expect_tx(&full[st], C::TX);
+          tma_load_4d(a, &maps.x, kc * BK, tap % 3 - 1, y0 + tap / 3 - 1, n, &full[st]);
+          tma_load_3d(a + C::A_BYTES, &maps.w, kc * BK, tap, co0, &full[st]);
+        }
+      }
+      for (int i = 0; i < S && i < c; ++i)
+        mbar_wait_ok(&full[i], (unsigned)((c - 1 - ((c - 1 - i) % S)) / S) & 1u, false);
+    }
+    __syncwarp();
+  } else if (warp == kCvEpiWarps + 1) {
+    uint32_t leader;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(leader));
+    constexpr uint32_t idesc = instr_desc<kTcBM, BN>();
+    const uint64_t a0 = smem_desc_sw<C::ROW>(smem_u32(smem), 16, 8 * C::ROW);
+    const uint64_t w0 = smem_desc_sw<C::ROW>(smem_u32(smem + C::A_BYTES), 16, 8 * C::ROW);
+    bool ok = true;
+    int c = 0;
+    for (int j = 0; j < mine && ok; ++j) {
+      const int b = j & 1;
+      if (j >= 2) ok = mbar_wait_ok(&acce[b], (unsigned)((j - 2) >> 1) & 1u, true);
+      for (int k = 0; k < nst && ok; ++k, ++c) {
+        const int st = c % S;
+        ok = mbar_wait_ok(&full[st], (unsigned)(c / S) & 1u, true);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint64_t off = (uint64_t)(st * C::STAGE / 16);
+        if (leader) {
+#pragma unroll
+          for (int s = 0; s < BK / 16; ++s)
+            tc_mma(tmem + (uint32_t)(b * BN), a0 + off + (uint64_t)(s * 2), w0 + off + (uint64_t)(s * 2), idesc,
+                   s > 0 ? 1u : (k > 0 ? 1u : 0u));
+          tc_commit(&empty[st]);
+          if (k == nst - 1) tc_commit(&accf[b]);
+        }
+        __syncwarp();
+      }
+    }
+    for (int i = 0; i < S && i < c; ++i)
+      mbar_wait_ok(&empty[i], (unsigned)((c - 1 - ((c - 1 - i) % S)) / S) & 1u, false);
+  } else {
+    const int q = warp & 3, h = warp >> 2;
+    const int m = q * 32 + lane;  // pixel of the tile
+    for (int j = 0; j < mine; ++j) {
+      const int b = j & 1;
+      int n, y0;
+      tile_of(j, n, y0);
+      mbar_wait_ok(&accf[b], (unsigned)(j >> 1) & 1u, true);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int yy = y0 + m / sh.W;
+#pragma unroll 1
+      for (int i = h; i < BN / 16; i += 2) {
+        float v[16];
+        tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + i * 16), v);
+        if (yy < sh.H)
+          cv_store16(v, sbias + i * 16, sh.act, z, y,
+                     (((size_t)n * sh.H + yy) * sh.W + m % sh.W) * sh.Cout + co0 + i * 16);
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acce[b])) : "memory");
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C::COLS) : "memory");
+  }
+}
+
+// Tensor maps of one call: x as (C, W, H, N) with boxes of CH channels x box_w
+// pixels x box_h rows, the weights [co][tap][ci] as (Cin, 9, Cout) with boxes of
 // CH channels x 1 tap x BN output channels.
 inline int encode_conv_maps(ConvMaps& m, const bf16* x, int N, int H, int W, int Cin, const bf16* w, int Cout,
-                            int R, int BN, int CH) {
+                            int box_w, int box_h, int BN, int CH) {
   const fd::EncodeTiledFn fn = fd::encode_tiled_fn();
   FD_REQUIRE(fn != nullptr, FD_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-  const CUtensorMapSwizzle sw = CH == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
+  const CUtensorMapSwizzle sw = CH == 64 ? CU_TENSOR_MAP_SWIZZLE_128B
+                                         : (CH == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
   const cuuint64_t es = 2;
   const cuuint64_t xd[4] = {(cuuint64_t)Cin, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
   const cuuint64_t xs[3] = {Cin * es, (cuuint64_t)W * Cin * es, (cuuint64_t)H * W * Cin * es};
-  const cuuint32_t xb[4] = {(cuuint32_t)CH, (cuuint32_t)kHaloPx, (cuuint32_t)(R + 2), 1u};
+  const cuuint32_t xb[4] = {(cuuint32_t)CH, (cuuint32_t)box_w, (cuuint32_t)box_h, 1u};
   const cuuint32_t e4[4] = {1u, 1u, 1u, 1u};
   CUresult r = fn(&m.x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(x), xd, xs, xb, e4,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -285,7 +439,7 @@ int launch_rows(const CvCall& c) {
   const long long ntiles = (long long)c.N * (c.H / R) * (c.W / kTcBM) * nco;
   const long long grid = std::min<long long>(ntiles, std::max(1, c.sms / nco) * (long long)nco);
   ConvMaps maps;
-  if (int r = encode_conv_maps(maps, c.x, c.N, c.H, c.W, c.Cin, c.w, c.Cout, R, BN, CH)) return r;
+  if (int r = encode_conv_maps(maps, c.x, c.N, c.H, c.W, c.Cin, c.w, c.Cout, kHaloPx, R + 2, BN, CH)) return r;
   kern<<<(unsigned)grid, kCvThreads, 227 * 1024, c.s>>>(maps, sh, c.b, c.z, c.y);
   return fd::check_launch("sg_conv3x3_tma");
 }
@@ -313,6 +467,40 @@ int rows_n(const CvCall& c) {
   return rows_r<16, CH>(c);
 }
 
+template <int BN, int BK>
+int launch_narrow(const CvCall& c) {
+  using C = CnCfg<BN, BK>;
+  auto kern = k_conv3x3_narrow<BN, BK>;
+  static std::atomic<unsigned long long> attr_done{0};
+  if (fd::ensure_smem_attr(kern, 227 * 1024, attr_done) != cudaSuccess)
+    return fd::check_launch("sg_conv3x3_tc: shared-memory attribute");
+  const int rows = kTcBM / c.W, nco = c.Cout / BN;
+  const CvShape sh{c.N, c.H, c.W, c.Cin, c.Cout, c.act, c.Cin / BK, C::S, 0};
+  const long long ntiles = (long long)c.N * ((c.H + rows - 1) / rows) * nco;
+  const long long grid = std::min<long long>(ntiles, std::max(1, c.sms / nco) * (long long)nco);
+  ConvMaps maps;
+  if (int r = encode_conv_maps(maps, c.x, c.N, c.H, c.W, c.Cin, c.w, c.Cout, c.W, rows, BN, BK)) return r;
+  kern<<<(unsigned)grid, kCvThreads, 227 * 1024, c.s>>>(maps, sh, c.b, c.z, c.y);
+  return fd::check_launch("sg_conv3x3_tc");
+}
+
+// Output channels per tile: 128 where the tiles still give every SM one, else 64
+// (a batch of one at 32 x 64 has 16 tiles of pixels).
+template <int BK>
+int narrow_n(const CvCall& c) {
+  const long long px_tiles = (long long)c.N * ((c.H + kTcBM / c.W - 1) / (kTcBM / c.W));
+  if (c.Cout % 128 == 0 && px_tiles * (c.Cout / 128) >= c.sms) return launch_narrow<128, BK>(c);
+  if (c.Cout % 64 == 0 && px_tiles * (c.Cout / 64) >= c.sms / 2) return launch_narrow<64, BK>(c);
+  if (c.Cout % 32 == 0) return launch_narrow<32, BK>(c);
+  return launch_narrow<16, BK>(c);
+}
+
+void set_sms(CvCall& c) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&c.sms, cudaDevAttrMultiProcessorCount, dev);
+}
+
 int conv_rows(const void* x, int N, int H, int W, int Cin, const void* w, const float* bias, int Cout, int act, void* z,
               void* y, void* stream, const char* what) {
   FD_REQUIRE(x && w && (z || y) && N > 0 && H > 0 && W > 0, FD_ERR_ARG, "%s: bad arguments", what);
@@ -321,16 +509,23 @@ int conv_rows(const void* x, int N, int H, int W, int Cin, const void* w, const 
   FD_REQUIRE(act == SG_ACT_NONE || act == SG_ACT_GELU, FD_ERR_ARG, "%s: activation %d", what, act);
   FD_REQUIRE(((uintptr_t)x | (uintptr_t)w | (uintptr_t)z | (uintptr_t)y) % 16 == 0, FD_ERR_ARG,
              "%s: tensors must be 16-byte aligned", what);
-  int dev = 0, sms = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const CvCall c{(const bf16*)x, N, H, W, Cin, (const bf16*)w, bias, Cout, act, (bf16*)z, (bf16*)y, fd::as_stream(stream), sms};
+  CvCall c{(const bf16*)x, N, H, W, Cin, (const bf16*)w, bias, Cout, act, (bf16*)z, (bf16*)y, fd::as_stream(stream), 1};
+  set_sms(c);
   return Cin % 32 == 0 ? rows_n<32>(c) : rows_n<16>(c);
 }
 
 }  // namespace
 
 int conv_error_word(unsigned* out, bool clear) { return tc_error_word(out, clear); }
+
+// sg_conv3x3_tc on the widths that divide 128 (arguments checked by the caller).
+int conv_narrow(const void* x, int N, int H, int W, int Cin, const void* w, const float* bias, int Cout, int act, void* z,
+                void* y, cudaStream_t s) {
+  CvCall c{(const bf16*)x, N, H, W, Cin, (const bf16*)w, bias, Cout, act, (bf16*)z, (bf16*)y, s, 1};
+  set_sms(c);
+  if (Cin % 64 == 0) return narrow_n<64>(c);
+  return Cin % 32 == 0 ? narrow_n<32>(c) : narrow_n<16>(c);
+}
 
 }  // namespace sg
 

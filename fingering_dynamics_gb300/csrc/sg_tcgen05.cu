@@ -23,6 +23,8 @@ namespace sg {
 
 int conv_error_word(unsigned* out, bool clear);
 int wgrad_error_word(unsigned* out, bool clear);
+int conv_narrow(const void* x, int N, int H, int W, int Cin, const void* w, const float* bias, int Cout, int act, void* z,
+                void* y, cudaStream_t s);
 
 namespace {
 
@@ -428,6 +430,7 @@ int sg_conv3x3_tc(const void* x, int N, int H, int W, int Cin, const void* w, co
     if (Cout % 32 == 0) return sg::launch_tch<32, 16>(xb, N, H, W, Cin, wb, bias, Cout, act, zb, yb, s);
     return sg::launch_tch<16, 16>(xb, N, H, W, Cin, wb, bias, Cout, act, zb, yb, s);
   }
+  if (W >= 8 && sg::kTcBM % W == 0) return sg::conv_narrow(x, N, H, W, Cin, w, bias, Cout, act, z, y, s);
   if (Cin % 64 == 0) return sg::tc_bk<64>(xb, N, H, W, Cin, wb, bias, Cout, act, (bf16*)z, (bf16*)y, s);
   if (Cin % 32 == 0) return sg::tc_bk<32>(xb, N, H, W, Cin, wb, bias, Cout, act, (bf16*)z, (bf16*)y, s);
   return sg::tc_bk<16>(xb, N, H, W, Cin, wb, bias, Cout, act, (bf16*)z, (bf16*)y, s);
