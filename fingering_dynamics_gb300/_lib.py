@@ -61,6 +61,11 @@ class fd_instance(C.Structure):
                 ("pop_b", C.c_void_p), ("side_a", C.c_void_p), ("side_b", C.c_void_p), ("seed", C.c_uint32)]
 
 
+class sg_adamw_item(C.Structure):
+    _fields_ = [("w", C.c_void_p), ("w16", C.c_void_p), ("g", C.c_void_p), ("m", C.c_void_p), ("v", C.c_void_p),
+                ("n", C.c_size_t), ("weight_decay", C.c_float)]
+
+
 class fd_fields(C.Structure):
     _fields_ = [(n, C.c_void_p) for n in ("f", "g", "psi", "npx", "npy", "np2", "rho", "ux", "uy", "p", "mu",
                                           "mix_tau")]
@@ -133,6 +138,13 @@ SIGNATURES = {
     "sg_masked_mse": [_VP, _VP, _VP, _SZ, _I, _VP, _VP, _FL, _VP],
     "sg_loss_blocks": [],
     "sg_adamw": [_VP, _VP, _VP, _VP, _VP, _SZ, _FL, _FL, _FL, _FL, _FL, _I, _VP],
+    "sg_adamw_list": [_VP, _I, _FL, _FL, _FL, _FL, _I, _VP],
+    "sg_gelu_bias_bwd": [_I, _VP, _VP, _I, _I, _I, _I, _I, _VP, _I, _VP, _VP, _VP, _VP],
+    "sg_up2_concat": [_VP, _I, _I, _I, _I, _VP, _I, _VP, _VP],
+    "sg_loss_scale": [_VP, _SZ, _I, _VP, _VP, _VP],
+    "sg_masked_mse_scaled": [_VP, _VP, _VP, _SZ, _I, _VP, _VP, _VP, _VP],
+    "sg_add_prediction": [_VP, _VP, _SZ, _I, _VP, _VP],
+    "sg_run": [_VP, _I, _VP],
     "sg_to_bf16": [_VP, _SZ, _VP, _VP],
 }
 _RET = {"fd_last_error": C.c_char_p, "fd_packed_bytes": C.c_size_t, "fd_diag_scratch_bytes": C.c_size_t,

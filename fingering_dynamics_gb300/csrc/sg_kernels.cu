@@ -389,11 +389,23 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(const bf16* __restrict__ x, 
     }
 }
 
+// Sums over the splits in order, 32 loads in flight at a time: the bias sums are a
+// few warps adding 512 partials each, so their time is the loads' latency (19 us
+// with a load per addition, 16.5 with eight in flight).
 __global__ void k_sum_partials(const float* __restrict__ partial, int splits, size_t n, float* __restrict__ out) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
+  const float* p = partial + i;
   float s = 0.0f;
-  for (int k = 0; k < splits; ++k) s += partial[(size_t)k * n + i];
+  int k = 0;
+  for (; k + 32 <= splits; k += 32, p += 32 * n) {
+    float v[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = __ldg(p + j * n);
+#pragma unroll
+    for (int j = 0; j < 32; ++j) s += v[j];
+  }
+  for (; k < splits; ++k, p += n) s += __ldg(p);
   out[i] = s;
 }
 
@@ -473,6 +485,8 @@ __global__ void k_gelu_bwd(const bf16* __restrict__ dy, const bf16* __restrict__
   st8(dz + 8 * i, a);
 }
 
+constexpr size_t kIndex32 = (size_t)1 << 31;  // element groups that 32-bit indexes count
+
 constexpr int kBiasBlocks = 512;
 constexpr int kBiasThreads = 256;
 
@@ -505,21 +519,107 @@ __global__ void __launch_bounds__(kBiasThreads) k_bias_partial(const bf16* __res
   }
 }
 
-// 8 channels per thread: i indexes (output pixel, channel group)
-__global__ void k_pool2(const bf16* __restrict__ x, int N, int H, int W, int C, bf16* __restrict__ y) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int h = H / 2, w = W / 2, cg = C / 8;
-  const size_t n_out = (size_t)N * h * w * cg;
+// Where the gradient dy of a layer's output comes from.
+enum DySource {
+  kDyPlain = 0,  // a tensor
+  kDyUp = 1,     // the 2x upsampling's backward: channels [coff, coff + C) of the four pixels of a (N, 2H, 2W, Cy) tensor
+  kDyPool = 2    // the 2x2 mean's backward plus the skip connection's channels [coff, coff + C) of a (N, H, W, Cy) tensor
+};
+
+// dz = bf16(dy) GELU'(z) and the per-block channel sums of dz, in one pass: the
+// blocks, threads and order of k_bias_partial, so the sums are those of a pass of
+// its own over dz.  dy is rounded to bfloat16 between the operations, as when each
+// was a kernel that stored it.  As separate kernels (pool or upsampling backward,
+// skip addition, GELU backward, bias) a layer of 32 channels at 32 x 256 x 512 moved
+// up to 1.9 GB, in one pass 0.8.
+template <int SRC>
+__global__ void __launch_bounds__(kBiasThreads) k_gelu_bias_bwd(const bf16* __restrict__ a, const bf16* __restrict__ skip,
+                                                                unsigned H, unsigned W, int Cy, int coff,
+                                                                const bf16* __restrict__ z, size_t P, int C,
+                                                                bf16* __restrict__ dz, float* __restrict__ partial) {
+  __shared__ float s[kBiasThreads * 8];
+  const int vpp = C / 8, ppi = kBiasThreads / vpp;
+  const int lv = threadIdx.x % vpp, lp = threadIdx.x / vpp;
+  float acc[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+  auto dy_of = [&](size_t p) -> V8 {
+    if constexpr (SRC == kDyPlain) {
+      return ld8(a + p * C + 8 * lv);
+    } else {
+      const unsigned q = (unsigned)(p / W), x = (unsigned)(p - (size_t)q * W), n = q / H, y = q - n * H;
+      V8 r;
+      if constexpr (SRC == kDyUp) {
+        const size_t row = (size_t)2 * W * Cy;
+        const bf16* b = a + ((size_t)n * 2 * H + 2 * y) * row + (size_t)2 * x * Cy + coff + 8 * lv;
+        const V8 v0 = ld8(b), v1 = ld8(b + Cy), v2 = ld8(b + row), v3 = ld8(b + row + Cy);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) r.v[k] = (v0.v[k] + v1.v[k]) + (v2.v[k] + v3.v[k]);
+      } else {
+        const V8 d = ld8(a + (((size_t)n * (H / 2) + y / 2) * (W / 2) + x / 2) * C + 8 * lv);
+        const V8 k8 = ld8(skip + p * Cy + coff + 8 * lv);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) r.v[k] = __bfloat162float(__float2bfloat16_rn(d.v[k] * 0.25f)) + k8.v[k];
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) r.v[k] = __bfloat162float(__float2bfloat16_rn(r.v[k]));
+      return r;
+    }
+  };
+  if (lp < ppi) {
+    const size_t per = (P + gridDim.x - 1) / gridDim.x;
+    const size_t lo = (size_t)blockIdx.x * per, hi = min(P, lo + per);
+#pragma unroll 2
+    for (size_t p = lo + lp; p < hi; p += ppi) {
+      V8 v = dy_of(p);
+      const V8 zz = ld8(z + p * C + 8 * lv);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v.v[k] *= gelu_grad_f(zz.v[k]);
+      st8(dz + p * C + 8 * lv, v);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) acc[k] += __bfloat162float(__float2bfloat16_rn(v.v[k]));
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) s[threadIdx.x * 8 + k] = acc[k];
+  __syncthreads();
+  for (int c = threadIdx.x; c < C; c += blockDim.x) {
+    const int v = c / 8, k = c % 8;
+    float t = 0.0f;
+    for (int q = 0; q < ppi; ++q) t += s[(q * vpp + v) * 8 + k];
+    partial[(size_t)blockIdx.x * C + c] = t;
+  }
+}
+
+// y = [nearest 2x upsampling of x (C channels), skip (Cs channels)] per pixel
+template <typename I>
+__global__ void k_up_concat(const bf16* __restrict__ x, I n_out, I H, I W, I cg, I csg, const bf16* __restrict__ skip,
+                            bf16* __restrict__ y) {
+  const I i = (I)blockIdx.x * blockDim.x + threadIdx.x;  // (output pixel, group of 8 channels)
   if (i >= n_out) return;
-  const int c = (int)(i % cg) * 8;
-  const size_t pix = i / cg;
-  const int xo = (int)(pix % w), yo = (int)((pix / w) % h), n = (int)(pix / ((size_t)w * h));
-  const size_t b = (((size_t)n * H + 2 * yo) * W + 2 * xo) * C + c;
-  const V8 a = ld8(x + b), bb = ld8(x + b + C), cc = ld8(x + b + (size_t)W * C), d = ld8(x + b + (size_t)W * C + C);
+  const I g = cg + csg, pix = i / g, c = i - pix * g;
+  uint4 v;
+  if (c < cg) {
+    const I q = pix / W, xx = pix - q * W, n = q / H, yy = q - n * H;
+    v = *reinterpret_cast<const uint4*>(x + (((size_t)n * (H / 2) + yy / 2) * (W / 2) + xx / 2) * cg * 8 + (size_t)c * 8);
+  } else {
+    v = *reinterpret_cast<const uint4*>(skip + (size_t)pix * csg * 8 + (size_t)(c - cg) * 8);
+  }
+  *reinterpret_cast<uint4*>(y + (size_t)i * 8) = v;
+}
+
+// 8 channels per thread: i indexes (output pixel, channel group)
+// (32-bit indexes where they suffice: 64-bit divisions cost more than the loads)
+template <typename I>
+__global__ void k_pool2(const bf16* __restrict__ x, I n_out, I h, I w, I cg, bf16* __restrict__ y) {
+  const I i = (I)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_out) return;
+  const I pix = i / cg, c = (i - pix * cg) * 8, q = pix / w, xo = pix - q * w, n = q / h, yo = q - n * h;
+  const size_t C = (size_t)cg * 8, W = (size_t)2 * w;
+  const size_t b = (((size_t)n * 2 * h + 2 * yo) * W + 2 * xo) * C + c;
+  const V8 a = ld8(x + b), bb = ld8(x + b + C), cc = ld8(x + b + W * C), d = ld8(x + b + W * C + C);
   V8 r;
 #pragma unroll
   for (int k = 0; k < 8; ++k) r.v[k] = 0.25f * ((a.v[k] + bb.v[k]) + (cc.v[k] + d.v[k]));
-  st8(y + pix * C + c, r);
+  st8(y + (size_t)pix * C + c, r);
 }
 
 __global__ void k_pool2_bwd(const bf16* __restrict__ dy, int N, int H, int W, int C, bf16* __restrict__ dx) {
@@ -592,21 +692,60 @@ __global__ void k_add_ch(const bf16* __restrict__ src, size_t P, int Cs, int cof
 
 constexpr int kLossBlocks = 512;
 
+// Fluid pixels of a batch of frames, and the two scales of its loss: inv[0] = 1 /
+// (3 count) for the gradient, inv[1] the same through single precision for the sum.
+__global__ void k_count_fluid(const bf16* __restrict__ x, size_t P, int C, unsigned* __restrict__ count) {
+  unsigned n = 0;
+  for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < P; p += (size_t)gridDim.x * blockDim.x)
+    n += __bfloat162float(x[p * C + 3]) == 0.0f ? 1u : 0u;
+  n = __reduce_add_sync(0xffffffffu, n);
+  if ((threadIdx.x & 31) == 0 && n) atomicAdd(count, n);
+}
+__global__ void k_loss_scale(const unsigned* __restrict__ count, float* __restrict__ inv) {
+  const double n = 3.0 * (double)(*count > 0u ? *count : 1u);
+  inv[0] = (float)(1.0 / n);
+  inv[1] = __frcp_rn((float)n);
+}
+
+// `dev_inv`: the gradient's scale in device memory, or NULL (inv_count).  Frames of
+// 16 channels move as vectors: the live channels of a pixel in one load, its 32
+// bytes of dout in two stores (409 us with a load and a store per channel at 32 x
+// 256 x 512, 79 as vectors).
 __global__ void k_masked_mse(const bf16* __restrict__ x, const bf16* __restrict__ out, const bf16* __restrict__ xn,
-                             size_t P, int C, bf16* __restrict__ dout, float* __restrict__ partial, float inv_count) {
+                             size_t P, int C, bf16* __restrict__ dout, float* __restrict__ partial, float inv_count,
+                             const float* __restrict__ dev_inv) {
   __shared__ float s_e[kEw], s_n[kEw];
   float e = 0.0f, nf = 0.0f;
+  const float inv = dev_inv ? *dev_inv : inv_count;
+  const bool vec = C == 16 && (((uintptr_t)x | (uintptr_t)out | (uintptr_t)xn | (uintptr_t)dout) & 15) == 0;
   for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < P; p += (size_t)gridDim.x * blockDim.x) {
     const size_t b = p * C;
-    const bool fluid = __bfloat162float(x[b + 3]) == 0.0f;
-    for (int c = 0; c < C; ++c) {
-      float g = 0.0f;
+    bf16 xv[4], ov[4], nv[4], g[4];
+    if (vec) {
+      *reinterpret_cast<uint2*>(xv) = *reinterpret_cast<const uint2*>(x + b);
+      *reinterpret_cast<uint2*>(ov) = *reinterpret_cast<const uint2*>(out + b);
+      *reinterpret_cast<uint2*>(nv) = *reinterpret_cast<const uint2*>(xn + b);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) { xv[c] = x[b + c]; ov[c] = out[b + c]; nv[c] = xn[b + c]; }
+    }
+    const bool fluid = __bfloat162float(xv[3]) == 0.0f;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      float gr = 0.0f;
       if (c < 3 && fluid) {
-        const float d = (__bfloat162float(x[b + c]) + __bfloat162float(out[b + c])) - __bfloat162float(xn[b + c]);
+        const float d = (__bfloat162float(xv[c]) + __bfloat162float(ov[c])) - __bfloat162float(nv[c]);
         e += d * d;
-        g = 2.0f * d * inv_count;
+        gr = 2.0f * d * inv;
       }
-      dout[b + c] = __float2bfloat16_rn(g);
+      g[c] = __float2bfloat16_rn(gr);
+    }
+    if (vec) {
+      const uint2 lo = *reinterpret_cast<const uint2*>(g);
+      reinterpret_cast<uint4*>(dout + b)[0] = make_uint4(lo.x, lo.y, 0u, 0u);
+      reinterpret_cast<uint4*>(dout + b)[1] = make_uint4(0u, 0u, 0u, 0u);
+    } else {
+      for (int c = 0; c < C; ++c) dout[b + c] = c < 4 ? g[c] : __float2bfloat16_rn(0.0f);
     }
     nf += fluid ? 1.0f : 0.0f;
   }
@@ -626,6 +765,23 @@ __global__ void k_masked_mse(const bf16* __restrict__ x, const bf16* __restrict_
   }
 }
 
+// y = x with its first three channels replaced by bf16(x + out)
+__global__ void k_add_prediction(const bf16* __restrict__ x, const bf16* __restrict__ out, size_t P, int C,
+                                 bf16* __restrict__ y) {
+  const int cg = C / 8;
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= P * cg) return;
+  uint4 v = *reinterpret_cast<const uint4*>(x + 8 * i);
+  if (cg == 1 || i % cg == 0) {
+    bf16* h = reinterpret_cast<bf16*>(&v);
+    const uint2 o = *reinterpret_cast<const uint2*>(out + 8 * i);
+    const bf16* oh = reinterpret_cast<const bf16*>(&o);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) h[c] = __float2bfloat16_rn(__bfloat162float(h[c]) + __bfloat162float(oh[c]));
+  }
+  *reinterpret_cast<uint4*>(y + 8 * i) = v;
+}
+
 __global__ void k_adamw(float* __restrict__ w, bf16* __restrict__ w16, const float* __restrict__ g,
                         float* __restrict__ m, float* __restrict__ v, size_t n, float lr, float b1, float b2, float eps,
                         float wd, float c1, float c2) {
@@ -639,6 +795,31 @@ __global__ void k_adamw(float* __restrict__ w, bf16* __restrict__ w16, const flo
   const float wi = w[i] - lr * ((mi * c1) / (sqrtf(vi * c2) + eps) + wd * w[i]);
   w[i] = wi;
   if (w16) w16[i] = __float2bfloat16_rn(wi);
+}
+
+// The same over a list of tensors, one launch: block b works on the tensor whose
+// block range holds it (30 launches a training step, most of a few hundred
+// elements, before).
+struct AdamwList {
+  sg_adamw_item item[SG_ADAMW_MAX];
+  unsigned first[SG_ADAMW_MAX + 1];  // first block of each tensor
+  int n;
+};
+__global__ void __launch_bounds__(kEw) k_adamw_list(const __grid_constant__ AdamwList L, float lr, float b1, float b2,
+                                                    float eps, float c1, float c2) {
+  int t = 0;
+  while (blockIdx.x >= L.first[t + 1]) ++t;
+  const sg_adamw_item& a = L.item[t];
+  const size_t i = (size_t)(blockIdx.x - L.first[t]) * kEw + threadIdx.x;
+  if (i >= a.n) return;
+  const float gi = a.g[i];
+  const float mi = fmaf(b1, a.m[i], (1.0f - b1) * gi);
+  const float vi = fmaf(b2, a.v[i], (1.0f - b2) * gi * gi);
+  a.m[i] = mi;
+  a.v[i] = vi;
+  const float wi = a.w[i] - lr * ((mi * c1) / (sqrtf(vi * c2) + eps) + a.weight_decay * a.w[i]);
+  a.w[i] = wi;
+  if (a.w16) reinterpret_cast<bf16*>(a.w16)[i] = __float2bfloat16_rn(wi);
 }
 
 __global__ void k_to_bf16(const float* __restrict__ src, size_t n, bf16* __restrict__ dst) {
@@ -737,7 +918,11 @@ int sg_gelu_bwd(const void* dy, const void* z, size_t n, void* dz, void* stream)
 int sg_pool2(const void* x, int N, int H, int W, int C, void* y, void* stream) {
   FD_REQUIRE(x && y && H % 2 == 0 && W % 2 == 0 && C % 8 == 0, FD_ERR_ARG, "sg_pool2: bad arguments");
   const size_t n = (size_t)N * (H / 2) * (W / 2) * (C / 8);
-  k_pool2<<<ew_blocks(n), kEw, 0, as_stream(stream)>>>((const bf16*)x, N, H, W, C, (bf16*)y);
+  cudaStream_t s = as_stream(stream);
+  if (n < kIndex32)
+    k_pool2<uint32_t><<<ew_blocks(n), kEw, 0, s>>>((const bf16*)x, (uint32_t)n, H / 2, W / 2, C / 8, (bf16*)y);
+  else
+    k_pool2<size_t><<<ew_blocks(n), kEw, 0, s>>>((const bf16*)x, n, H / 2, W / 2, C / 8, (bf16*)y);
   return check_launch("sg_pool2");
 }
 
@@ -784,7 +969,7 @@ int sg_masked_mse(const void* x, const void* out, const void* xn, size_t P, int 
                   float inv_count, void* stream) {
   FD_REQUIRE(x && out && xn && dout && loss_partial && C >= 4, FD_ERR_ARG, "sg_masked_mse: bad arguments");
   k_masked_mse<<<kLossBlocks, kEw, 0, as_stream(stream)>>>((const bf16*)x, (const bf16*)out, (const bf16*)xn, P, C,
-                                                          (bf16*)dout, loss_partial, inv_count);
+                                                          (bf16*)dout, loss_partial, inv_count, nullptr);
   return check_launch("sg_masked_mse");
 }
 
@@ -798,10 +983,130 @@ int sg_adamw(float* w, void* w16, const float* g, float* m, float* v, size_t n, 
   return check_launch("sg_adamw");
 }
 
+int sg_adamw_list(const sg_adamw_item* items, int count, float lr, float beta1, float beta2, float eps, int step,
+                  void* stream) {
+  FD_REQUIRE(items && count > 0 && count <= SG_ADAMW_MAX && step >= 1, FD_ERR_ARG, "sg_adamw_list: bad arguments");
+  AdamwList L;
+  L.n = count;
+  L.first[0] = 0;
+  for (int i = 0; i < count; ++i) {
+    const sg_adamw_item& a = items[i];
+    FD_REQUIRE(a.w && a.g && a.m && a.v && a.n > 0, FD_ERR_ARG, "sg_adamw_list: tensor %d", i);
+    L.item[i] = a;
+    L.first[i + 1] = L.first[i] + ew_blocks(a.n);
+  }
+  const float c1 = 1.0f / (1.0f - powf(beta1, (float)step));
+  const float c2 = 1.0f / (1.0f - powf(beta2, (float)step));
+  k_adamw_list<<<L.first[count], kEw, 0, as_stream(stream)>>>(L, lr, beta1, beta2, eps, c1, c2);
+  return check_launch("sg_adamw_list");
+}
+
+int sg_gelu_bias_bwd(int source, const void* dy, const void* skip, int N, int H, int W, int Cy, int coff, const void* z,
+                     int C, void* dz, float* db, float* partial, void* stream) {
+  FD_REQUIRE(source >= SG_DY_PLAIN && source <= SG_DY_POOL, FD_ERR_ARG, "sg_gelu_bias_bwd: source %d", source);
+  FD_REQUIRE(dy && z && dz && db && partial && N > 0 && H > 0 && W > 0 && C > 0 && C % 8 == 0 && C <= 8 * kBiasThreads,
+             FD_ERR_ARG, "sg_gelu_bias_bwd: bad arguments");
+  FD_REQUIRE(source == SG_DY_PLAIN || (coff >= 0 && coff % 8 == 0 && Cy % 8 == 0 && coff + C <= Cy), FD_ERR_ARG,
+             "sg_gelu_bias_bwd: channels [%d, %d) of %d", coff, coff + C, Cy);
+  FD_REQUIRE(source != SG_DY_POOL || (skip && H % 2 == 0 && W % 2 == 0), FD_ERR_ARG, "sg_gelu_bias_bwd: bad arguments");
+  const size_t P = (size_t)N * H * W;
+  cudaStream_t s = as_stream(stream);
+  const bf16 *a = (const bf16*)dy, *k = (const bf16*)skip, *zb = (const bf16*)z;
+  switch (source) {
+    case SG_DY_UP:
+      k_gelu_bias_bwd<kDyUp><<<kBiasBlocks, kBiasThreads, 0, s>>>(a, k, H, W, Cy, coff, zb, P, C, (bf16*)dz, partial);
+      break;
+    case SG_DY_POOL:
+      k_gelu_bias_bwd<kDyPool><<<kBiasBlocks, kBiasThreads, 0, s>>>(a, k, H, W, Cy, coff, zb, P, C, (bf16*)dz, partial);
+      break;
+    default:
+      k_gelu_bias_bwd<kDyPlain><<<kBiasBlocks, kBiasThreads, 0, s>>>(a, k, H, W, Cy, coff, zb, P, C, (bf16*)dz, partial);
+  }
+  k_sum_partials<<<ew_blocks((size_t)C), kEw, 0, s>>>(partial, kBiasBlocks, (size_t)C, db);
+  return check_launch("sg_gelu_bias_bwd");
+}
+
+int sg_up2_concat(const void* x, int N, int h, int w, int C, const void* skip, int Cs, void* y, void* stream) {
+  FD_REQUIRE(x && skip && y && N > 0 && h > 0 && w > 0 && C > 0 && Cs > 0 && C % 8 == 0 && Cs % 8 == 0, FD_ERR_ARG,
+             "sg_up2_concat: bad arguments");
+  const size_t n = (size_t)N * 4 * h * w * ((C + Cs) / 8);
+  cudaStream_t s = as_stream(stream);
+  if (n < kIndex32)
+    k_up_concat<uint32_t><<<ew_blocks(n), kEw, 0, s>>>((const bf16*)x, (uint32_t)n, 2 * h, 2 * w, C / 8, Cs / 8,
+                                                       (const bf16*)skip, (bf16*)y);
+  else
+    k_up_concat<size_t><<<ew_blocks(n), kEw, 0, s>>>((const bf16*)x, n, 2 * h, 2 * w, C / 8, Cs / 8, (const bf16*)skip,
+                                                     (bf16*)y);
+  return check_launch("sg_up2_concat");
+}
+
+int sg_loss_scale(const void* x, size_t P, int C, unsigned* count, float* inv, void* stream) {
+  FD_REQUIRE(x && count && inv && C >= 4 && P < ((size_t)1 << 32), FD_ERR_ARG, "sg_loss_scale: bad arguments");
+  cudaStream_t s = as_stream(stream);
+  if (cudaMemsetAsync(count, 0, sizeof(unsigned), s) != cudaSuccess) return check_launch("sg_loss_scale");
+  k_count_fluid<<<kLossBlocks, kEw, 0, s>>>((const bf16*)x, P, C, count);
+  k_loss_scale<<<1, 1, 0, s>>>(count, inv);
+  return check_launch("sg_loss_scale");
+}
+
+int sg_masked_mse_scaled(const void* x, const void* out, const void* xn, size_t P, int C, void* dout, float* loss_partial,
+                         const float* inv, void* stream) {
+  FD_REQUIRE(x && out && xn && dout && loss_partial && inv && C >= 4, FD_ERR_ARG, "sg_masked_mse_scaled: bad arguments");
+  k_masked_mse<<<kLossBlocks, kEw, 0, as_stream(stream)>>>((const bf16*)x, (const bf16*)out, (const bf16*)xn, P, C,
+                                                          (bf16*)dout, loss_partial, 0.0f, inv);
+  return check_launch("sg_masked_mse_scaled");
+}
+
+int sg_add_prediction(const void* x, const void* out, size_t P, int C, void* y, void* stream) {
+  FD_REQUIRE(x && out && y && C >= 8 && C % 8 == 0, FD_ERR_ARG, "sg_add_prediction: bad arguments");
+  if (P == 0) return FD_OK;
+  k_add_prediction<<<ew_blocks(P * (C / 8)), kEw, 0, as_stream(stream)>>>((const bf16*)x, (const bf16*)out, P, C,
+                                                                          (bf16*)y);
+  return check_launch("sg_add_prediction");
+}
+
 int sg_to_bf16(const float* src, size_t n, void* dst, void* stream) {
   FD_REQUIRE(src && dst, FD_ERR_ARG, "sg_to_bf16: NULL pointer");
   k_to_bf16<<<ew_blocks(n), kEw, 0, as_stream(stream)>>>(src, n, (bf16*)dst);
   return check_launch("sg_to_bf16");
+}
+
+int sg_run(const sg_op* ops, int count, void* stream) {
+  FD_REQUIRE(count >= 0 && (ops || count == 0), FD_ERR_ARG, "sg_run: bad arguments");
+  for (int k = 0; k < count; ++k) {
+    const sg_op& o = ops[k];
+    const int64_t* i = o.i;
+    auto n = [&](int j) { return (int)i[j]; };
+    auto p = [&](int j) { return reinterpret_cast<void*>((uintptr_t)o.p[j]); };
+    int r;
+    switch (o.kind) {
+      case SG_OP_CONV:
+      case SG_OP_CONV_TC:
+      case SG_OP_CONV_TMA: {
+        auto fn = o.kind == SG_OP_CONV ? sg_conv3x3 : (o.kind == SG_OP_CONV_TC ? sg_conv3x3_tc : sg_conv3x3_tma);
+        r = fn(p(0), n(0), n(1), n(2), n(3), p(1), (const float*)p(2), n(4), n(5), p(3), p(4), stream);
+        break;
+      }
+      case SG_OP_WGRAD:
+      case SG_OP_WGRAD_TC: {
+        auto fn = o.kind == SG_OP_WGRAD ? sg_conv3x3_wgrad : sg_conv3x3_wgrad_tc;
+        r = fn(p(0), p(1), n(0), n(1), n(2), n(3), n(4), (float*)p(2), (float*)p(3), (size_t)i[5], 0, stream);
+        break;
+      }
+      case SG_OP_POOL: r = sg_pool2(p(0), n(0), n(1), n(2), n(3), p(1), stream); break;
+      case SG_OP_UP_CONCAT: r = sg_up2_concat(p(0), n(0), n(1), n(2), n(3), p(1), n(4), p(2), stream); break;
+      case SG_OP_GELU_BIAS:
+        r = sg_gelu_bias_bwd(n(0), p(0), p(1), n(1), n(2), n(3), n(4), n(5), p(2), n(6), p(3), (float*)p(4), (float*)p(5),
+                             stream);
+        break;
+      case SG_OP_BIAS: r = sg_bias_grad(p(0), (size_t)i[0], n(1), (float*)p(1), (float*)p(2), stream); break;
+      case SG_OP_FLIP: r = sg_flip_weights(p(0), n(0), n(1), p(1), stream); break;
+      case SG_OP_ADD_PREDICTION: r = sg_add_prediction(p(0), p(1), (size_t)i[0], n(1), p(2), stream); break;
+      default: FD_REQUIRE(false, FD_ERR_ARG, "sg_run: unknown operation %d", (int)o.kind);
+    }
+    if (r != FD_OK) return r;
+  }
+  return FD_OK;
 }
 
 }  // extern "C"

@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_wgrad_tc(const __grid_constan
   }
 }
 
-// Sum of the splits' partials in order; eight loads are in flight while they are added.
+// Sum of the splits' partials in order; sixteen loads are in flight while they are added.
 __global__ void __launch_bounds__(64) k_wg_sum(const float* __restrict__ partial, int splits, size_t n,
                                                float* __restrict__ out) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -195,12 +195,12 @@ __global__ void __launch_bounds__(64) k_wg_sum(const float* __restrict__ partial
   const float* p = partial + i;
   float s = 0.0f;
   int k = 0;
-  for (; k + 8 <= splits; k += 8, p += 8 * n) {
-    float v[8];
+  for (; k + 16 <= splits; k += 16, p += 16 * n) {
+    float v[16];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = __ldg(p + j * n);
+    for (int j = 0; j < 16; ++j) v[j] = __ldg(p + j * n);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) s += v[j];
+    for (int j = 0; j < 16; ++j) s += v[j];
   }
   for (; k < splits; ++k, p += n) s += __ldg(p);
   out[i] = s;

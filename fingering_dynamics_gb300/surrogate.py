@@ -25,6 +25,7 @@ zero, so the untrained network predicts "no change" (persistence).
 """
 from __future__ import annotations
 
+import array
 import ctypes as C
 import math
 import time
@@ -125,6 +126,8 @@ class UNet:
         self.vb = {n: torch.zeros_like(t) for n, t in self.b.items()}
         self.steps = 0
         self._buf = {}
+        self._ops = []        # operations collected for the next sg_run
+        self._x, self._kept = None, False
         self._flipped = False
 
     @property
@@ -167,23 +170,44 @@ class UNet:
         for name, (ci, co) in self.shapes.items():
             B["z." + name] = t(level[name], co)
             B["y." + name] = t(level[name], co)
-            B["dy." + name] = t(level[name], co)
             B["dz." + name] = t(level[name], co)
             B["dx." + name] = t(level[name], ci)
         B["p1"], B["p2"], B["p3"] = t(2, c1), t(3, c2), t(4, c3)
         B["u3"], B["u2"], B["u1"] = t(3, c4 + c3), t(2, c3 + c2), t(1, c2 + c1)
-        B["de1"], B["de2"], B["de3"] = t(1, c1), t(2, c2), t(3, c3)
+        B["dy.out"] = t(1, self.shapes["out"][1])
         wp = max(L.lib().sg_wgrad_partial_floats(N, *lv[level[n]], ci, co) for n, (ci, co) in self.shapes.items())
         B["wpart"] = torch.empty(int(wp), dtype=torch.float32, device=dev)
         B["bpart"] = torch.empty(int(L.lib().sg_bias_partial_floats(max(c1, c2, c3, c4, FRAME_CHANNELS))),
                                  dtype=torch.float32, device=dev)
         B["lpart"] = torch.empty(2 * L.lib().sg_loss_blocks(), dtype=torch.float32, device=dev)
+        B["count"] = torch.zeros(1, dtype=torch.int32, device=dev)
+        B["inv"] = torch.zeros(2, dtype=torch.float32, device=dev)
         self._buf[key] = B
         return B
 
     _KERNELS = {"mma": "sg_conv3x3", "tcgen05": "sg_conv3x3_tc", "tma": "sg_conv3x3_tma",
                 "tma_ws": "sg_conv3x3_tma_ws"}
     _TIMED = ("mma", "tcgen05", "tma")  # "auto" times these ("tma_ws" names the kernel of "tma")
+    # operations of a pass (include/fdsurrogate.h sg_op_kind)
+    _OP = {"sg_conv3x3": 0, "sg_conv3x3_tc": 1, "sg_conv3x3_tma": 2, "sg_conv3x3_tma_ws": 2, "sg_conv3x3_wgrad": 3,
+           "sg_conv3x3_wgrad_tc": 4, "sg_pool2": 5, "sg_up2_concat": 6, "sg_gelu_bias_bwd": 7, "sg_bias_grad": 8,
+           "sg_flip_weights": 9, "sg_add_prediction": 10}
+
+    # A pass collects its operations and runs them in one call (sg_run): a call
+    # of each from Python costs about ten microseconds, more than its kernel on a
+    # batch of one.
+    def _op(self, fn, ints, tensors):
+        o = [0] * 16
+        o[0] = self._OP[fn]
+        o[1:1 + len(ints)] = ints
+        o[9:9 + len(tensors)] = [0 if t is None else t.data_ptr() for t in tensors]
+        self._ops.extend(o)
+
+    def _run_ops(self):
+        if self._ops:
+            ops = array.array("q", self._ops)
+            self._ops.clear()
+            L.call("sg_run", C.c_void_p(ops.buffer_info()[0]), len(ops) // 16, _s())
 
     @staticmethod
     def _takes(kernel, w, ci, co):
@@ -191,33 +215,35 @@ class UNet:
         multiples of 128, channel counts that are multiples of 16)."""
         return not kernel.startswith("tma") or (w % 128 == 0 and ci % 16 == 0 and co % 16 == 0)
 
-    def _run_conv(self, x, N, h, w, ci, wt, bias, co, act, z, y):
-        """One 3x3 convolution with the kernel chosen for its shape."""
-        key = (N, h, w, ci, co)
-        args = (_p(x), N, h, w, ci, _p(wt), _p(bias), co, act, _p(z), _p(y), _s())
-        if self.conv != "auto":
-            k = self.conv if self._takes(self.conv, w, ci, co) else "tcgen05"
-            fn = self._KERNELS[k]
-        elif key in self.conv_choice:
-            fn = self.conv_choice[key]
-        else:  # time each kernel that takes the shape once on the real operands; the last call's result stands
+    def _fastest(self, key, fns, call):
+        """The fastest of the calls, timed once per shape on the real operands
+        (after the pass's pending operations); kept in conv_choice."""
+        if key not in self.conv_choice:
+            self._run_ops()
             best = None
-            for k in self._TIMED:
-                fn = self._KERNELS[k]
-                if not self._takes(k, w, ci, co):
-                    continue
-                L.call(fn, *args)
+            for fn in fns:
+                call(fn)
                 e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
                 e0.record()
                 for _ in range(2):
-                    L.call(fn, *args)
+                    call(fn)
                 e1.record()
                 e1.synchronize()
                 t = e0.elapsed_time(e1)
                 if best is None or t < best[0]:
                     best = (t, fn)
-            fn = self.conv_choice[key] = best[1]
-        L.call(fn, *args)
+            self.conv_choice[key] = best[1]
+        return self.conv_choice[key]
+
+    def _run_conv(self, x, N, h, w, ci, wt, bias, co, act, z, y):
+        """One 3x3 convolution with the kernel chosen for its shape."""
+        if self.conv != "auto":
+            fn = self._KERNELS[self.conv if self._takes(self.conv, w, ci, co) else "tcgen05"]
+        else:
+            fns = [self._KERNELS[k] for k in self._TIMED if self._takes(k, w, ci, co)]
+            fn = self._fastest((N, h, w, ci, co), fns,
+                               lambda f: L.call(f, _p(x), N, h, w, ci, _p(wt), _p(bias), co, act, _p(z), _p(y), _s()))
+        self._op(fn, (N, h, w, ci, co, act), (x, wt, bias, z, y))
 
     _WGRAD = {"mma": "sg_conv3x3_wgrad", "tcgen05": "sg_conv3x3_wgrad_tc"}
 
@@ -226,136 +252,125 @@ class UNet:
         multiples of 128) or the warp-level one; with conv="auto" both are timed
         once per shape and the faster kept (their FP32 sums differ in the last
         bits only)."""
-        key = ("wgrad", N, h, w, ci, co)
-        args = (_p(inp), _p(dz), N, h, w, ci, co, _p(gw), _p(part), part.numel(), 0, _s())
         ok_tc = w % 128 == 0
         if self.conv == "mma" or not ok_tc:
             fn = self._WGRAD["mma"]
         elif self.conv != "auto":
             fn = self._WGRAD["tcgen05"]
-        elif key in self.conv_choice:
-            fn = self.conv_choice[key]
         else:
-            best = None
-            for fn in self._WGRAD.values():
-                L.call(fn, *args)
-                e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-                e0.record()
-                for _ in range(2):
-                    L.call(fn, *args)
-                e1.record()
-                e1.synchronize()
-                t = e0.elapsed_time(e1)
-                if best is None or t < best[0]:
-                    best = (t, fn)
-            fn = self.conv_choice[key] = best[1]
-        L.call(fn, *args)
+            fn = self._fastest(("wgrad", N, h, w, ci, co), list(self._WGRAD.values()),
+                               lambda f: L.call(f, _p(inp), _p(dz), N, h, w, ci, co, _p(gw), _p(part), part.numel(), 0,
+                                                _s()))
+        self._op(fn, (N, h, w, ci, co, part.numel()), (inp, dz, gw, part))
 
-    def _conv(self, name, x, B, act=True):
+    def _conv(self, name, x, B, act=True, keep=True):
         ci, co = self.shapes[name]
         N, h, w, c = x.shape
         assert c == ci, (name, c, ci)
         self._run_conv(x, N, h, w, ci, self.w16[name], self.b[name], co, 1 if act else 0,
-                       B["z." + name] if act else None, B["y." + name])
+                       B["z." + name] if act and keep else None, B["y." + name])
         return B["y." + name]
 
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
-        """x: (N, H, W, 16) bfloat16 frames -> out (N, H, W, 16) bfloat16 (the
-        prediction is x[..., :3] + out[..., :3])."""
+    def _pass(self, x, keep):
+        """The operations of a forward pass; ``keep``: store the pre-activations
+        that the backward pass reads."""
         N, H, W, _ = x.shape
         B = self._buffers(N, H, W)
         c1, c2, c3, c4 = self.widths
         lv = B["lv"]
-        s = _s()
-        self._x = x
-        e1 = self._conv("enc1b", self._conv("enc1a", x, B), B)
-        L.call("sg_pool2", _p(e1), N, H, W, c1, _p(B["p1"]), s)
-        e2 = self._conv("enc2b", self._conv("enc2a", B["p1"], B), B)
-        L.call("sg_pool2", _p(e2), N, *lv[2], c2, _p(B["p2"]), s)
-        e3 = self._conv("enc3b", self._conv("enc3a", B["p2"], B), B)
-        L.call("sg_pool2", _p(e3), N, *lv[3], c3, _p(B["p3"]), s)
-        e4 = self._conv("enc4b", self._conv("enc4a", B["p3"], B), B)
-        L.call("sg_up2", _p(e4), N, *lv[4], c4, _p(B["u3"]), c4 + c3, 0, s)
-        L.call("sg_copy_channels", _p(e3), N * lv[3][0] * lv[3][1], c3, _p(B["u3"]), c4 + c3, c4, s)
-        d3 = self._conv("dec3b", self._conv("dec3a", B["u3"], B), B)
-        L.call("sg_up2", _p(d3), N, *lv[3], c3, _p(B["u2"]), c3 + c2, 0, s)
-        L.call("sg_copy_channels", _p(e2), N * lv[2][0] * lv[2][1], c2, _p(B["u2"]), c3 + c2, c3, s)
-        d2 = self._conv("dec2b", self._conv("dec2a", B["u2"], B), B)
-        L.call("sg_up2", _p(d2), N, *lv[2], c2, _p(B["u1"]), c2 + c1, 0, s)
-        L.call("sg_copy_channels", _p(e1), N * H * W, c1, _p(B["u1"]), c2 + c1, c2, s)
-        d1 = self._conv("dec1b", self._conv("dec1a", B["u1"], B), B)
+        self._ops.clear()  # what a pass that raised left behind
+        self._x, self._kept = x, keep
+        e1 = self._conv("enc1b", self._conv("enc1a", x, B, keep=keep), B, keep=keep)
+        self._op("sg_pool2", (N, H, W, c1), (e1, B["p1"]))
+        e2 = self._conv("enc2b", self._conv("enc2a", B["p1"], B, keep=keep), B, keep=keep)
+        self._op("sg_pool2", (N, *lv[2], c2), (e2, B["p2"]))
+        e3 = self._conv("enc3b", self._conv("enc3a", B["p2"], B, keep=keep), B, keep=keep)
+        self._op("sg_pool2", (N, *lv[3], c3), (e3, B["p3"]))
+        e4 = self._conv("enc4b", self._conv("enc4a", B["p3"], B, keep=keep), B, keep=keep)
+        self._op("sg_up2_concat", (N, *lv[4], c4, c3), (e4, e3, B["u3"]))
+        d3 = self._conv("dec3b", self._conv("dec3a", B["u3"], B, keep=keep), B, keep=keep)
+        self._op("sg_up2_concat", (N, *lv[3], c3, c2), (d3, e2, B["u2"]))
+        d2 = self._conv("dec2b", self._conv("dec2a", B["u2"], B, keep=keep), B, keep=keep)
+        self._op("sg_up2_concat", (N, *lv[2], c2, c1), (d2, e1, B["u1"]))
+        d1 = self._conv("dec1b", self._conv("dec1a", B["u1"], B, keep=keep), B, keep=keep)
         return self._conv("out", d1, B, act=False)
+
+    def forward(self, x: torch.Tensor) -> torch.Tensor:
+        """x: (N, H, W, 16) bfloat16 frames -> out (N, H, W, 16) bfloat16 (the
+        prediction is x[..., :3] + out[..., :3])."""
+        out = self._pass(x, True)
+        self._run_ops()
+        return out
 
     def predict(self, x: torch.Tensor) -> torch.Tensor:
         """Frames one jump later: x[..., :3] + out[..., :3], other channels of x."""
-        out = self.forward(x)
+        out = self._pass(x, False)
+        if x.is_contiguous() and x.dtype == torch.bfloat16 and x.shape[-1] == out.shape[-1]:
+            y = torch.empty_like(x)
+            self._op("sg_add_prediction", (x.numel() // x.shape[-1], x.shape[-1]), (x, out, y))
+            self._run_ops()
+            return y
+        self._run_ops()
         y = x.clone()
         y[..., :3] = (x[..., :3].float() + out[..., :3].float()).to(torch.bfloat16)
         return y
 
     # ------------------------------------------------------------------
-    def _flip_all(self):
-        s = _s()
-        for name, (ci, co) in self.shapes.items():
-            L.call("sg_flip_weights", _p(self.w16[name]), ci, co, _p(self.wt16[name]), s)
-        self._flipped = True
-
     def _layer_back(self, name, inp, dz, B, need_dx=True):
-        """Weight / bias gradients of layer `name` from dz; returns dx."""
+        """Weight gradient of layer `name` from dz; returns dx."""
         ci, co = self.shapes[name]
         N, h, w, _ = inp.shape
-        s = _s()
         self._run_wgrad(inp, dz, N, h, w, ci, co, self.gw[name], B["wpart"])
-        L.call("sg_bias_grad", _p(dz), N * h * w, co, _p(self.gb[name]), _p(B["bpart"]), s)
         if not need_dx:
             return None
         dx = B["dx." + name]
         self._run_conv(dz, N, h, w, co, self.wt16[name], None, ci, 0, None, dx)
         return dx
 
-    def _gelu_back(self, name, dy, B):
-        dz = B["dz." + name]
-        L.call("sg_gelu_bwd", _p(dy), _p(B["z." + name]), dy.numel(), _p(dz), _s())
-        return dz
+    # where a layer's output gradient comes from (include/fdsurrogate.h sg_dy)
+    _PLAIN, _UP, _POOL = 0, 1, 2
 
-    def _block_back(self, name, inp, dy, B, need_dx=True):
-        return self._layer_back(name, inp, self._gelu_back(name, dy, B), B, need_dx)
+    def _block_back(self, name, inp, dy, B, need_dx=True, source=0, skip=None, cy=0, coff=0):
+        """GELU backward and bias gradient of layer `name`, then its weight
+        gradient; returns dx."""
+        ci, co = self.shapes[name]
+        N, h, w, _ = inp.shape
+        dz = B["dz." + name]
+        self._op("sg_gelu_bias_bwd", (source, N, h, w, cy, coff, co),
+                 (dy, skip, B["z." + name], dz, self.gb[name], B["bpart"]))
+        return self._layer_back(name, inp, dz, B, need_dx)
 
     def backward(self, dout: torch.Tensor):
         """Gradients (self.gw, self.gb) of the loss whose gradient w.r.t. the
         output of the last forward() is dout."""
+        self._ops.clear()
+        if not self._kept:  # the last pass was predict()'s, which keeps no pre-activations
+            self._pass(self._x, True)
         if not self._flipped:
-            self._flip_all()
+            for name, (ci, co) in self.shapes.items():
+                self._op("sg_flip_weights", (ci, co), (self.w16[name], self.wt16[name]))
+            self._flipped = True
         x = self._x
         N, H, W, _ = x.shape
         B = self._buffers(N, H, W)
-        lv = B["lv"]
         c1, c2, c3, c4 = self.widths
-        s = _s()
         y = lambda n: B["y." + n]
+        self._op("sg_bias_grad", (N * H * W, self.shapes["out"][1]), (dout, self.gb["out"], B["bpart"]))
         dd1 = self._layer_back("out", y("dec1b"), dout, B)
         du1 = self._block_back("dec1a", B["u1"], self._block_back("dec1b", y("dec1a"), dd1, B), B)
-        dd2 = B["dy.dec2b"]
-        L.call("sg_up2_bwd", _p(du1), N, *lv[2], c2 + c1, 0, c2, _p(dd2), s)
-        du2 = self._block_back("dec2a", B["u2"], self._block_back("dec2b", y("dec2a"), dd2, B), B)
-        dd3 = B["dy.dec3b"]
-        L.call("sg_up2_bwd", _p(du2), N, *lv[3], c3 + c2, 0, c3, _p(dd3), s)
-        du3 = self._block_back("dec3a", B["u3"], self._block_back("dec3b", y("dec3a"), dd3, B), B)
-        de4 = B["dy.enc4b"]
-        L.call("sg_up2_bwd", _p(du3), N, *lv[4], c4 + c3, 0, c4, _p(de4), s)
-        dp3 = self._block_back("enc4a", B["p3"], self._block_back("enc4b", y("enc4a"), de4, B), B)
-        de3 = B["de3"]
-        L.call("sg_pool2_bwd", _p(dp3), N, *lv[3], c3, _p(de3), s)
-        L.call("sg_add_channels", _p(du3), N * lv[3][0] * lv[3][1], c4 + c3, c4, c3, _p(de3), s)
-        dp2 = self._block_back("enc3a", B["p2"], self._block_back("enc3b", y("enc3a"), de3, B), B)
-        de2 = B["de2"]
-        L.call("sg_pool2_bwd", _p(dp2), N, *lv[2], c2, _p(de2), s)
-        L.call("sg_add_channels", _p(du2), N * lv[2][0] * lv[2][1], c3 + c2, c3, c2, _p(de2), s)
-        dp1 = self._block_back("enc2a", B["p1"], self._block_back("enc2b", y("enc2a"), de2, B), B)
-        de1 = B["de1"]
-        L.call("sg_pool2_bwd", _p(dp1), N, H, W, c1, _p(de1), s)
-        L.call("sg_add_channels", _p(du1), N * H * W, c2 + c1, c2, c1, _p(de1), s)
-        self._block_back("enc1a", x, self._block_back("enc1b", y("enc1a"), de1, B), B, need_dx=False)
+        dd2 = self._block_back("dec2b", y("dec2a"), du1, B, source=self._UP, cy=c2 + c1)
+        du2 = self._block_back("dec2a", B["u2"], dd2, B)
+        dd3 = self._block_back("dec3b", y("dec3a"), du2, B, source=self._UP, cy=c3 + c2)
+        du3 = self._block_back("dec3a", B["u3"], dd3, B)
+        de4 = self._block_back("enc4b", y("enc4a"), du3, B, source=self._UP, cy=c4 + c3)
+        dp3 = self._block_back("enc4a", B["p3"], de4, B)
+        de3 = self._block_back("enc3b", y("enc3a"), dp3, B, source=self._POOL, skip=du3, cy=c4 + c3, coff=c4)
+        dp2 = self._block_back("enc3a", B["p2"], de3, B)
+        de2 = self._block_back("enc2b", y("enc2a"), dp2, B, source=self._POOL, skip=du2, cy=c3 + c2, coff=c3)
+        dp1 = self._block_back("enc2a", B["p1"], de2, B)
+        de1 = self._block_back("enc1b", y("enc1a"), dp1, B, source=self._POOL, skip=du1, cy=c2 + c1, coff=c2)
+        self._block_back("enc1a", x, de1, B, need_dx=False)
+        self._run_ops()
 
     def loss_grad(self, x: torch.Tensor, xn: torch.Tensor) -> torch.Tensor:
         """Forward, masked MSE of the prediction against xn, backward.
@@ -363,22 +378,23 @@ class UNet:
         N, H, W, Cc = x.shape
         out = self.forward(x)
         B = self._buffers(N, H, W)
-        count = max(float((x[..., 3] == 0).sum().item()), 1.0)
         dout = B["dy.out"]
-        L.call("sg_masked_mse", _p(x), _p(out), _p(xn), N * H * W, Cc, _p(dout), _p(B["lpart"]),
-               C.c_float(1.0 / (3.0 * count)), _s())
+        s = _s()
+        L.call("sg_loss_scale", _p(x), N * H * W, Cc, _p(B["count"]), _p(B["inv"]), s)
+        L.call("sg_masked_mse_scaled", _p(x), _p(out), _p(xn), N * H * W, Cc, _p(dout), _p(B["lpart"]), _p(B["inv"]), s)
         self.backward(dout)
         lp = B["lpart"].view(-1, 2)
-        return lp[:, 0].sum() / (3.0 * count)
+        return lp[:, 0].sum() * B["inv"][1]
 
     def adamw(self, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=1e-2):
         self.steps += 1
-        s = _s()
-        for n in LAYERS:
-            L.call("sg_adamw", _p(self.w[n]), _p(self.w16[n]), _p(self.gw[n]), _p(self.mw[n]), _p(self.vw[n]),
-                   self.w[n].numel(), lr, beta1, beta2, eps, weight_decay, self.steps, s)
-            L.call("sg_adamw", _p(self.b[n]), None, _p(self.gb[n]), _p(self.mb[n]), _p(self.vb[n]),
-                   self.b[n].numel(), lr, beta1, beta2, eps, 0.0, self.steps, s)
+        items = (L.sg_adamw_item * (2 * len(LAYERS)))()
+        for k, n in enumerate(LAYERS):
+            for j, (w, w16, g, m, v, wd) in enumerate(((self.w, self.w16, self.gw, self.mw, self.vw, weight_decay),
+                                                       (self.b, None, self.gb, self.mb, self.vb, 0.0))):
+                items[2 * k + j] = L.sg_adamw_item(w[n].data_ptr(), None if w16 is None else w16[n].data_ptr(),
+                                                   g[n].data_ptr(), m[n].data_ptr(), v[n].data_ptr(), w[n].numel(), wd)
+        L.call("sg_adamw_list", items, len(items), lr, beta1, beta2, eps, self.steps, _s())
         self._flipped = False
 
 

@@ -110,6 +110,67 @@ int sg_loss_blocks(void);
 int sg_adamw(float* w, void* w16, const float* g, float* m, float* v, size_t n, float lr, float beta1, float beta2,
              float eps, float weight_decay, int step, void* stream);
 
+/* sg_adamw over a HOST list of tensors in one launch. */
+#define SG_ADAMW_MAX 40
+typedef struct sg_adamw_item {
+  float* w;
+  void* w16; /* may be NULL */
+  const float* g;
+  float *m, *v;
+  size_t n;
+  float weight_decay;
+} sg_adamw_item;
+int sg_adamw_list(const sg_adamw_item* items, int count, float lr, float beta1, float beta2, float eps, int step,
+                  void* stream);
+
+/* sg_gelu_bwd and sg_bias_grad of a layer (N,H,W,C) in one pass, the gradient dy
+ * taken from where it arises: a tensor (SG_DY_PLAIN), the backward of sg_up2
+ * (SG_DY_UP: dy is (N,2H,2W,Cy), channels [coff, coff+C)), or the backward of
+ * sg_pool2 plus a skip connection (SG_DY_POOL: dy is (N,H/2,W/2,C), skip
+ * (N,H,W,Cy), channels [coff, coff+C)).  The same bits as the separate calls. */
+enum sg_dy { SG_DY_PLAIN = 0, SG_DY_UP = 1, SG_DY_POOL = 2 };
+int sg_gelu_bias_bwd(int source, const void* dy, const void* skip, int N, int H, int W, int Cy, int coff, const void* z,
+                     int C, void* dz, float* db, float* partial, void* stream);
+
+/* y (N,2h,2w,C+Cs) = [sg_up2 of x, skip]: sg_up2 and sg_copy_channels in one pass. */
+int sg_up2_concat(const void* x, int N, int h, int w, int C, const void* skip, int Cs, void* y, void* stream);
+
+/* Scales of the masked loss from the batch itself, without the host waiting:
+ * *count = fluid pixels, inv[0] = 1 / (3 max(count, 1)) for sg_masked_mse_scaled
+ * (sg_masked_mse with its inv_count in device memory), inv[1] the reciprocal of
+ * 3 max(count, 1) in single precision (device memory). */
+int sg_loss_scale(const void* x, size_t P, int C, unsigned* count, float* inv, void* stream);
+int sg_masked_mse_scaled(const void* x, const void* out, const void* xn, size_t P, int C, void* dout,
+                         float* loss_partial, const float* inv, void* stream);
+
+/* y = x (NHWC, C channels) with its first three channels replaced by x + out. */
+int sg_add_prediction(const void* x, const void* out, size_t P, int C, void* y, void* stream);
+
+/* A HOST list of the calls above on one stream, in order: a network's pass in one
+ * call (from Python a call of each costs more than its kernel on small batches).
+ * i and p are the call's integers and pointers in their order, without the
+ * stream; a weight gradient's i[5] is partial_floats and its split automatic.
+ * Stops at the first call that fails and returns its status. */
+enum sg_op_kind {
+  SG_OP_CONV = 0,       /* sg_conv3x3:        i N H W Cin Cout act; p x w bias z y */
+  SG_OP_CONV_TC = 1,    /* sg_conv3x3_tc */
+  SG_OP_CONV_TMA = 2,   /* sg_conv3x3_tma */
+  SG_OP_WGRAD = 3,      /* sg_conv3x3_wgrad:  i N H W Cin Cout partial_floats; p x dz dw partial */
+  SG_OP_WGRAD_TC = 4,   /* sg_conv3x3_wgrad_tc */
+  SG_OP_POOL = 5,       /* sg_pool2:          i N H W C; p x y */
+  SG_OP_UP_CONCAT = 6,  /* sg_up2_concat:     i N h w C Cs; p x skip y */
+  SG_OP_GELU_BIAS = 7,  /* sg_gelu_bias_bwd:  i source N H W Cy coff C; p dy skip z dz db partial */
+  SG_OP_BIAS = 8,       /* sg_bias_grad:      i P C; p dz db partial */
+  SG_OP_FLIP = 9,       /* sg_flip_weights:   i Cin Cout; p w wt */
+  SG_OP_ADD_PREDICTION = 10 /* sg_add_prediction: i P C; p x out y */
+};
+typedef struct sg_op {
+  int64_t kind;
+  int64_t i[8];
+  uint64_t p[7];
+} sg_op;
+int sg_run(const sg_op* ops, int count, void* stream);
+
 /* FP32 -> bfloat16 (round to nearest even), n elements. */
 int sg_to_bf16(const float* src, size_t n, void* dst, void* stream);
 
