@@ -332,8 +332,8 @@ __device__ __forceinline__ unsigned mask_at(const char* sm, int mrow, int lx) {
 // FP16/BF16: the 17 values in the storage type (f_0..f_8 then g_1..g_8) are
 // converted two at a time with one instruction (pair_from_f, pair_from_f_sr:
 // one 32-bit random word per pair) and written as 16-bit stores; g_0 stays FP32.
-template <typename SF, bool SCALED, bool STOCH>
-__device__ __forceinline__ void store_cell(const DevArgs<SF>& a, size_t q, const float (&f)[9], const float (&g)[9]) {
+template <typename SF, bool SCALED, bool STOCH, typename I = size_t>
+__device__ __forceinline__ void store_cell(const DevArgs<SF>& a, I q, const float (&f)[9], const float (&g)[9]) {
   if constexpr (std::is_same_v<SF, float>) {
     float* pf = a.dst_f + q;
 #pragma unroll

@@ -33,16 +33,20 @@ constexpr int kTileTX = 32;
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// The addresses a cell pulls from: rows y-1, y, y+1 and columns x-1, x, x+1 (wrapped).
+// The elements a cell pulls from, as offsets of type I from the first plane
+// (32-bit ones where nine planes are below 2^32 elements: 64-bit address
+// arithmetic was a fifth of the kernel's instructions).  Rows wrap; columns do
+// not: what streams in across x = 0 and x = W - 1 is replaced by the Zou-He rules,
+// and an element before or after a row lies inside the packed buffer for every
+// direction that asks for one.
+template <typename I>
 struct TilePull {
-  size_t row[3];  // offsets of rows y-1, y, y+1
-  int col[3];
+  I row[3];  // the cell's element in rows y-1, y, y+1
   __device__ __forceinline__ TilePull(int x, int y, int H, int W)
-      : row{(size_t)wrap(y - 1, H) * W, (size_t)y * W, (size_t)wrap(y + 1, H) * W},
-        col{wrap(x - 1, W), x, wrap(x + 1, W)} {}
+      : row{(I)wrap(y - 1, H) * (I)W + (I)x, (I)y * (I)W + (I)x, (I)wrap(y + 1, H) * (I)W + (I)x} {}
   // population i streams from (x - e_x, y - e_y)
-  __device__ __forceinline__ size_t from(int i) const { return row[1 - ey_of(i)] + col[1 - ex_of(i)]; }
-  __device__ __forceinline__ size_t own() const { return row[1] + col[1]; }
+  __device__ __forceinline__ I from(int i) const { return row[1 - ey_of(i)] - (I)ex_of(i); }
+  __device__ __forceinline__ I own() const { return row[1]; }
 };
 
 // Loads of the state go to L2 (ld.global.cg): the SM's L1 may hold lines of the
@@ -57,24 +61,27 @@ __device__ __forceinline__ float tile_ld(const S* p, float scale) {
 }
 
 // f of a cell: stream, then the bounce-back links (the opposite population of the same cell)
-template <typename SF, bool RING, bool SCALED>
-__device__ __forceinline__ void tile_pull_f(const DevArgs<SF>& a, const TilePull& t, unsigned bits, float (&v)[9]) {
+template <typename SF, bool RING, bool SCALED, typename I>
+__device__ __forceinline__ void tile_pull_f(const DevArgs<SF>& a, const TilePull<I>& t, unsigned bits, float (&v)[9]) {
+  const I ps = (I)a.pstride_f;
 #pragma unroll
   for (int i = 0; i < 9; ++i) {
     const bool link = i > 0 && ((bits >> (i - 1)) & 1u);
-    v[i] = tile_ld<SF, RING, SCALED>(a.src_f + (size_t)(link ? opp_of(i) : i) * a.pstride_f + (link ? t.own() : t.from(i)),
-                                     a.c.inv_sf);
+    const I o = link ? (I)opp_of(i) * ps + t.own() : (I)i * ps + t.from(i);
+    v[i] = tile_ld<SF, RING, SCALED>(a.src_f + o, a.c.inv_sf);
   }
 }
 
-template <typename SF, bool RING, bool SCALED>
-__device__ __forceinline__ void tile_pull_g(const DevArgs<SF>& a, const TilePull& t, unsigned bits, float (&v)[9]) {
+template <typename SF, bool RING, bool SCALED, typename I>
+__device__ __forceinline__ void tile_pull_g(const DevArgs<SF>& a, const TilePull<I>& t, unsigned bits, float (&v)[9]) {
+  const I ps = (I)a.pstride_f;
+  const SF* f0 = a.src_gi - a.pstride_f;  // a plane before g_1's, so that every offset is positive
   v[0] = __ldcg(a.src_g0 + t.own());
 #pragma unroll
   for (int i = 1; i < 9; ++i) {
     const bool link = (bits >> (i - 1)) & 1u;
-    v[i] = tile_ld<SF, RING, SCALED>(a.src_gi + (size_t)((link ? opp_of(i) : i) - 1) * a.pstride_f +
-                                         (link ? t.own() : t.from(i)), a.c.inv_sg);
+    const I o = link ? (I)opp_of(i) * ps + t.own() : (I)i * ps + t.from(i);
+    v[i] = tile_ld<SF, RING, SCALED>(f0 + o, a.c.inv_sg);
   }
 }
 
@@ -125,8 +132,8 @@ struct TilePsi {
 };
 
 // Stores of one cell in the arithmetic of widths that are not a multiple of 8
-template <typename SF, bool STOCH>
-__device__ __forceinline__ void tile_store_scalar(const DevArgs<SF>& a, size_t q, const float (&f)[9],
+template <typename SF, bool STOCH, typename I>
+__device__ __forceinline__ void tile_store_scalar(const DevArgs<SF>& a, I q, const float (&f)[9],
                                                   const float (&g)[9]) {
   uint32_t rs = 0;
   if constexpr (STOCH) rs = sr_hash((uint32_t)q ^ a.seed);
@@ -141,22 +148,22 @@ __device__ __forceinline__ void tile_store_scalar(const DevArgs<SF>& a, size_t q
     }
   };
 #pragma unroll
-  for (int i = 0; i < 9; ++i) a.dst_f[i * a.pstride_f + q] = conv(f[i], a.c.sf);
+  for (int i = 0; i < 9; ++i) (a.dst_f + i * a.pstride_f)[q] = conv(f[i], a.c.sf);
   a.dst_g0[q] = g[0];
 #pragma unroll
-  for (int i = 1; i < 9; ++i) a.dst_gi[(i - 1) * a.pstride_f + q] = conv(g[i], a.c.sg);
+  for (int i = 1; i < 9; ++i) (a.dst_gi + (i - 1) * a.pstride_f)[q] = conv(g[i], a.c.sg);
 }
 
 // rho_inlet - 1 of row yn (1 or H-2) of the walled variant's inlet column
 // (fingering.py:341, 357), as inlet_corner_drho, from f pulled through L2.
-template <typename SF, bool RING, bool SCALED>
+template <typename SF, bool RING, bool SCALED, typename I>
 __device__ __forceinline__ float tile_corner_drho(const DevArgs<SF>& a, int yn) {
   float d[9];
-  tile_pull_f<SF, RING, SCALED>(a, TilePull(0, yn, a.H, a.W), a.mask[(size_t)yn * a.W] & 0xFFu, d);
+  tile_pull_f<SF, RING, SCALED>(a, TilePull<I>(0, yn, a.H, a.W), a.mask[(size_t)yn * a.W] & 0xFFu, d);
   return dev_inlet_drho(d, (float)a.inlet_ux[yn], __ldcg(a.side_in + yn), __ldcg(a.side_in + 2 * a.H + yn));
 }
 
-template <typename SF, bool RING, bool SCALED, bool STOCH, int TY>
+template <typename SF, bool RING, bool SCALED, bool STOCH, int TY, typename I>
 __global__ void __launch_bounds__(32 * TY) k_tile_step(const __grid_constant__ DevArgs<SF> a, int ntx) {
   using Psi = TilePsi<SF, RING, TY>;
   constexpr int PW = Psi::PW;
@@ -190,7 +197,7 @@ __global__ void __launch_bounds__(32 * TY) k_tile_step(const __grid_constant__ D
   pdl_launch_dependents();
 
   float g[9], f[9];
-  const TilePull at(x, in ? y : 0, a.H, a.W);
+  const TilePull<I> at(x, in ? y : 0, a.H, a.W);
   if (in) {
     tile_pull_g<SF, RING, SCALED>(a, at, m & 0xFFu, g);
     tile_pull_f<SF, RING, SCALED>(a, at, m & 0xFFu, f);
@@ -201,7 +208,7 @@ __global__ void __launch_bounds__(32 * TY) k_tile_step(const __grid_constant__ D
       v.x = a.c.psi_wall;
     } else if (hcell) {
       float gh[9];
-      tile_pull_g<SF, RING, SCALED>(a, TilePull(hx, hy, a.H, a.W), hm & 0xFFu, gh);
+      tile_pull_g<SF, RING, SCALED>(a, TilePull<I>(hx, hy, a.H, a.W), hm & 0xFFu, gh);
       v = tile_psi<SF, RING>(a, hx, hy, hm, gh);
     }
     psi.put(he, v);
@@ -218,7 +225,7 @@ __global__ void __launch_bounds__(32 * TY) k_tile_step(const __grid_constant__ D
     } else if (y == a.H && x < a.W) {
       const unsigned gm = __ldg(a.mask + x);
       float gh[9];
-      tile_pull_g<SF, RING, SCALED>(a, TilePull(x, 0, a.H, a.W), gm & 0xFFu, gh);
+      tile_pull_g<SF, RING, SCALED>(a, TilePull<I>(x, 0, a.H, a.W), gm & 0xFFu, gh);
       v = tile_psi<SF, RING>(a, x, 0, gm, gh);
     }
     psi.put(e, v);
@@ -231,7 +238,7 @@ __global__ void __launch_bounds__(32 * TY) k_tile_step(const __grid_constant__ D
       const int o = (x == 0) ? 0 : 3;
       float drho_nb = 0.0f;
       if (walls && x == 0 && (y == 0 || y == a.H - 1))
-        drho_nb = tile_corner_drho<SF, RING, SCALED>(a, y == 0 ? 1 : a.H - 2);
+        drho_nb = tile_corner_drho<SF, RING, SCALED, I>(a, y == 0 ? 1 : a.H - 2);
       dev_zou_he_f(a.c, a.variant, a.H, a.W, x, y, f, (float)a.inlet_ux[y], __ldcg(a.side_in + (o + 0) * a.H + y),
                    __ldcg(a.side_in + (o + 1) * a.H + y), __ldcg(a.side_in + (o + 2) * a.H + y), drho_nb);
       a.side_out[(o + 0) * a.H + y] = st.gx;
@@ -244,8 +251,8 @@ __global__ void __launch_bounds__(32 * TY) k_tile_step(const __grid_constant__ D
       if constexpr (RING) dev_collide_for<SF>(a.c, mc, f, g);
       else dev_collide(a.c, mc, f, g);
     }
-    if constexpr (RING) store_cell<SF, SCALED, STOCH>(a, at.own(), f, g);
-    else tile_store_scalar<SF, STOCH>(a, at.own(), f, g);
+    if constexpr (RING) store_cell<SF, SCALED, STOCH, I>(a, at.own(), f, g);
+    else tile_store_scalar<SF, STOCH, I>(a, at.own(), f, g);
   }
   if (__any_sync(0xffffffffu, bad) && lx == 0) report_nonfinite(a);
 }
@@ -290,8 +297,15 @@ int launch_tile(const fd_params& p, const DevCoef& c, const uint16_t* mask, cons
     const bool even = s % 2 == 0;
     tma_set_step(a, even ? pa : pb, even ? pb : pa, even ? sa : sb, even ? sb : sa, seed + (uint32_t)s);
     // the first step's masks may have been written by the work just before it
-    if (launch_pdl(k_tile_step<SF, RING, SCALED, STOCH, TY>, blocks, 32 * TY, st, s > 0, a, ntx) != cudaSuccess)
-      return FD_ERR_CUDA;
+    cudaError_t e;
+    if (9 * L.pstride < ((size_t)1 << 32)) {
+      e = launch_pdl(k_tile_step<SF, RING, SCALED, STOCH, TY, uint32_t>, blocks, 32 * TY, st, s > 0, a, ntx);
+    } else if constexpr (!RING) {
+      e = launch_pdl(k_tile_step<SF, RING, SCALED, STOCH, TY, size_t>, blocks, 32 * TY, st, s > 0, a, ntx);
+    } else {
+      return FD_ERR_SHAPE;  // not reached: the rule sends lattices of this size to the staged kernel
+    }
+    if (e != cudaSuccess) return FD_ERR_CUDA;
   }
   return FD_OK;
 }
