@@ -328,6 +328,20 @@ __device__ __forceinline__ unsigned mask_at(const char* sm, int mrow, int lx) {
 // (fingering_periodic.py:210-212, 278-302); the pulled g is returned in g.
 // `mrow` is the byte offset of row y's mask row.
 
+// An element by its byte offset from a base pointer.
+template <typename T, typename I>
+__device__ __forceinline__ T* byte_at(T* base, I off) {
+  return reinterpret_cast<T*>((char*)base + off);
+}
+
+// Element q of plane k.  With a 32-bit q the byte offset is formed in 32 bits as
+// well (the caller's planes are below 4 GB); with a 64-bit one the plane's base is.
+template <typename S, typename I>
+__device__ __forceinline__ S* plane_el(S* base, size_t pstride, int k, I q) {
+  if constexpr (sizeof(I) == 4) return byte_at(base, ((I)k * (I)pstride + q) * (I)sizeof(S));
+  else return base + (size_t)k * pstride + q;
+}
+
 // Stores of one cell's new populations into the packed layout (q = y W + x).
 // FP16/BF16: the 17 values in the storage type (f_0..f_8 then g_1..g_8) are
 // converted two at a time with one instruction (pair_from_f, pair_from_f_sr:
@@ -335,13 +349,11 @@ __device__ __forceinline__ unsigned mask_at(const char* sm, int mrow, int lx) {
 template <typename SF, bool SCALED, bool STOCH, typename I = size_t>
 __device__ __forceinline__ void store_cell(const DevArgs<SF>& a, I q, const float (&f)[9], const float (&g)[9]) {
   if constexpr (std::is_same_v<SF, float>) {
-    float* pf = a.dst_f + q;
 #pragma unroll
-    for (int i = 0; i < 9; ++i, pf += a.pstride_f) *pf = f[i];
-    a.dst_g0[q] = g[0];
-    float* pg = a.dst_gi + q;
+    for (int i = 0; i < 9; ++i) *plane_el(a.dst_f, a.pstride_f, i, q) = f[i];
+    *plane_el(a.dst_g0, 0, 0, q) = g[0];
 #pragma unroll
-    for (int i = 1; i < 9; ++i, pg += a.pstride_f) *pg = g[i];
+    for (int i = 1; i < 9; ++i) *plane_el(a.dst_gi, a.pstride_f, i - 1, q) = g[i];
   } else {
     float v[18];
 #pragma unroll
@@ -352,7 +364,7 @@ __device__ __forceinline__ void store_cell(const DevArgs<SF>& a, I q, const floa
     uint32_t rs = 0;
     if constexpr (STOCH) rs = sr_hash((uint32_t)q ^ a.seed);
     auto plane = [&](int k) -> uint16_t* {
-      SF* p = k < 9 ? a.dst_f + (size_t)k * a.pstride_f + q : a.dst_gi + (size_t)(k - 9) * a.pstride_f + q;
+      SF* p = k < 9 ? plane_el(a.dst_f, a.pstride_f, k, q) : plane_el(a.dst_gi, a.pstride_f, k - 9, q);
       return reinterpret_cast<uint16_t*>(p);
     };
 #pragma unroll
@@ -367,7 +379,7 @@ __device__ __forceinline__ void store_cell(const DevArgs<SF>& a, I q, const floa
       *plane(k) = (uint16_t)w;
       if (k + 1 < 17) *plane(k + 1) = (uint16_t)(w >> 16);
     }
-    a.dst_g0[q] = g[0];
+    *plane_el(a.dst_g0, 0, 0, q) = g[0];
   }
 }
 

@@ -13,8 +13,8 @@
 // the populations.
 //
 // Measured, us per step (the kernel before -> this one): FP32 64 x 128 26 -> 3.5
-// and 380 x 380 15.7 -> 7.2, BF16 1021 x 1500 82 -> 47.5 (there it is bound by
-// instruction issue).  Tiles of 4 rows: 8 rows lose 7-11% on FP32 from 1024 x 1024
+// and 380 x 380 15.7 -> 6.2, BF16 1021 x 1500 82 -> 41.4 (there it is bound by
+// instruction issue; 47.5 with 64-bit addresses).  Tiles of 4 rows: 8 rows lose 7-11% on FP32 from 1024 x 1024
 // up and gain on single sizes below (256 x 512 6.2 vs 7.0).
 //
 // The arithmetic and the rounding of the stores are those of the kernel that the
@@ -33,20 +33,25 @@ constexpr int kTileTX = 32;
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// The elements a cell pulls from, as offsets of type I from the first plane
-// (32-bit ones where nine planes are below 2^32 elements: 64-bit address
-// arithmetic was a fifth of the kernel's instructions).  Rows wrap; columns do
-// not: what streams in across x = 0 and x = W - 1 is replaced by the Zou-He rules,
-// and an element before or after a row lies inside the packed buffer for every
-// direction that asks for one.
-template <typename I>
+// The elements a cell pulls from, as byte offsets of type I from the first plane
+// (32-bit ones where nine planes are below 4 GB, which load and store
+// instructions add to a uniform base: 64-bit address arithmetic was a fifth of
+// the kernel's instructions).  Rows wrap; columns do not: what streams in across
+// x = 0 and x = W - 1 is replaced by the Zou-He rules, and an element before or
+// after a row lies inside the packed buffer for every direction that asks for one.
+template <typename SF, typename I>
 struct TilePull {
   I row[3];  // the cell's element in rows y-1, y, y+1
   __device__ __forceinline__ TilePull(int x, int y, int H, int W)
-      : row{(I)wrap(y - 1, H) * (I)W + (I)x, (I)y * (I)W + (I)x, (I)wrap(y + 1, H) * (I)W + (I)x} {}
+      : row{el(x, wrap(y - 1, H), W), el(x, y, W), el(x, wrap(y + 1, H), W)} {}
+  static __device__ __forceinline__ I el(int x, int y, int W) { return ((I)y * (I)W + (I)x) * (I)sizeof(SF); }
   // population i streams from (x - e_x, y - e_y)
-  __device__ __forceinline__ I from(int i) const { return row[1 - ey_of(i)] - (I)ex_of(i); }
+  __device__ __forceinline__ I from(int i) const { return row[1 - ey_of(i)] - (I)(ex_of(i) * (int)sizeof(SF)); }
   __device__ __forceinline__ I own() const { return row[1]; }
+  __device__ __forceinline__ I pull(int i, unsigned bits, I plane) const {  // plane: bytes of one
+    const bool link = i > 0 && ((bits >> (i - 1)) & 1u);
+    return link ? (I)opp_of(i) * plane + own() : (I)i * plane + from(i);
+  }
 };
 
 // Loads of the state go to L2 (ld.global.cg): the SM's L1 may hold lines of the
@@ -62,27 +67,21 @@ __device__ __forceinline__ float tile_ld(const S* p, float scale) {
 
 // f of a cell: stream, then the bounce-back links (the opposite population of the same cell)
 template <typename SF, bool RING, bool SCALED, typename I>
-__device__ __forceinline__ void tile_pull_f(const DevArgs<SF>& a, const TilePull<I>& t, unsigned bits, float (&v)[9]) {
-  const I ps = (I)a.pstride_f;
+__device__ __forceinline__ void tile_pull_f(const DevArgs<SF>& a, const TilePull<SF, I>& t, unsigned bits, float (&v)[9]) {
+  const I plane = (I)a.pstride_f * (I)sizeof(SF);
 #pragma unroll
-  for (int i = 0; i < 9; ++i) {
-    const bool link = i > 0 && ((bits >> (i - 1)) & 1u);
-    const I o = link ? (I)opp_of(i) * ps + t.own() : (I)i * ps + t.from(i);
-    v[i] = tile_ld<SF, RING, SCALED>(a.src_f + o, a.c.inv_sf);
-  }
+  for (int i = 0; i < 9; ++i)
+    v[i] = tile_ld<SF, RING, SCALED>(byte_at(a.src_f, t.pull(i, bits, plane)), a.c.inv_sf);
 }
 
 template <typename SF, bool RING, bool SCALED, typename I>
-__device__ __forceinline__ void tile_pull_g(const DevArgs<SF>& a, const TilePull<I>& t, unsigned bits, float (&v)[9]) {
-  const I ps = (I)a.pstride_f;
-  const SF* f0 = a.src_gi - a.pstride_f;  // a plane before g_1's, so that every offset is positive
-  v[0] = __ldcg(a.src_g0 + t.own());
+__device__ __forceinline__ void tile_pull_g(const DevArgs<SF>& a, const TilePull<SF, I>& t, unsigned bits, float (&v)[9]) {
+  const I plane = (I)a.pstride_f * (I)sizeof(SF);
+  const SF* before = a.src_gi - a.pstride_f;  // a plane before g_1's, so that every offset is positive
+  v[0] = __ldcg(byte_at(a.src_g0, t.own() * (I)(4 / sizeof(SF))));
 #pragma unroll
-  for (int i = 1; i < 9; ++i) {
-    const bool link = (bits >> (i - 1)) & 1u;
-    const I o = link ? (I)opp_of(i) * ps + t.own() : (I)i * ps + t.from(i);
-    v[i] = tile_ld<SF, RING, SCALED>(f0 + o, a.c.inv_sg);
-  }
+  for (int i = 1; i < 9; ++i)
+    v[i] = tile_ld<SF, RING, SCALED>(byte_at(before, t.pull(i, bits, plane)), a.c.inv_sg);
 }
 
 // psi of a lattice cell from its pulled g after Zou-He (g is updated)
@@ -148,10 +147,10 @@ __device__ __forceinline__ void tile_store_scalar(const DevArgs<SF>& a, I q, con
     }
   };
 #pragma unroll
-  for (int i = 0; i < 9; ++i) (a.dst_f + i * a.pstride_f)[q] = conv(f[i], a.c.sf);
-  a.dst_g0[q] = g[0];
+  for (int i = 0; i < 9; ++i) *plane_el(a.dst_f, a.pstride_f, i, q) = conv(f[i], a.c.sf);
+  *plane_el(a.dst_g0, 0, 0, q) = g[0];
 #pragma unroll
-  for (int i = 1; i < 9; ++i) (a.dst_gi + (i - 1) * a.pstride_f)[q] = conv(g[i], a.c.sg);
+  for (int i = 1; i < 9; ++i) *plane_el(a.dst_gi, a.pstride_f, i - 1, q) = conv(g[i], a.c.sg);
 }
 
 // rho_inlet - 1 of row yn (1 or H-2) of the walled variant's inlet column
@@ -159,12 +158,13 @@ __device__ __forceinline__ void tile_store_scalar(const DevArgs<SF>& a, I q, con
 template <typename SF, bool RING, bool SCALED, typename I>
 __device__ __forceinline__ float tile_corner_drho(const DevArgs<SF>& a, int yn) {
   float d[9];
-  tile_pull_f<SF, RING, SCALED>(a, TilePull<I>(0, yn, a.H, a.W), a.mask[(size_t)yn * a.W] & 0xFFu, d);
+  tile_pull_f<SF, RING, SCALED>(a, TilePull<SF, I>(0, yn, a.H, a.W), a.mask[(size_t)yn * a.W] & 0xFFu, d);
   return dev_inlet_drho(d, (float)a.inlet_ux[yn], __ldcg(a.side_in + yn), __ldcg(a.side_in + 2 * a.H + yn));
 }
 
-template <typename SF, bool RING, bool SCALED, bool STOCH, int TY, typename I>
-__global__ void __launch_bounds__(32 * TY) k_tile_step(const __grid_constant__ DevArgs<SF> a, int ntx) {
+// MINB: CTAs per SM that the registers are cut for (launch_tile)
+template <typename SF, bool RING, bool SCALED, bool STOCH, int TY, typename I, int MINB>
+__global__ void __launch_bounds__(32 * TY, MINB) k_tile_step(const __grid_constant__ DevArgs<SF> a, int ntx) {
   using Psi = TilePsi<SF, RING, TY>;
   constexpr int PW = Psi::PW;
   __shared__ Psi psi;
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(32 * TY) k_tile_step(const __grid_constant__ D
   pdl_launch_dependents();
 
   float g[9], f[9];
-  const TilePull<I> at(x, in ? y : 0, a.H, a.W);
+  const TilePull<SF, I> at(x, in ? y : 0, a.H, a.W);
   if (in) {
     tile_pull_g<SF, RING, SCALED>(a, at, m & 0xFFu, g);
     tile_pull_f<SF, RING, SCALED>(a, at, m & 0xFFu, f);
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(32 * TY) k_tile_step(const __grid_constant__ D
       v.x = a.c.psi_wall;
     } else if (hcell) {
       float gh[9];
-      tile_pull_g<SF, RING, SCALED>(a, TilePull<I>(hx, hy, a.H, a.W), hm & 0xFFu, gh);
+      tile_pull_g<SF, RING, SCALED>(a, TilePull<SF, I>(hx, hy, a.H, a.W), hm & 0xFFu, gh);
       v = tile_psi<SF, RING>(a, hx, hy, hm, gh);
     }
     psi.put(he, v);
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(32 * TY) k_tile_step(const __grid_constant__ D
     } else if (y == a.H && x < a.W) {
       const unsigned gm = __ldg(a.mask + x);
       float gh[9];
-      tile_pull_g<SF, RING, SCALED>(a, TilePull<I>(x, 0, a.H, a.W), gm & 0xFFu, gh);
+      tile_pull_g<SF, RING, SCALED>(a, TilePull<SF, I>(x, 0, a.H, a.W), gm & 0xFFu, gh);
       v = tile_psi<SF, RING>(a, x, 0, gm, gh);
     }
     psi.put(e, v);
@@ -251,8 +251,8 @@ __global__ void __launch_bounds__(32 * TY) k_tile_step(const __grid_constant__ D
       if constexpr (RING) dev_collide_for<SF>(a.c, mc, f, g);
       else dev_collide(a.c, mc, f, g);
     }
-    if constexpr (RING) store_cell<SF, SCALED, STOCH, I>(a, at.own(), f, g);
-    else tile_store_scalar<SF, STOCH, I>(a, at.own(), f, g);
+    if constexpr (RING) store_cell<SF, SCALED, STOCH, I>(a, at.own() / (I)sizeof(SF), f, g);
+    else tile_store_scalar<SF, STOCH, I>(a, at.own() / (I)sizeof(SF), f, g);
   }
   if (__any_sync(0xffffffffu, bad) && lx == 0) report_nonfinite(a);
 }
@@ -276,6 +276,11 @@ cudaError_t launch_pdl(void (*kern)(P...), unsigned blocks, unsigned threads, cu
 #ifndef FD_TILE_TY
 #define FD_TILE_TY 4
 #endif
+// Cells up to which the registers are cut for 8 CTAs per SM (more loads of a cell
+// in flight), above which for 10 (more cells in flight).  us per step, 8 / 10:
+// FP32 380 x 380 6.2 / 6.8, 512 x 1024 14.6 / 14.6, 768 x 1024 26.4 / 25.4, 1021 x
+// 1500 49.7 / 47.6; BF16 380 x 380 6.3 / 7.0, 1021 x 1500 42.4 / 41.4.
+constexpr size_t kTileFewCells = 600000;
 
 template <typename SF, bool RING, bool SCALED, bool STOCH>
 int launch_tile(const fd_params& p, const DevCoef& c, const uint16_t* mask, const double* inlet_ux, char* pa, char* pb,
@@ -297,13 +302,15 @@ int launch_tile(const fd_params& p, const DevCoef& c, const uint16_t* mask, cons
     const bool even = s % 2 == 0;
     tma_set_step(a, even ? pa : pb, even ? pb : pa, even ? sa : sb, even ? sb : sa, seed + (uint32_t)s);
     // the first step's masks may have been written by the work just before it
+    auto go = [&](auto kern) { return launch_pdl(kern, blocks, 32 * TY, st, s > 0, a, ntx); };
     cudaError_t e;
-    if (9 * L.pstride < ((size_t)1 << 32)) {
-      e = launch_pdl(k_tile_step<SF, RING, SCALED, STOCH, TY, uint32_t>, blocks, 32 * TY, st, s > 0, a, ntx);
-    } else if constexpr (!RING) {
-      e = launch_pdl(k_tile_step<SF, RING, SCALED, STOCH, TY, size_t>, blocks, 32 * TY, st, s > 0, a, ntx);
+    if (9 * L.pstride * sizeof(SF) >= ((size_t)1 << 32)) {
+      if constexpr (RING) return FD_ERR_SHAPE;  // not reached: lattices of this size take the staged kernel
+      else e = go(k_tile_step<SF, RING, SCALED, STOCH, TY, size_t, 8>);
+    } else if (L.P <= kTileFewCells) {
+      e = go(k_tile_step<SF, RING, SCALED, STOCH, TY, uint32_t, 8>);
     } else {
-      return FD_ERR_SHAPE;  // not reached: the rule sends lattices of this size to the staged kernel
+      e = go(k_tile_step<SF, RING, SCALED, STOCH, TY, uint32_t, 10>);
     }
     if (e != cudaSuccess) return FD_ERR_CUDA;
   }
