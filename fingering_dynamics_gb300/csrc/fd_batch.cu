@@ -1,13 +1,14 @@
 // Batched ensemble: many independent lattices (uneven sizes, geometries and
 // parameters) advanced together by one persistent launch per iteration over a
 // table of (instance, band, strip) tiles, with the iteration loop replayed
-// from a CUDA graph.
+// from a CUDA graph; small batches by one launch of the tile kernel per
+// iteration (tile_batch_cells).
 #include <algorithm>
 #include <vector>
 
 #include "fd_batch_plan.h"
-#include "fd_fused_tma.cuh"
 #include "fd_host.h"
+#include "fd_tile.cuh"
 
 struct fd_batch {
   int n = 0;
@@ -21,6 +22,8 @@ struct fd_batch {
   int ntiles = 0;  // tiles of the shape asked for (fd_batch_tiles)
   int nwork = 0;   // tiles of the table, whose strips may be shorter (fd_batch_plan.h)
   int grid = 0;
+  int2* d_cells = nullptr;  // (member, tile) of the tile kernel; ncells 0: the staged kernel
+  int ncells = 0;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   cudaStream_t graph_stream = nullptr;
@@ -62,6 +65,83 @@ DevArgs<SF> instance_args(const fd_instance& in, const fd_storage& st, int rows,
   a.seed = in.seed;  // hashed with the batch step counter in the kernel
   a.status = status;
   return a;
+}
+
+// Cells of a batch's live members up to which its iterations run on the tile
+// kernel (the staged kernel's strips leave a small batch's SMs partly idle).  us
+// per iteration, tile / staged, lattices of 256 x 512: FP32 one 6.7 / 16.4, 2 10.3 /
+// 18.5, 4 18.2 / 24.8, 8 39.6 / 44.8, 24 109 / 115, 32 143 / 146; FP16 one 7.2 /
+// 14.4, 4 17.6 / 22.6, 8 33.0 / 34.9, 16 65.0 / 64.7, 32 125 / 116.
+constexpr long long tile_batch_cells(int dtype) { return dtype == FD_F32 ? 4000000 : 1500000; }
+
+// The tile kernel over a batch: a CTA copies its member's arguments to shared
+// memory while the previous iteration drains.
+struct TileMember {
+  bool live;
+  uint32_t seed;
+  __device__ __forceinline__ bool stepped() const { return live; }
+  __device__ __forceinline__ uint32_t step_seed() const { return seed; }
+};
+
+template <typename SF, bool STOCH, int TY>
+__global__ void __launch_bounds__(32 * TY, 8)
+    k_tile_step_batch(const BatchInst<SF>* __restrict__ inst, const int2* __restrict__ cells, int parity,
+                      unsigned* __restrict__ ctl) {
+  __shared__ TilePsi<SF, true, TY> psi;
+  __shared__ DevArgs<SF> a;
+  static_assert(sizeof(DevArgs<SF>) % 4 == 0, "copied in words");
+  const int2 c = cells[blockIdx.x];
+  const uint32_t* from = reinterpret_cast<const uint32_t*>(&inst[c.x].args[parity]);
+  for (int i = threadIdx.x; i < (int)(sizeof(DevArgs<SF>) / 4); i += 32 * TY)
+    reinterpret_cast<uint32_t*>(&a)[i] = from[i];
+  __syncthreads();
+  tile_cells_step<SF, true, false, STOCH, TY, uint32_t>(a, (a.W + kTileTX - 1) / kTileTX, c.y, psi, [&] {
+    tile_step_begins();
+    unsigned done = 0;
+    if constexpr (STOCH) done = __ldcg(ctl + parity);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // the counters as k_fused_tma_batch keeps them
+      if constexpr (STOCH) ctl[parity ^ 1] = done + 1;
+      ctl[2 + (parity ^ 1)] = 0;
+    }
+    // a quarantined member (non-finite cell seen) is not stepped any more
+    const unsigned flagged = *reinterpret_cast<volatile unsigned*>(a.status);
+    return TileMember{flagged == 0u, STOCH ? sr_hash(a.seed + done) : 0u};
+  });
+}
+
+// The table of the tile kernel, if the batch takes it: its live members are
+// few cells, and the strips are the default ones (another shape asks for the
+// staged kernel).
+int prepare_cells(fd_batch* b, const std::vector<unsigned>& flagged) {
+  cudaFree(b->d_cells);
+  b->d_cells = nullptr;
+  b->ncells = 0;
+  long long live = 0;
+  int lowest = 3;
+  for (int i = 0; i < b->n; ++i) {
+    if (flagged[(size_t)i] != 0u) continue;
+    live += (long long)b->inst[i].prm.H * b->inst[i].prm.W;
+    lowest = std::min(lowest, b->inst[i].prm.H);
+  }
+  if (live == 0 || lowest < 3 || live > tile_batch_cells(b->st.dtype) || b->rows != 32 || b->band != 128) return FD_OK;
+  std::vector<int2> cells;
+  for (int i = 0; i < b->n; ++i) {
+    if (flagged[(size_t)i] != 0u) continue;
+    const fd_params& p = b->inst[i].prm;
+    const int k = ((p.W + kTileTX - 1) / kTileTX) * ((p.H + FD_TILE_TY - 1) / FD_TILE_TY);
+    for (int j = 0; j < k; ++j) cells.push_back(make_int2(i, j));
+  }
+  if (cudaMalloc(&b->d_cells, sizeof(int2) * cells.size()) != cudaSuccess ||
+      cudaMemcpy(b->d_cells, cells.data(), sizeof(int2) * cells.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+    return check_launch("fd_batch: tile table");
+  b->ncells = (int)cells.size();
+  return FD_OK;
+}
+
+template <typename SF, bool STOCH>
+void launch_cells(const fd_batch* b, int parity, bool early, cudaStream_t st) {
+  launch_pdl(k_tile_step_batch<SF, STOCH, FD_TILE_TY>, (unsigned)b->ncells, 32 * FD_TILE_TY, st, early,
+             (const BatchInst<SF>*)b->d_inst, (const int2*)b->d_cells, parity, b->d_ctl);
 }
 
 template <typename SF, int NT, bool STOCH>
@@ -119,7 +199,7 @@ int prepare(fd_batch* b) {
   b->nwork = (int)tiles.size();
   if (b->grid > b->nwork) b->grid = b->nwork;
   if (b->grid < 1) b->grid = 1;
-  return FD_OK;
+  return prepare_cells(b, flagged);
 }
 
 template <typename SF, int NT, bool STOCH>
@@ -166,6 +246,20 @@ void launch_any(const fd_batch* b, int parity, cudaStream_t st) {
       sr ? launch_t<__nv_bfloat16, true>(b, parity, st) : launch_t<__nv_bfloat16, false>(b, parity, st);
       break;
     default: launch_t<float, false>(b, parity, st); break;
+  }
+}
+
+void launch_cells_any(const fd_batch* b, int parity, bool early, cudaStream_t st) {
+  const bool sr = stochastic(b);
+  switch (b->st.dtype) {
+    case FD_F16:
+      sr ? launch_cells<__half, true>(b, parity, early, st) : launch_cells<__half, false>(b, parity, early, st);
+      break;
+    case FD_BF16:
+      sr ? launch_cells<__nv_bfloat16, true>(b, parity, early, st)
+         : launch_cells<__nv_bfloat16, false>(b, parity, early, st);
+      break;
+    default: launch_cells<float, false>(b, parity, early, st); break;
   }
 }
 
@@ -246,6 +340,13 @@ int fd_batch_step(fd_batch* b, int nsteps, int use_graph, void* stream) {
   cudaStream_t st = as_stream(stream);
   FD_REQUIRE(!use_graph || st != nullptr, FD_ERR_ARG, "fd_batch_step: graph replay needs a non-default stream");
   int left = nsteps;
+  if (b->ncells > 0) {  // programmatic launches, whose CTAs start as the previous iteration drains, need no graph
+    for (; left > 0; --left) {
+      launch_cells_any(b, b->parity, left < nsteps, st);
+      b->parity ^= 1;
+    }
+    return check_launch("fd_batch_step");
+  }
   if (use_graph && left >= 2) {
     if (b->parity == 1) {  // the graph starts at parity 0
       launch_any(b, 1, st);
@@ -295,6 +396,7 @@ int fd_batch_destroy(fd_batch* b) {
   drop_graph(b);
   cudaFree(b->d_inst);
   cudaFree(b->d_tiles);
+  cudaFree(b->d_cells);
   cudaFree(b->d_ctl);
   cudaFree(b->d_status);
   delete b;

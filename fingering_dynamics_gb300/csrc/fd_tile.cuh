@@ -132,10 +132,10 @@ struct TilePsi {
 
 // Stores of one cell in the arithmetic of widths that are not a multiple of 8
 template <typename SF, bool STOCH, typename I>
-__device__ __forceinline__ void tile_store_scalar(const DevArgs<SF>& a, I q, const float (&f)[9],
+__device__ __forceinline__ void tile_store_scalar(const DevArgs<SF>& a, uint32_t seed, I q, const float (&f)[9],
                                                   const float (&g)[9]) {
   uint32_t rs = 0;
-  if constexpr (STOCH) rs = sr_hash((uint32_t)q ^ a.seed);
+  if constexpr (STOCH) rs = sr_hash((uint32_t)q ^ seed);
   auto conv = [&](float v, float scale) -> SF {
     if constexpr (STOCH) {
       rs = sr_next(rs);
@@ -162,14 +162,22 @@ __device__ __forceinline__ float tile_corner_drho(const DevArgs<SF>& a, int yn) 
   return dev_inlet_drho(d, (float)a.inlet_ux[yn], __ldcg(a.side_in + yn), __ldcg(a.side_in + 2 * a.H + yn));
 }
 
-// MINB: CTAs per SM that the registers are cut for (launch_tile)
-template <typename SF, bool RING, bool SCALED, bool STOCH, int TY, typename I, int MINB>
-__global__ void __launch_bounds__(32 * TY, MINB) k_tile_step(const __grid_constant__ DevArgs<SF> a, int ntx) {
+// What a step of a lattice of its own knows of its state: always stepped, the launch's seed.
+struct TileAlone {
+  uint32_t seed;
+  __device__ __forceinline__ bool stepped() const { return true; }
+  __device__ __forceinline__ uint32_t step_seed() const { return seed; }
+};
+
+// Tile `tile` (of `ntx` in a row of tiles) of one lattice.  `ready` is called
+// before the first access to the populations and returns the step's state.
+template <typename SF, bool RING, bool SCALED, bool STOCH, int TY, typename I, typename Ready>
+__device__ __forceinline__ void tile_cells_step(const DevArgs<SF>& a, int ntx, int tile, TilePsi<SF, RING, TY>& psi,
+                                                Ready ready) {
   using Psi = TilePsi<SF, RING, TY>;
   constexpr int PW = Psi::PW;
-  __shared__ Psi psi;
   const int t = threadIdx.x, lx = t & 31, ly = t >> 5;
-  const int x0 = (int)(blockIdx.x % ntx) * kTileTX, y0 = (int)(blockIdx.x / ntx) * TY;
+  const int x0 = (tile % ntx) * kTileTX, y0 = (tile / ntx) * TY;
   const int x = x0 + lx, y = y0 + ly;
   const bool walls = a.variant == FD_VARIANT_WALLS;
   const bool in = x < a.W && y < a.H;
@@ -192,9 +200,7 @@ __global__ void __launch_bounds__(32 * TY, MINB) k_tile_step(const __grid_consta
   if (hcell) hy = wrap(hy, a.H);
   const unsigned m = in ? __ldg(a.mask + (size_t)y * a.W + x) : 0u;
   const unsigned hm = hcell ? __ldg(a.mask + (size_t)hy * a.W + hx) : 0u;
-  pdl_wait();
-  // only now: a step that started before the step two before it had ended could overwrite what that one reads
-  pdl_launch_dependents();
+  const auto state = ready();
 
   float g[9], f[9];
   const TilePull<SF, I> at(x, in ? y : 0, a.H, a.W);
@@ -232,7 +238,7 @@ __global__ void __launch_bounds__(32 * TY, MINB) k_tile_step(const __grid_consta
   }
   __syncthreads();
   bool bad = false;  // a fluid cell with a non-finite rho or psi
-  if (in) {
+  if (in && state.stepped()) {
     const DevStencil st = psi.stencil(e);
     if (x == 0 || x == a.W - 1) {
       const int o = (x == 0) ? 0 : 3;
@@ -251,10 +257,27 @@ __global__ void __launch_bounds__(32 * TY, MINB) k_tile_step(const __grid_consta
       if constexpr (RING) dev_collide_for<SF>(a.c, mc, f, g);
       else dev_collide(a.c, mc, f, g);
     }
-    if constexpr (RING) store_cell<SF, SCALED, STOCH, I>(a, at.own() / (I)sizeof(SF), f, g);
-    else tile_store_scalar<SF, STOCH, I>(a, at.own() / (I)sizeof(SF), f, g);
+    if constexpr (RING) store_cell<SF, SCALED, STOCH, I>(a, state.step_seed(), at.own() / (I)sizeof(SF), f, g);
+    else tile_store_scalar<SF, STOCH, I>(a, state.step_seed(), at.own() / (I)sizeof(SF), f, g);
   }
   if (__any_sync(0xffffffffu, bad) && lx == 0) report_nonfinite(a);
+}
+
+// The previous step has ended, and the next one may start (only now: a step that
+// started before the step two before it had ended could overwrite what that one reads).
+__device__ __forceinline__ void tile_step_begins() {
+  pdl_wait();
+  pdl_launch_dependents();
+}
+
+// MINB: CTAs per SM that the registers are cut for (launch_tile)
+template <typename SF, bool RING, bool SCALED, bool STOCH, int TY, typename I, int MINB>
+__global__ void __launch_bounds__(32 * TY, MINB) k_tile_step(const __grid_constant__ DevArgs<SF> a, int ntx) {
+  __shared__ TilePsi<SF, RING, TY> psi;
+  tile_cells_step<SF, RING, SCALED, STOCH, TY, I>(a, ntx, (int)blockIdx.x, psi, [&] {
+    tile_step_begins();
+    return TileAlone{a.seed};
+  });
 }
 
 // Launch a kernel whose CTAs may start before the previous kernel of the stream

@@ -40,3 +40,27 @@ def test_tile_step_equals_the_staged_step(H, W, variant, dtype, rounding, scales
     a.exit_fused()
     b.exit_fused()
     assert torch.equal(a.f, b.f) and torch.equal(a.g, b.g) and torch.equal(a.side[a.scur], b.side[b.scur])
+
+
+@pytest.mark.parametrize("dtype,rounding", [("f32", "nearest"), ("f16", "stochastic"), ("bf16", "nearest")])
+def test_small_batch_equals_the_staged_batch(dtype, rounding):
+    """A batch small enough for the tile kernel, against the same batch in strips
+    of 31 rows (the staged kernel)."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from fingering_dynamics_gb300.ensemble import Ensemble
+    sizes = [(3, 8, "walls"), (16, 24, "walls"), (33, 136, "walls"), (64, 128, "periodic")]
+
+    def batch():
+        lats = [_lattice(H, W, v, dtype, rounding, (0, 0)) for H, W, v in sizes]
+        return Ensemble.from_lattices(lats)
+    a, b = batch(), batch()
+    b.configure(128, 31)
+    for n, graph in ((5, True), (1, False), (4, True)):
+        a.step(n, use_graph=graph)
+        b.step(n, use_graph=graph)
+    for p, q in zip(a.lattices, b.lattices):
+        p.exit_fused()
+        q.exit_fused()
+        assert not torch.isnan(p.f).any()
+        assert torch.equal(p.f, q.f) and torch.equal(p.g, q.g) and torch.equal(p.side[p.scur], q.side[q.scur])
