@@ -70,9 +70,11 @@ DevArgs<SF> instance_args(const fd_instance& in, const fd_storage& st, int rows,
 // Cells of a batch's live members up to which its iterations run on the tile
 // kernel (the staged kernel's strips leave a small batch's SMs partly idle).  us
 // per iteration, tile / staged, lattices of 256 x 512: FP32 one 6.7 / 16.4, 2 10.3 /
-// 18.5, 4 18.2 / 24.8, 8 39.6 / 44.8, 24 109 / 115, 32 143 / 146; FP16 one 7.2 /
-// 14.4, 4 17.6 / 22.6, 8 33.0 / 34.9, 16 65.0 / 64.7, 32 125 / 116.
+// 18.5, 4 17.4 / 24.4, 8 37.8 / 43.1, 24 103 / 111; FP16 one 7.2 / 14.4, 4 17.7 /
+// 22.6, 8 31.9 / 35.3, 12 50.4 / 50.4, 32 125 / 116.
 constexpr long long tile_batch_cells(int dtype) { return dtype == FD_F32 ? 4000000 : 1500000; }
+
+constexpr int kTileBatchFew = 2432;  // tiles: two rounds of 8 CTAs on each of 152 SMs
 
 // The tile kernel over a batch: a CTA copies its member's arguments to shared
 // memory while the previous iteration drains.
@@ -83,8 +85,8 @@ struct TileMember {
   __device__ __forceinline__ uint32_t step_seed() const { return seed; }
 };
 
-template <typename SF, bool STOCH, int TY>
-__global__ void __launch_bounds__(32 * TY, 8)
+template <typename SF, bool STOCH, int TY, int MINB>
+__global__ void __launch_bounds__(32 * TY, MINB)
     k_tile_step_batch(const BatchInst<SF>* __restrict__ inst, const int2* __restrict__ cells, int parity,
                       unsigned* __restrict__ ctl) {
   __shared__ TilePsi<SF, true, TY> psi;
@@ -140,8 +142,14 @@ int prepare_cells(fd_batch* b, const std::vector<unsigned>& flagged) {
 
 template <typename SF, bool STOCH>
 void launch_cells(const fd_batch* b, int parity, bool early, cudaStream_t st) {
-  launch_pdl(k_tile_step_batch<SF, STOCH, FD_TILE_TY>, (unsigned)b->ncells, 32 * FD_TILE_TY, st, early,
-             (const BatchInst<SF>*)b->d_inst, (const int2*)b->d_cells, parity, b->d_ctl);
+  auto go = [&](auto kern) {
+    launch_pdl(kern, (unsigned)b->ncells, 32 * FD_TILE_TY, 0, st, early, (const BatchInst<SF>*)b->d_inst,
+               (const int2*)b->d_cells, parity, b->d_ctl);
+  };
+  // registers for 8 or 9 CTAs per SM (launch_tile); FP32, lattices of 256 x 512: one 6.7 / 7.3 us, four 18.4 /
+  // 17.4, eight 39.5 / 37.8, 24 109 / 103; 10 is slower than 9 (40.4 for eight)
+  if (b->ncells <= kTileBatchFew) go(k_tile_step_batch<SF, STOCH, FD_TILE_TY, 8>);
+  else go(k_tile_step_batch<SF, STOCH, FD_TILE_TY, 9>);
 }
 
 template <typename SF, int NT, bool STOCH>

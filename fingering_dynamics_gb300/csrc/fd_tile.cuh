@@ -25,13 +25,11 @@
 #pragma once
 
 #include "fd_fused_tma.cuh"
+#include "fd_pdl.cuh"
 
 namespace fd {
 
 constexpr int kTileTX = 32;
-
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // The elements a cell pulls from, as byte offsets of type I from the first plane
 // (32-bit ones where nine planes are below 4 GB, which load and store
@@ -280,22 +278,6 @@ __global__ void __launch_bounds__(32 * TY, MINB) k_tile_step(const __grid_consta
   });
 }
 
-// Launch a kernel whose CTAs may start before the previous kernel of the stream
-// has ended (they wait for it in griddepcontrol.wait).
-template <typename... P, typename... A>
-cudaError_t launch_pdl(void (*kern)(P...), unsigned blocks, unsigned threads, cudaStream_t st, bool early, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(blocks);
-  cfg.blockDim = dim3(threads);
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = early ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, args...);
-}
-
 #ifndef FD_TILE_TY
 #define FD_TILE_TY 4
 #endif
@@ -325,7 +307,7 @@ int launch_tile(const fd_params& p, const DevCoef& c, const uint16_t* mask, cons
     const bool even = s % 2 == 0;
     tma_set_step(a, even ? pa : pb, even ? pb : pa, even ? sa : sb, even ? sb : sa, seed + (uint32_t)s);
     // the first step's masks may have been written by the work just before it
-    auto go = [&](auto kern) { return launch_pdl(kern, blocks, 32 * TY, st, s > 0, a, ntx); };
+    auto go = [&](auto kern) { return launch_pdl(kern, blocks, 32 * TY, 0, st, s > 0, a, ntx); };
     cudaError_t e;
     if (9 * L.pstride * sizeof(SF) >= ((size_t)1 << 32)) {
       if constexpr (RING) return FD_ERR_SHAPE;  // not reached: lattices of this size take the staged kernel
