@@ -17,8 +17,10 @@
 
 #include "../../include/fdsurrogate.h"
 #include "fd_host.h"
+#include "fd_pdl.cuh"
 
 namespace sg {
+thread_local bool t_op_follows = false;  // sg_tc.cuh
 namespace {
 
 using bf16 = __nv_bfloat16;
@@ -455,8 +457,7 @@ __global__ void k_flip(const bf16* __restrict__ w, int Cin, int Cout, bf16* __re
 struct V8 {
   float v[8];
 };
-__device__ __forceinline__ V8 ld8(const bf16* p) {
-  const uint4 u = *reinterpret_cast<const uint4*>(p);
+__device__ __forceinline__ V8 v8_of(const uint4& u) {
   const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
   V8 r;
 #pragma unroll
@@ -467,6 +468,10 @@ __device__ __forceinline__ V8 ld8(const bf16* p) {
   }
   return r;
 }
+__device__ __forceinline__ V8 ld8(const bf16* p) { return v8_of(*reinterpret_cast<const uint4*>(p)); }
+// through L2, for kernels that may start before the writer of the operand has ended
+__device__ __forceinline__ uint4 ldcg16(const bf16* p) { return __ldcg(reinterpret_cast<const uint4*>(p)); }
+__device__ __forceinline__ V8 ldcg8(const bf16* p) { return v8_of(ldcg16(p)); }
 __device__ __forceinline__ void st8(bf16* p, const V8& r) {
   uint4 u;
   __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&u);
@@ -594,14 +599,16 @@ template <typename I>
 __global__ void k_up_concat(const bf16* __restrict__ x, I n_out, I H, I W, I cg, I csg, const bf16* __restrict__ skip,
                             bf16* __restrict__ y) {
   const I i = (I)blockIdx.x * blockDim.x + threadIdx.x;  // (output pixel, group of 8 channels)
+  fd::pdl_wait();
+  fd::pdl_launch_dependents();
   if (i >= n_out) return;
   const I g = cg + csg, pix = i / g, c = i - pix * g;
   uint4 v;
   if (c < cg) {
     const I q = pix / W, xx = pix - q * W, n = q / H, yy = q - n * H;
-    v = *reinterpret_cast<const uint4*>(x + (((size_t)n * (H / 2) + yy / 2) * (W / 2) + xx / 2) * cg * 8 + (size_t)c * 8);
+    v = ldcg16(x + (((size_t)n * (H / 2) + yy / 2) * (W / 2) + xx / 2) * cg * 8 + (size_t)c * 8);
   } else {
-    v = *reinterpret_cast<const uint4*>(skip + (size_t)pix * csg * 8 + (size_t)(c - cg) * 8);
+    v = ldcg16(skip + (size_t)pix * csg * 8 + (size_t)(c - cg) * 8);
   }
   *reinterpret_cast<uint4*>(y + (size_t)i * 8) = v;
 }
@@ -611,11 +618,13 @@ __global__ void k_up_concat(const bf16* __restrict__ x, I n_out, I H, I W, I cg,
 template <typename I>
 __global__ void k_pool2(const bf16* __restrict__ x, I n_out, I h, I w, I cg, bf16* __restrict__ y) {
   const I i = (I)blockIdx.x * blockDim.x + threadIdx.x;
+  fd::pdl_wait();
+  fd::pdl_launch_dependents();
   if (i >= n_out) return;
   const I pix = i / cg, c = (i - pix * cg) * 8, q = pix / w, xo = pix - q * w, n = q / h, yo = q - n * h;
   const size_t C = (size_t)cg * 8, W = (size_t)2 * w;
   const size_t b = (((size_t)n * 2 * h + 2 * yo) * W + 2 * xo) * C + c;
-  const V8 a = ld8(x + b), bb = ld8(x + b + C), cc = ld8(x + b + W * C), d = ld8(x + b + W * C + C);
+  const V8 a = ldcg8(x + b), bb = ldcg8(x + b + C), cc = ldcg8(x + b + W * C), d = ldcg8(x + b + W * C + C);
   V8 r;
 #pragma unroll
   for (int k = 0; k < 8; ++k) r.v[k] = 0.25f * ((a.v[k] + bb.v[k]) + (cc.v[k] + d.v[k]));
@@ -770,11 +779,13 @@ __global__ void k_add_prediction(const bf16* __restrict__ x, const bf16* __restr
                                  bf16* __restrict__ y) {
   const int cg = C / 8;
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  fd::pdl_wait();
+  fd::pdl_launch_dependents();
   if (i >= P * cg) return;
-  uint4 v = *reinterpret_cast<const uint4*>(x + 8 * i);
+  uint4 v = ldcg16(x + 8 * i);
   if (cg == 1 || i % cg == 0) {
     bf16* h = reinterpret_cast<bf16*>(&v);
-    const uint2 o = *reinterpret_cast<const uint2*>(out + 8 * i);
+    const uint2 o = __ldcg(reinterpret_cast<const uint2*>(out + 8 * i));
     const bf16* oh = reinterpret_cast<const bf16*>(&o);
 #pragma unroll
     for (int c = 0; c < 3; ++c) h[c] = __float2bfloat16_rn(__bfloat162float(h[c]) + __bfloat162float(oh[c]));
@@ -920,9 +931,11 @@ int sg_pool2(const void* x, int N, int H, int W, int C, void* y, void* stream) {
   const size_t n = (size_t)N * (H / 2) * (W / 2) * (C / 8);
   cudaStream_t s = as_stream(stream);
   if (n < kIndex32)
-    k_pool2<uint32_t><<<ew_blocks(n), kEw, 0, s>>>((const bf16*)x, (uint32_t)n, H / 2, W / 2, C / 8, (bf16*)y);
+    fd::launch_pdl(k_pool2<uint32_t>, ew_blocks(n), kEw, 0, s, t_op_follows, (const bf16*)x, (uint32_t)n, (uint32_t)(H / 2),
+                   (uint32_t)(W / 2), (uint32_t)(C / 8), (bf16*)y);
   else
-    k_pool2<size_t><<<ew_blocks(n), kEw, 0, s>>>((const bf16*)x, n, H / 2, W / 2, C / 8, (bf16*)y);
+    fd::launch_pdl(k_pool2<size_t>, ew_blocks(n), kEw, 0, s, t_op_follows, (const bf16*)x, n, (size_t)(H / 2),
+                   (size_t)(W / 2), (size_t)(C / 8), (bf16*)y);
   return check_launch("sg_pool2");
 }
 
@@ -1032,11 +1045,11 @@ int sg_up2_concat(const void* x, int N, int h, int w, int C, const void* skip, i
   const size_t n = (size_t)N * 4 * h * w * ((C + Cs) / 8);
   cudaStream_t s = as_stream(stream);
   if (n < kIndex32)
-    k_up_concat<uint32_t><<<ew_blocks(n), kEw, 0, s>>>((const bf16*)x, (uint32_t)n, 2 * h, 2 * w, C / 8, Cs / 8,
-                                                       (const bf16*)skip, (bf16*)y);
+    fd::launch_pdl(k_up_concat<uint32_t>, ew_blocks(n), kEw, 0, s, t_op_follows, (const bf16*)x, (uint32_t)n,
+                   (uint32_t)(2 * h), (uint32_t)(2 * w), (uint32_t)(C / 8), (uint32_t)(Cs / 8), (const bf16*)skip, (bf16*)y);
   else
-    k_up_concat<size_t><<<ew_blocks(n), kEw, 0, s>>>((const bf16*)x, n, 2 * h, 2 * w, C / 8, Cs / 8, (const bf16*)skip,
-                                                     (bf16*)y);
+    fd::launch_pdl(k_up_concat<size_t>, ew_blocks(n), kEw, 0, s, t_op_follows, (const bf16*)x, n, (size_t)2 * h,
+                   (size_t)2 * w, (size_t)(C / 8), (size_t)(Cs / 8), (const bf16*)skip, (bf16*)y);
   return check_launch("sg_up2_concat");
 }
 
@@ -1060,8 +1073,8 @@ int sg_masked_mse_scaled(const void* x, const void* out, const void* xn, size_t 
 int sg_add_prediction(const void* x, const void* out, size_t P, int C, void* y, void* stream) {
   FD_REQUIRE(x && out && y && C >= 8 && C % 8 == 0, FD_ERR_ARG, "sg_add_prediction: bad arguments");
   if (P == 0) return FD_OK;
-  k_add_prediction<<<ew_blocks(P * (C / 8)), kEw, 0, as_stream(stream)>>>((const bf16*)x, (const bf16*)out, P, C,
-                                                                          (bf16*)y);
+  fd::launch_pdl(k_add_prediction, ew_blocks(P * (C / 8)), kEw, 0, as_stream(stream), t_op_follows, (const bf16*)x,
+                 (const bf16*)out, P, C, (bf16*)y);
   return check_launch("sg_add_prediction");
 }
 
@@ -1073,6 +1086,9 @@ int sg_to_bf16(const float* src, size_t n, void* dst, void* stream) {
 
 int sg_run(const sg_op* ops, int count, void* stream) {
   FD_REQUIRE(count >= 0 && (ops || count == 0), FD_ERR_ARG, "sg_run: bad arguments");
+  struct Follows {  // cleared on every way out
+    ~Follows() { t_op_follows = false; }
+  } follows;
   for (int k = 0; k < count; ++k) {
     const sg_op& o = ops[k];
     const int64_t* i = o.i;
@@ -1105,6 +1121,7 @@ int sg_run(const sg_op* ops, int count, void* stream) {
       default: FD_REQUIRE(false, FD_ERR_ARG, "sg_run: unknown operation %d", (int)o.kind);
     }
     if (r != FD_OK) return r;
+    t_op_follows = true;
   }
   return FD_OK;
 }

@@ -14,9 +14,15 @@
 
 #include "../../include/fdsurrogate.h"
 #include "fd_host.h"
+#include "fd_pdl.cuh"
 #include "fd_tmap.h"
 
 namespace sg {
+
+// Whether this thread is launching the second or a later operation of a list
+// (sg_run): its kernels may then start while the previous operation's drain.  An
+// operation on its own starts in stream order.
+extern thread_local bool t_op_follows;
 
 namespace {
 

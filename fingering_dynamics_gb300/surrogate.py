@@ -197,17 +197,25 @@ class UNet:
     # of each from Python costs about ten microseconds, more than its kernel on a
     # batch of one.
     def _op(self, fn, ints, tensors):
+        self._ops.extend(self._words(fn, ints, tensors))
+
+    def _words(self, fn, ints, tensors):
         o = [0] * 16
         o[0] = self._OP[fn]
         o[1:1 + len(ints)] = ints
         o[9:9 + len(tensors)] = [0 if t is None else t.data_ptr() for t in tensors]
-        self._ops.extend(o)
+        return o
 
     def _run_ops(self):
         if self._ops:
-            ops = array.array("q", self._ops)
+            words = list(self._ops)
             self._ops.clear()
-            L.call("sg_run", C.c_void_p(ops.buffer_info()[0]), len(ops) // 16, _s())
+            self._run_words(words)
+
+    @staticmethod
+    def _run_words(words):
+        ops = array.array("q", words)
+        L.call("sg_run", C.c_void_p(ops.buffer_info()[0]), len(ops) // 16, _s())
 
     @staticmethod
     def _takes(kernel, w, ci, co):
@@ -215,18 +223,20 @@ class UNet:
         multiples of 128, channel counts that are multiples of 16)."""
         return not kernel.startswith("tma") or (w % 128 == 0 and ci % 16 == 0 and co % 16 == 0)
 
-    def _fastest(self, key, fns, call):
-        """The fastest of the calls, timed once per shape on the real operands
-        (after the pass's pending operations); kept in conv_choice."""
+    def _fastest(self, key, fns, ints, tensors):
+        """The fastest of the kernels, timed once per shape on the real operands
+        (after the pass's pending operations) in a list, as a pass runs them:
+        calls of their own are bound by Python on a batch of one.  Kept in
+        conv_choice."""
         if key not in self.conv_choice:
             self._run_ops()
             best = None
             for fn in fns:
-                call(fn)
+                words = self._words(fn, ints, tensors)
+                self._run_words(words)
                 e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
                 e0.record()
-                for _ in range(2):
-                    call(fn)
+                self._run_words(words * 4)
                 e1.record()
                 e1.synchronize()
                 t = e0.elapsed_time(e1)
@@ -241,8 +251,7 @@ class UNet:
             fn = self._KERNELS[self.conv if self._takes(self.conv, w, ci, co) else "tcgen05"]
         else:
             fns = [self._KERNELS[k] for k in self._TIMED if self._takes(k, w, ci, co)]
-            fn = self._fastest((N, h, w, ci, co), fns,
-                               lambda f: L.call(f, _p(x), N, h, w, ci, _p(wt), _p(bias), co, act, _p(z), _p(y), _s()))
+            fn = self._fastest((N, h, w, ci, co), fns, (N, h, w, ci, co, act), (x, wt, bias, z, y))
         self._op(fn, (N, h, w, ci, co, act), (x, wt, bias, z, y))
 
     _WGRAD = {"mma": "sg_conv3x3_wgrad", "tcgen05": "sg_conv3x3_wgrad_tc"}
@@ -259,8 +268,7 @@ class UNet:
             fn = self._WGRAD["tcgen05"]
         else:
             fn = self._fastest(("wgrad", N, h, w, ci, co), list(self._WGRAD.values()),
-                               lambda f: L.call(f, _p(inp), _p(dz), N, h, w, ci, co, _p(gw), _p(part), part.numel(), 0,
-                                                _s()))
+                               (N, h, w, ci, co, part.numel()), (inp, dz, gw, part))
         self._op(fn, (N, h, w, ci, co, part.numel()), (inp, dz, gw, part))
 
     def _conv(self, name, x, B, act=True, keep=True):

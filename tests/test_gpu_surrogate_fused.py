@@ -117,3 +117,18 @@ def test_adamw_list_and_predict_then_backward():
     for n in LAYERS:
         assert torch.equal(net.w[n], want[n + "w"][0]) and torch.equal(net.w16[n], want[n + "w"][1])
         assert torch.equal(net.b[n], want[n + "b"][0])
+
+
+@pytest.mark.parametrize("n,h,w", [(1, 64, 128), (2, 128, 256)])
+def test_a_list_equals_its_operations(n, h, w):
+    """Operations of a list overlap (a kernel starts while the previous one
+    drains); the buffers are reused by every pass, so a missing wait would show."""
+    from fingering_dynamics_gb300.surrogate import UNet
+    net = UNet(seed=3, conv="tma")
+    net.w16["out"] = _rand(99, *net.w16["out"].shape)  # zero in a new network
+    xs = [_rand(k, n, h, w, 16) for k in range(12)]
+    listed = [net.predict(x).clone() for x in xs]
+    run = net._run_words
+    net._run_words = lambda words: [run(words[k:k + 16]) for k in range(0, len(words), 16)]
+    for x, y in zip(xs, listed):
+        assert torch.equal(net.predict(x), y)
