@@ -64,7 +64,17 @@ __device__ __forceinline__ void cv_store16(const float (&v)[16], const float* sb
   }
 }
 
-template <int BN, int R, int CH>
+// FLAT: the tile of k_conv3x3_rows at widths that are not a multiple of 128 and few
+// channels (sg_conv3x3_tc; 64 channels a chunk and up run on k_conv3x3_narrow).  bw
+// x rows pixels of an image are the first bw of every bw + 2 operand rows, so that
+// the tile's halo is still one box and every tap one window of it; the two rows
+// between are not read back.  K advances chunk by chunk, the nine taps of a chunk
+// back to back, 16 channels at a time within a tap, as in k_conv3x3_narrow.  With a
+// box per tap the copies' 32- and 64-byte rows bound the thin layers: at 32 x 200 x
+// 328, GELU, us, box per tap -> halo (the kernel fed by 16-byte copies, the
+// warp-level one; at batch 8): 16 -> 32 292 -> 132, 32 -> 32 292 -> 132 (8: 102, 89 ->
+// 40), 96 -> 32 697 -> 270 (257, 179 -> 77), 32 -> 16 267 -> 116.
+template <int BN, int R, int CH, bool FLAT>
 struct CvCfg {
   static constexpr int ROW = CH * 2;                                        // bytes of a pixel or output channel
   static constexpr int A_TX = (R + 2) * kHaloPx * ROW;
@@ -74,6 +84,7 @@ struct CvCfg {
   static constexpr int COLS = NCOL <= 32 ? 32 : (NCOL <= 64 ? 64 : (NCOL <= 128 ? 128 : (NCOL <= 256 ? 256 : 512)));
   static constexpr int S_MAX = 6;
   static constexpr int TAIL = (2 * S_MAX + 5) * 8 + BN * 4 + 16 + 1024;       // barriers, bias, TMEM address, alignment
+  static_assert(!FLAT || R == 1, "one accumulator");
   static_assert(NCOL <= 512 && TAP % (8 * ROW) == 0, "tile");
 };
 
@@ -81,13 +92,14 @@ struct CvShape {
   int N, H, W, Cin, Cout, act;
   int nk, S;       // chunks, ring stages
   int resident;    // the weights of all chunks stay in shared memory
+  int bw, rows;    // tiles of widths that are not a multiple of 128: pixels, rows
 };
 
-template <int BN, int R, int CH>
+template <int BN, int R, int CH, bool FLAT>
 __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_rows(const __grid_constant__ ConvMaps maps, const CvShape sh,
                                                                const float* __restrict__ bias, bf16* __restrict__ z,
                                                                bf16* __restrict__ y) {
-  using C = CvCfg<BN, R, CH>;
+  using C = CvCfg<BN, R, CH, FLAT>;
   extern __shared__ char smem_raw[];
   char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const int S = sh.S, nk = sh.nk, stage = C::A_BYTES + (sh.resident ? 0 : C::B_BYTES);
@@ -98,8 +110,10 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_rows(const __grid_con
   float* sbias = reinterpret_cast<float*>(wfull + 1);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sbias + BN);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tiles_x = sh.W / kTcBM, nco = sh.Cout / BN;
-  const int ntiles = sh.N * (sh.H / R) * tiles_x * nco;
+  const int tw = FLAT ? sh.bw : kTcBM, rows = FLAT ? sh.rows : R, pitch = FLAT ? sh.bw + 2 : kHaloPx;
+  const int tiles_x = FLAT ? (sh.W + tw - 1) / tw : sh.W / kTcBM, tiles_y = FLAT ? (sh.H + rows - 1) / rows : sh.H / R;
+  const int nco = sh.Cout / BN;
+  const int ntiles = sh.N * tiles_y * tiles_x * nco;
   const int mine = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;  // this CTA's tiles
   // the grid is a multiple of the output-channel tiles, so a CTA keeps one of them
   const int co0 = ((int)blockIdx.x % nco) * BN;
@@ -125,11 +139,12 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_rows(const __grid_con
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
 
-  // tile j of this CTA -> (first output row n H + yy, x0)
-  auto tile_of = [&](int j, int& row, int& x0) {
-    const int pt = ((int)blockIdx.x + j * (int)gridDim.x) / nco;
-    x0 = (pt % tiles_x) * kTcBM;
-    row = (pt / tiles_x) * R;
+  // tile j of this CTA -> image n, first row yy, first pixel x0
+  auto tile_of = [&](int j, int& n, int& yy, int& x0) {
+    const int pt = ((int)blockIdx.x + j * (int)gridDim.x) / nco, py = pt / tiles_x;
+    x0 = (pt - py * tiles_x) * tw;
+    n = py / tiles_y;
+    yy = (py - n * tiles_y) * rows;
   };
 
   if (warp == kCvEpiWarps) {
@@ -142,13 +157,12 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_rows(const __grid_con
         mbar_expect_tx(wfull, (unsigned)(nk * 9 * C::TAP));
         for (int kc = 0; kc < nk; ++kc) load_b(wres + kc * C::B_BYTES, kc, wfull);
       }
-      const unsigned tx = (unsigned)(C::A_TX + (sh.resident ? 0 : 9 * C::TAP));
+      const unsigned tx = (unsigned)((FLAT ? (rows + 2) * pitch * C::ROW : C::A_TX) + (sh.resident ? 0 : 9 * C::TAP));
       int c = 0;  // chunks issued
       bool ok = true;
       for (int j = 0; j < mine && ok; ++j) {
-        int row, x0;
-        tile_of(j, row, x0);
-        const int n = row / sh.H, yy = row % sh.H;
+        int n, yy, x0;
+        tile_of(j, n, yy, x0);
         for (int kc = 0; kc < nk; ++kc, ++c) {
           const int st = c % S;
           if (c >= S) ok = mbar_wait_ok(&empty[st], (unsigned)(c / S - 1) & 1u, true);
@@ -186,16 +200,27 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_rows(const __grid_con
         const uint64_t as = a0 + (uint64_t)(st * stage / 16);
         const uint64_t bs = w0 + (uint64_t)((sh.resident ? kc * C::B_BYTES : st * stage) / 16);
         if (leader) {
-#pragma unroll
-          for (int s = 0; s < CH / 16; ++s) {
+          if constexpr (FLAT) {
 #pragma unroll
             for (int tap = 0; tap < 9; ++tap) {
-              const int ky = tap / 3, kx = tap % 3;
-              const uint32_t acc = (s > 0 || tap > 0) ? 1u : (kc > 0 ? 1u : 0u);
+              const uint64_t at = as + (uint64_t)(((tap / 3) * pitch + tap % 3) * C::ROW / 16);
 #pragma unroll
-              for (int r = 0; r < R; ++r)
-                tc_mma(d0 + (uint32_t)(r * BN), as + (uint64_t)((((r + ky) * kHaloPx + kx) * C::ROW + s * 32) / 16),
-                       bs + (uint64_t)((tap * C::TAP + s * 32) / 16), idesc, acc);
+              for (int s = 0; s < CH / 16; ++s)
+                tc_mma(d0, at + (uint64_t)(s * 2), bs + (uint64_t)((tap * C::TAP + s * 32) / 16), idesc,
+                       (s > 0 || tap > 0) ? 1u : (kc > 0 ? 1u : 0u));
+            }
+          } else {
+#pragma unroll
+            for (int s = 0; s < CH / 16; ++s) {
+#pragma unroll
+              for (int tap = 0; tap < 9; ++tap) {
+                const int ky = tap / 3, kx = tap % 3;
+                const uint32_t acc = (s > 0 || tap > 0) ? 1u : (kc > 0 ? 1u : 0u);
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                  tc_mma(d0 + (uint32_t)(r * BN), as + (uint64_t)((((r + ky) * kHaloPx + kx) * C::ROW + s * 32) / 16),
+                         bs + (uint64_t)((tap * C::TAP + s * 32) / 16), idesc, acc);
+              }
             }
           }
           tc_commit(&empty[st]);
@@ -211,10 +236,12 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_rows(const __grid_con
     // epilogue: warp w reads TMEM lanes 32 q .. 32 q + 31 (pixels x0 + 32 q + lane of each row, q = w % 4) of every
     // second group of 16 columns (w / 4)
     const int q = warp & 3, h = warp >> 2;
+    const int m = q * 32 + lane, my = FLAT ? m / pitch : 0, mx = m - my * pitch;
     for (int j = 0; j < mine; ++j) {
       const int b = j & 1;
-      int row, x0;
-      tile_of(j, row, x0);
+      int n, yy, x0;
+      tile_of(j, n, yy, x0);
+      const bool in = !FLAT || (mx < tw && my < rows && yy + my < sh.H && x0 + mx < sh.W);
       mbar_wait_ok(&accf[b], (unsigned)(j >> 1) & 1u, true);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
@@ -222,8 +249,8 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_rows(const __grid_con
         const int r = i / (BN / 16), c0 = (i % (BN / 16)) * 16;
         float v[16];
         tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * R * BN + i * 16), v);
-        const size_t o = ((size_t)(row + r) * sh.W + x0 + q * 32 + lane) * sh.Cout + co0 + c0;
-        cv_store16(v, sbias + c0, sh.act, z, y, o);
+        const size_t o = (((size_t)n * sh.H + yy + r + my) * sh.W + x0 + mx) * sh.Cout + co0 + c0;
+        if (in) cv_store16(v, sbias + c0, sh.act, z, y, o);
       }
       // this warp's reads of buffer b are complete (tcgen05.wait::ld in tmem_ld16)
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -239,22 +266,23 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_rows(const __grid_con
 }
 
 // ---------------------------------------------------------------------------
-// Narrow images (widths 8, 16, 32 and 64; sg_conv3x3_tc): a tile is 128 pixels,
-// 128 / W rows of one image.  A halo would not be 128 evenly spaced operand rows,
-// so a stage is one tap of a chunk of BK channels: a box of the tile's pixels
-// shifted by the tap (zeros outside the image), 128 rows of BK channels, and the
-// tap's weights.  K advances chunk by chunk, the nine taps of a chunk back to
-// back, 16 channels at a time within a tap, as in k_conv3x3_tc, which all threads
-// fed by 16-byte copies: at 32 x 32 x 64, us, 128 -> 256 channels 247 -> 50, 256 ->
-// 256 445 -> 71, 256 -> 128 255 -> 38 (the warp-level kernel 157, 283, 143); one image,
-// 256 -> 256, 48 -> 14.5 (25).
+// Widths that are not a multiple of 128 (sg_conv3x3_tc): a tile is bw x rows pixels
+// of one image, at most 128 (tile_box), and ends with the image.  A halo would not
+// be evenly spaced operand rows, so a stage is one tap of a chunk of BK channels: a
+// box of the tile's pixels shifted by the tap (zeros outside the image) and the
+// tap's weights; operand rows past the tile hold whatever the stage held before and
+// their sums are not read.  K advances chunk by chunk, the nine taps of a chunk
+// back to back, 16 channels at a time within a tap, as in the kernel it replaced,
+// which all threads fed by 16-byte copies: at 32 x 32 x 64, us, 128 -> 256 channels
+// 247 -> 50, 256 -> 256 445 -> 71, 256 -> 128 255 -> 38 (the warp-level kernel 157,
+// 283, 143); one image, 256 -> 256, 48 -> 14.5 (25); at 8 x 50 x 82, 128 -> 128 77 -> 20
+// (48), 384 -> 128 189 -> 34 (118).
 // Same roles as k_conv3x3_rows.
 // ---------------------------------------------------------------------------
 template <int BN, int BK>
 struct CnCfg {
   static constexpr int ROW = BK * 2;
   static constexpr int A_BYTES = kTcBM * ROW, B_BYTES = (BN * ROW + 1023) / 1024 * 1024, STAGE = A_BYTES + B_BYTES;
-  static constexpr uint32_t TX = (uint32_t)(A_BYTES + BN * ROW);
   static constexpr int COLS = 2 * BN < 32 ? 32 : 2 * BN;
   static constexpr int S = 220 * 1024 / STAGE > 8 ? 8 : 220 * 1024 / STAGE;
   static constexpr int OFF_BAR = S * STAGE;
@@ -275,8 +303,9 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_narrow(const __grid_c
   float* sbias = reinterpret_cast<float*>(acce + 2);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sbias + BN);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int rows = kTcBM / sh.W, tiles_y = (sh.H + rows - 1) / rows, nco = sh.Cout / BN;
-  const int ntiles = sh.N * tiles_y * nco, nst = sh.nk * 9;  // stages of a tile
+  const int bw = sh.bw, rows = sh.rows, tiles_x = (sh.W + bw - 1) / bw, tiles_y = (sh.H + rows - 1) / rows;
+  const int nco = sh.Cout / BN;
+  const int ntiles = sh.N * tiles_y * tiles_x * nco, nst = sh.nk * 9;  // stages of a tile
   const int mine = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
   const int co0 = ((int)blockIdx.x % nco) * BN;  // the grid is a multiple of the output-channel tiles
 
@@ -299,27 +328,29 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_narrow(const __grid_c
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  // tile j of this CTA -> image n, first row y0
-  auto tile_of = [&](int j, int& n, int& y0) {
-    const int pt = ((int)blockIdx.x + j * (int)gridDim.x) / nco;
-    n = pt / tiles_y;
-    y0 = (pt % tiles_y) * rows;
+  // tile j of this CTA -> image n, first row y0, first pixel x0
+  auto tile_of = [&](int j, int& n, int& y0, int& x0) {
+    const int pt = ((int)blockIdx.x + j * (int)gridDim.x) / nco, py = pt / tiles_x;
+    x0 = (pt - py * tiles_x) * bw;
+    n = py / tiles_y;
+    y0 = (py - n * tiles_y) * rows;
   };
 
   if (warp == kCvEpiWarps) {
     if (lane == 0 && mine > 0) {
+      const uint32_t tx = (uint32_t)((bw * rows + BN) * C::ROW);
       int c = 0;
       bool ok = true;
       for (int j = 0; j < mine && ok; ++j) {
-        int n, y0;
-        tile_of(j, n, y0);
+        int n, y0, x0;
+        tile_of(j, n, y0, x0);
         for (int k = 0; k < nst; ++k, ++c) {
           const int st = c % S, kc = k / 9, tap = k % 9;
           if (c >= S) ok = mbar_wait_ok(&empty[st], (unsigned)(c / S - 1) & 1u, true);
           if (!ok) break;
           char* a = smem + st * C::STAGE;
-          mbar_expect_tx(&full[st], C::TX);
-          tma_load_4d(a, &maps.x, kc * BK, tap % 3 - 1, y0 + tap / 3 - 1, n, &full[st]);
+          mbar_expect_tx(&full[st], tx);
+          tma_load_4d(a, &maps.x, kc * BK, x0 + tap % 3 - 1, y0 + tap / 3 - 1, n, &full[st]);
           tma_load_3d(a + C::A_BYTES, &maps.w, kc * BK, tap, co0, &full[st]);
         }
       }
@@ -359,21 +390,21 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_narrow(const __grid_c
       mbar_wait_ok(&empty[i], (unsigned)((c - 1 - ((c - 1 - i) % S)) / S) & 1u, false);
   } else {
     const int q = warp & 3, h = warp >> 2;
-    const int m = q * 32 + lane;  // pixel of the tile
+    const int m = q * 32 + lane, my = m / bw, mx = m - my * bw;  // pixel of the tile
     for (int j = 0; j < mine; ++j) {
       const int b = j & 1;
-      int n, y0;
-      tile_of(j, n, y0);
+      int n, y0, x0;
+      tile_of(j, n, y0, x0);
       mbar_wait_ok(&accf[b], (unsigned)(j >> 1) & 1u, true);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int yy = y0 + m / sh.W;
+      const int yy = y0 + my, xx = x0 + mx;
+      const bool in = my < rows && yy < sh.H && xx < sh.W;
 #pragma unroll 1
       for (int i = h; i < BN / 16; i += 2) {
         float v[16];
         tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + i * 16), v);
-        if (yy < sh.H)
-          cv_store16(v, sbias + i * 16, sh.act, z, y,
-                     (((size_t)n * sh.H + yy) * sh.W + m % sh.W) * sh.Cout + co0 + i * 16);
+        if (in)
+          cv_store16(v, sbias + i * 16, sh.act, z, y, (((size_t)n * sh.H + yy) * sh.W + xx) * sh.Cout + co0 + i * 16);
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
@@ -425,15 +456,15 @@ struct CvCall {
   int sms;
 };
 
-template <int BN, int R, int CH>
-int launch_rows(const CvCall& c) {
-  using C = CvCfg<BN, R, CH>;
-  auto kern = k_conv3x3_rows<BN, R, CH>;
+template <int BN, int R, int CH, bool FLAT = false>
+int launch_rows(const CvCall& c, int bw = kTcBM, int rows = R) {
+  using C = CvCfg<BN, R, CH, FLAT>;
+  auto kern = k_conv3x3_rows<BN, R, CH, FLAT>;
   static std::atomic<unsigned long long> attr_done{0};
   if (fd::ensure_smem_attr(kern, 227 * 1024, attr_done) != cudaSuccess)
     return fd::check_launch("sg_conv3x3_tma: shared-memory attribute");
   constexpr int kRoom = 227 * 1024 - C::TAIL;
-  CvShape sh{c.N, c.H, c.W, c.Cin, c.Cout, c.act, c.Cin / CH, 0, 0};
+  CvShape sh{c.N, c.H, c.W, c.Cin, c.Cout, c.act, c.Cin / CH, 0, 0, bw, rows};
   // the weights stay where two stages of the ring fit beside them (or all the chunks there are)
   const int need = sh.nk < 2 ? 1 : 2;
   sh.resident = sh.nk * C::B_BYTES + need * C::A_BYTES <= kRoom;
@@ -444,10 +475,10 @@ int launch_rows(const CvCall& c) {
     return FD_ERR_SHAPE;
   }
   const int nco = c.Cout / BN;
-  const long long ntiles = (long long)c.N * (c.H / R) * (c.W / kTcBM) * nco;
+  const long long ntiles = (long long)c.N * ((c.H + rows - 1) / rows) * ((c.W + bw - 1) / bw) * nco;
   const long long grid = std::min<long long>(ntiles, std::max(1, c.sms / nco) * (long long)nco);
   ConvMaps maps;
-  if (int r = encode_conv_maps(maps, c.x, c.N, c.H, c.W, c.Cin, c.w, c.Cout, kHaloPx, R + 2, BN, CH)) return r;
+  if (int r = encode_conv_maps(maps, c.x, c.N, c.H, c.W, c.Cin, c.w, c.Cout, bw + 2, rows + 2, BN, CH)) return r;
   fd::launch_pdl(kern, (unsigned)grid, kCvThreads, 227 * 1024, c.s, t_op_follows, maps, sh, c.b, c.z, c.y);
   return fd::check_launch("sg_conv3x3_tma");
 }
@@ -475,19 +506,35 @@ int rows_n(const CvCall& c) {
   return rows_r<16, CH>(c);
 }
 
+// The tile of a width: W in equal parts (the last may be shorter), as many rows as
+// fit 128 operand rows at a pitch of the part plus `gap`; the parts that give the
+// fewest tiles.
+inline void tile_box(int H, int W, int gap, int& bw, int& rows) {
+  long long best = 0;
+  for (int k = (W + kTcBM - 1) / kTcBM; k <= 16 && k <= W; ++k) {
+    const int w = (W + k - 1) / k, r = std::min((kTcBM + gap) / (w + gap), 254);
+    const long long tiles = (long long)((W + w - 1) / w) * ((H + r - 1) / r);
+    if (best == 0 || tiles < best) {
+      best = tiles;
+      bw = w;
+      rows = r;
+    }
+  }
+}
+
 template <int BN, int BK>
-int launch_narrow(const CvCall& c) {
+int launch_narrow(const CvCall& c, int bw, int rows) {
   using C = CnCfg<BN, BK>;
   auto kern = k_conv3x3_narrow<BN, BK>;
   static std::atomic<unsigned long long> attr_done{0};
   if (fd::ensure_smem_attr(kern, 227 * 1024, attr_done) != cudaSuccess)
     return fd::check_launch("sg_conv3x3_tc: shared-memory attribute");
-  const int rows = kTcBM / c.W, nco = c.Cout / BN;
-  const CvShape sh{c.N, c.H, c.W, c.Cin, c.Cout, c.act, c.Cin / BK, C::S, 0};
-  const long long ntiles = (long long)c.N * ((c.H + rows - 1) / rows) * nco;
+  const int nco = c.Cout / BN;
+  const CvShape sh{c.N, c.H, c.W, c.Cin, c.Cout, c.act, c.Cin / BK, C::S, 0, bw, rows};
+  const long long ntiles = (long long)c.N * ((c.H + rows - 1) / rows) * ((c.W + bw - 1) / bw) * nco;
   const long long grid = std::min<long long>(ntiles, std::max(1, c.sms / nco) * (long long)nco);
   ConvMaps maps;
-  if (int r = encode_conv_maps(maps, c.x, c.N, c.H, c.W, c.Cin, c.w, c.Cout, c.W, rows, BN, BK)) return r;
+  if (int r = encode_conv_maps(maps, c.x, c.N, c.H, c.W, c.Cin, c.w, c.Cout, bw, rows, BN, BK)) return r;
   fd::launch_pdl(kern, (unsigned)grid, kCvThreads, 227 * 1024, c.s, t_op_follows, maps, sh, c.b, c.z, c.y);
   return fd::check_launch("sg_conv3x3_tc");
 }
@@ -496,11 +543,23 @@ int launch_narrow(const CvCall& c) {
 // (a batch of one at 32 x 64 has 16 tiles of pixels).
 template <int BK>
 int narrow_n(const CvCall& c) {
-  const long long px_tiles = (long long)c.N * ((c.H + kTcBM / c.W - 1) / (kTcBM / c.W));
-  if (c.Cout % 128 == 0 && px_tiles * (c.Cout / 128) >= c.sms) return launch_narrow<128, BK>(c);
-  if (c.Cout % 64 == 0 && px_tiles * (c.Cout / 64) >= c.sms / 2) return launch_narrow<64, BK>(c);
-  if (c.Cout % 32 == 0) return launch_narrow<32, BK>(c);
-  return launch_narrow<16, BK>(c);
+  int bw = 1, rows = kTcBM;
+  tile_box(c.H, c.W, 0, bw, rows);
+  const long long px_tiles = (long long)c.N * ((c.H + rows - 1) / rows) * ((c.W + bw - 1) / bw);
+  if (c.Cout % 128 == 0 && px_tiles * (c.Cout / 128) >= c.sms) return launch_narrow<128, BK>(c, bw, rows);
+  if (c.Cout % 64 == 0 && px_tiles * (c.Cout / 64) >= c.sms / 2) return launch_narrow<64, BK>(c, bw, rows);
+  if (c.Cout % 32 == 0) return launch_narrow<32, BK>(c, bw, rows);
+  return launch_narrow<16, BK>(c, bw, rows);
+}
+
+template <int CH>
+int flat_n(const CvCall& c) {
+  int bw = 1, rows = 1;
+  tile_box(c.H, c.W, 2, bw, rows);
+  const long long px_tiles = (long long)c.N * ((c.H + rows - 1) / rows) * ((c.W + bw - 1) / bw);
+  if (c.Cout % 64 == 0 && px_tiles * (c.Cout / 64) >= c.sms / 2) return launch_rows<64, 1, CH, true>(c, bw, rows);
+  if (c.Cout % 32 == 0) return launch_rows<32, 1, CH, true>(c, bw, rows);
+  return launch_rows<16, 1, CH, true>(c, bw, rows);
 }
 
 void set_sms(CvCall& c) {
@@ -526,13 +585,13 @@ int conv_rows(const void* x, int N, int H, int W, int Cin, const void* w, const 
 
 int conv_error_word(unsigned* out, bool clear) { return tc_error_word(out, clear); }
 
-// sg_conv3x3_tc on the widths that divide 128 (arguments checked by the caller).
+// sg_conv3x3_tc on widths that are not a multiple of 128 (arguments checked by the caller).
 int conv_narrow(const void* x, int N, int H, int W, int Cin, const void* w, const float* bias, int Cout, int act, void* z,
                 void* y, cudaStream_t s) {
   CvCall c{(const bf16*)x, N, H, W, Cin, (const bf16*)w, bias, Cout, act, (bf16*)z, (bf16*)y, s, 1};
   set_sms(c);
   if (Cin % 64 == 0) return narrow_n<64>(c);
-  return Cin % 32 == 0 ? narrow_n<32>(c) : narrow_n<16>(c);
+  return Cin % 32 == 0 ? flat_n<32>(c) : flat_n<16>(c);
 }
 
 }  // namespace sg

@@ -1,22 +1,13 @@
 // 3x3 convolution (forward and data gradient) of the learned surrogate on the
-// fifth-generation tensor cores: tcgen05.mma with bfloat16 operands read from
-// shared memory through matrix descriptors and the FP32 accumulator in tensor
-// memory (TMEM).
+// fifth-generation tensor cores, widths that are multiples of 128, fed by
+// 16-byte copies of all threads (sg_conv3x3_tc; its other widths run on the
+// kernels of sg_conv.cu): tcgen05.mma with bfloat16 operands read from shared
+// memory through matrix descriptors and the FP32 accumulator in tensor memory.
 //
-// Implicit GEMM, M = pixels, N = output channels, K = 9 x input channels.  A
-// CTA of 128 threads owns 128 pixels x BN channels; the accumulator is 128
-// TMEM lanes x BN columns.  K advances in chunks of BK input channels of one
-// tap (the nine taps of a channel chunk back to back): all threads copy the
-// chunk's A (im2col rows) and B (weights) tiles into shared memory with
-// cp.async, in the canonical K-major layout without swizzle (core matrices
-// of 8 rows x 16 bytes; LBO = 128 B between the two core matrices of a K=16
-// slice, SBO = BK/8 x 128 B between 8-row groups), make them visible to the
-// async proxy, and one thread issues BK/16 MMAs (M=128, N=BN, K=16) and
-// commits them to the stage's mbarrier.  Four stages: three chunks are in
-// flight while one is multiplied, and a stage is refilled once the MMAs that
-// read it have completed.  The epilogue reads the accumulator
-// with tcgen05.ld (each warp its 32 lanes = 32 pixels), adds the bias,
-// applies GELU and stores bfloat16.
+// Implicit GEMM, M = pixels, N = output channels, K = 9 x input channels.  Operands
+// are in the canonical K-major layout without swizzle (core matrices of 8 rows x
+// 16 bytes).  The epilogue reads the accumulators with tcgen05.ld (each warp its
+// 32 lanes = 32 pixels), adds the bias, applies GELU and stores bfloat16.
 #include "sg_tc.cuh"
 
 namespace sg {
@@ -28,181 +19,14 @@ int conv_narrow(const void* x, int N, int H, int W, int Cin, const void* w, cons
 
 namespace {
 
-constexpr int kTcStages = 4;
-
-template <int BN, int BK>
-struct TcCfg {
-  static constexpr int S = kTcStages;
-  static constexpr int A_BYTES = kTcBM * BK * 2;  // 128 rows x BK bfloat16
-  static constexpr int B_BYTES = BN * BK * 2;
-  static constexpr int STAGE = A_BYTES + B_BYTES;
-  static constexpr int SBO = (BK / 8) * 128;       // bytes between 8-row groups
-  static constexpr int LBO = 128;                  // bytes between the K=0..7 and K=8..15 core matrices
-  static constexpr int SMEM = S * STAGE + 128;     // stages + barriers + TMEM address
-  static constexpr int COLS = BN < 32 ? 32 : BN;   // TMEM columns (power of two >= 32)
-  static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "N of an M=128 MMA");
-  static_assert(BK % 16 == 0, "K chunk");
-};
-
 // byte offset of element (row, k) in a canonical K-major tile
 template <int BK>
 __device__ __forceinline__ uint32_t tile_off(int row, int k) {
   return (uint32_t)((row & 7) * 16 + (row >> 3) * ((BK / 8) * 128) + (k >> 3) * 128 + (k & 7) * 2);
 }
 
-template <int BN, int BK>
-__global__ void __launch_bounds__(kTcThreads) k_conv3x3_tc(const bf16* __restrict__ x, int N, int H, int W,
-                                                          int Cin, const bf16* __restrict__ w,
-                                                          const float* __restrict__ bias, int Cout, int act,
-                                                          bf16* __restrict__ z, bf16* __restrict__ y) {
-  using C = TcCfg<BN, BK>;
-  extern __shared__ __align__(1024) char smem[];
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::S * C::STAGE);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::S * C::STAGE + 8 * C::S);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const long long M = (long long)N * H * W;
-  const long long m0 = (long long)blockIdx.x * kTcBM;
-  const int co0 = blockIdx.y * BN;
-  const int nk = 9 * (Cin / BK);
-
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(C::COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  if (tid == 0) {
-    for (int i = 0; i < C::S; ++i) mbar_init(&bars[i]);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tmem_slot;
-
-  // this thread's A rows: pixel bases at the centre tap and tap-validity masks
-  constexpr int VPR = BK / 8;
-  constexpr int A_PER = kTcBM * VPR / kTcThreads;
-  static_assert(A_PER * kTcThreads == kTcBM * VPR, "A vectors per thread");
-  const bf16* a_base[A_PER];
-  uint32_t a_valid[A_PER], a_soff[A_PER];
-#pragma unroll
-  for (int i = 0; i < A_PER; ++i) {
-    const int v = tid + i * kTcThreads;
-    const int row = v / VPR, kv = v % VPR;
-    const long long p = m0 + row;
-    a_soff[i] = tile_off<BK>(row, kv * 8);
-    a_base[i] = x;
-    a_valid[i] = 0u;
-    if (p < M) {
-      const int rem = (int)(p % ((long long)H * W));
-      const int yy = rem / W, xx = rem % W;
-      a_base[i] = x + p * Cin + kv * 8;
-#pragma unroll
-      for (int t = 0; t < 9; ++t) {
-        const int ty = yy + t / 3 - 1, tx = xx + t % 3 - 1;
-        if (ty >= 0 && ty < H && tx >= 0 && tx < W) a_valid[i] |= 1u << t;
-      }
-    }
-  }
-
-  auto load_chunk = [&](int kc, int st) {
-    char* As = smem + st * C::STAGE;
-    char* Bs = As + C::A_BYTES;
-    const int tap = kc % 9, ci0 = (kc / 9) * BK;
-    const long long toff = ((long long)(tap / 3 - 1) * W + (tap % 3 - 1)) * Cin + ci0;
-#pragma unroll
-    for (int i = 0; i < A_PER; ++i) {
-      const bool ok = (a_valid[i] >> tap) & 1u;
-      cp16_l1(As + a_soff[i], ok ? a_base[i] + toff : x, ok ? 16 : 0);
-    }
-    for (int v = tid; v < BN * VPR; v += kTcThreads) {
-      const int r = v / VPR, kv = v % VPR;
-      cp16(Bs + tile_off<BK>(r, kv * 8), w + ((long long)(co0 + r) * 9 + tap) * Cin + ci0 + kv * 8);
-    }
-  };
-
-  constexpr uint32_t idesc = instr_desc<kTcBM, BN>();
-  unsigned phase = 0;  // bit s: parity of the next completion of stage s
-  auto wait_stage = [&](int s) {
-    mbar_wait(&bars[s], (phase >> s) & 1u);
-    phase ^= 1u << s;
-  };
-  // prologue: chunks 0 .. S-2 in flight
-#pragma unroll
-  for (int i = 0; i < C::S - 1; ++i) {
-    if (i < nk) load_chunk(i, i);
-    cp_commit();
-  }
-  for (int kc = 0; kc < nk; ++kc) {
-    const int st = kc % C::S;
-    const int nxt = kc + C::S - 1;  // refills the stage chunk kc-1 used
-    if (nxt < nk) {
-      if (kc >= 1) wait_stage((kc - 1) % C::S);
-      load_chunk(nxt, nxt % C::S);
-    }
-    cp_commit();
-    cp_wait<C::S - 1>();  // chunk kc has landed
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // cp.async data -> tensor core reads
-    __syncthreads();
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t a0 = smem_u32(smem + st * C::STAGE), b0 = a0 + C::A_BYTES;
-#pragma unroll
-      for (int s = 0; s < BK / 16; ++s) {
-        const uint64_t ad = smem_desc(a0 + s * 2 * C::LBO, C::LBO, C::SBO);
-        const uint64_t bd = smem_desc(b0 + s * 2 * C::LBO, C::LBO, C::SBO);
-        tc_mma(tmem, ad, bd, idesc, (kc > 0 || s > 0) ? 1u : 0u);
-      }
-      tc_commit(&bars[st]);
-    }
-  }
-  // the commits not waited for in the loop: chunks max(0, nk-S) .. nk-1
-  for (int c = (nk > C::S ? nk - C::S : 0); c < nk; ++c) wait_stage(c % C::S);
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-
-  // epilogue: warp w holds pixels m0 + 32 w + lane
-  const long long p = m0 + warp * 32 + lane;
-#pragma unroll
-  for (int c0 = 0; c0 < BN; c0 += 16) {
-    float v[16];
-    tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-    if (p < M) {
-      const int co = co0 + c0;
-      uint32_t zw[8], yw[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        float t0 = v[2 * i] + (bias ? bias[co + 2 * i] : 0.0f);
-        float t1 = v[2 * i + 1] + (bias ? bias[co + 2 * i + 1] : 0.0f);
-        const __nv_bfloat162 zp = __floats2bfloat162_rn(t0, t1);
-        zw[i] = *reinterpret_cast<const uint32_t*>(&zp);
-        if (act == SG_ACT_GELU) {
-          t0 = gelu_f(t0);
-          t1 = gelu_f(t1);
-        }
-        const __nv_bfloat162 yp = __floats2bfloat162_rn(t0, t1);
-        yw[i] = *reinterpret_cast<const uint32_t*>(&yp);
-      }
-      const size_t o = (size_t)p * Cout + co;
-      if (z) {
-        reinterpret_cast<uint4*>(z + o)[0] = make_uint4(zw[0], zw[1], zw[2], zw[3]);
-        reinterpret_cast<uint4*>(z + o)[1] = make_uint4(zw[4], zw[5], zw[6], zw[7]);
-      }
-      if (y) {
-        reinterpret_cast<uint4*>(y + o)[0] = make_uint4(yw[0], yw[1], yw[2], yw[3]);
-        reinterpret_cast<uint4*>(y + o)[1] = make_uint4(yw[4], yw[5], yw[6], yw[7]);
-      }
-    }
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == 0) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C::COLS) : "memory");
-  }
-}
-
 // ---------------------------------------------------------------------------
-// Halo-tile variant for images whose width is a multiple of 128: a CTA owns
+// A CTA owns
 // 128 pixels of one image row.  Per input-channel chunk it copies the three
 // input rows y-1, y, y+1 over 130 pixels (x0-1 .. x0+128, zeros outside the
 // image) once, and the weights of all nine taps; each tap's A operand is the
@@ -381,28 +205,6 @@ int launch_tch(const bf16* x, int N, int H, int W, int Cin, const bf16* w, const
   return launch_tch_r<BN, BK, 1>(x, N, H, W, Cin, w, b, Cout, act, z, y, s);
 }
 
-template <int BN, int BK>
-int launch_tc(const bf16* x, int N, int H, int W, int Cin, const bf16* w, const float* b, int Cout, int act,
-              bf16* z, bf16* y, cudaStream_t s) {
-  using C = TcCfg<BN, BK>;
-  auto kern = k_conv3x3_tc<BN, BK>;
-  static std::atomic<unsigned long long> attr_done{0};
-  if (fd::ensure_smem_attr(kern, C::SMEM, attr_done) != cudaSuccess)
-    return fd::check_launch("sg_conv3x3_tc: shared-memory attribute");
-  const long long M = (long long)N * H * W;
-  dim3 grid((unsigned)((M + kTcBM - 1) / kTcBM), (unsigned)(Cout / BN));
-  kern<<<grid, kTcThreads, C::SMEM, s>>>(x, N, H, W, Cin, w, b, Cout, act, z, y);
-  return fd::check_launch("sg_conv3x3_tc");
-}
-
-template <int BK>
-int tc_bk(const bf16* x, int N, int H, int W, int Cin, const bf16* w, const float* b, int Cout, int act, bf16* z,
-          bf16* y, cudaStream_t s) {
-  if (Cout % 64 == 0) return launch_tc<64, BK>(x, N, H, W, Cin, w, b, Cout, act, z, y, s);
-  if (Cout % 32 == 0) return launch_tc<32, BK>(x, N, H, W, Cin, w, b, Cout, act, z, y, s);
-  return launch_tc<16, BK>(x, N, H, W, Cin, w, b, Cout, act, z, y, s);
-}
-
 }  // namespace
 }  // namespace sg
 
@@ -430,10 +232,7 @@ int sg_conv3x3_tc(const void* x, int N, int H, int W, int Cin, const void* w, co
     if (Cout % 32 == 0) return sg::launch_tch<32, 16>(xb, N, H, W, Cin, wb, bias, Cout, act, zb, yb, s);
     return sg::launch_tch<16, 16>(xb, N, H, W, Cin, wb, bias, Cout, act, zb, yb, s);
   }
-  if (W >= 8 && sg::kTcBM % W == 0) return sg::conv_narrow(x, N, H, W, Cin, w, bias, Cout, act, z, y, s);
-  if (Cin % 64 == 0) return sg::tc_bk<64>(xb, N, H, W, Cin, wb, bias, Cout, act, (bf16*)z, (bf16*)y, s);
-  if (Cin % 32 == 0) return sg::tc_bk<32>(xb, N, H, W, Cin, wb, bias, Cout, act, (bf16*)z, (bf16*)y, s);
-  return sg::tc_bk<16>(xb, N, H, W, Cin, wb, bias, Cout, act, (bf16*)z, (bf16*)y, s);
+  return sg::conv_narrow(x, N, H, W, Cin, w, bias, Cout, act, z, y, s);
 }
 
 int sg_tc_status(unsigned* out, int clear) {
