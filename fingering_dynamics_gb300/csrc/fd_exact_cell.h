@@ -22,7 +22,11 @@
 // bits below the normal range.  exact_cell() therefore checks the exponents of
 // the quantities they act on and returns false where one is outside 2^-800 ..
 // 2^800 and not zero (or not finite); the caller then evaluates the cell in
-// the reference's own operand order.
+// the reference's own operand order.  rho and 1 / tau stay within 2^+-100, psi, g
+// and u within 2^+-400, so that their squares stay within 2^+-800: away from the
+// interface u and g are products of rounding errors, 1e-36 and below, and with
+// 2^+-100 for them too a fifth of such cells were evaluated twice (a channel of
+// 194 x 2372 ahead of the front: 311 -> 242 us per iteration over the first twenty).
 #pragma once
 
 #include <cmath>
@@ -69,7 +73,7 @@ FD_CELL double cell_rcp(double b) {
 #endif
 }
 
-// true if v is zero or its magnitude lies in 2^-E .. 2^E (E = 800 or 100)
+// true if v is zero or its magnitude lies in 2^-E .. 2^E
 template <int E>
 FD_CELL bool cell_in_range(double v) {
   uint64_t b;
@@ -214,7 +218,7 @@ struct CellPair {
 };
 FD_CELL_CALL CellPair cell_relax(double w, double A, double B, double rho, double psi, double q, double SF, double P,
                                  double S, double inv_t, double tau_inv, double f, double g) {
-  bool ok = cell_in_range<100>(g);
+  bool ok = cell_in_range<400>(g);
   const double fe = cell_mul<0>(w, A + cell_mul<1>(rho, q, ok), ok);
   const double ge = cell_mul<2>(w, B + cell_mul<3>(psi, q, ok), ok);
   const double fn = cell_fma(SF, cell_mul<4>(P, S, ok), f - cell_mul<5>(inv_t, f - fe, ok));
@@ -233,7 +237,7 @@ FD_CELL ExactMacro exact_macros(const ExactConst& k, double rho, double psi, con
   ExactMacro m;
   const double mx = ((((f[1] - f[3]) + f[5]) - f[6]) - f[7]) + f[8];
   const double my = ((((f[2] - f[4]) + f[5]) + f[6]) - f[7]) - f[8];
-  bool ok = st.ok & cell_in_range<100>(rho) & (rho != 0.0) & cell_in_range<100>(psi);
+  bool ok = st.ok & cell_in_range<100>(rho) & (rho != 0.0) & cell_in_range<400>(psi);
   const double mu = cell_mul<7>(k.a * psi, 1.0 - cell_mul<8>(psi, psi, ok), ok) - cell_mul<9>(k.kappa, st.lap, ok);
   const double mgx = cell_mul<10>(mu, st.gx, ok), mgy = cell_mul<11>(mu, st.gy, ok);
   const double jx = cell_fma(0.5, mgx, mx), jy = cell_fma(0.5, mgy, my);
@@ -267,8 +271,8 @@ FD_CELL bool exact_collide(const ExactConst& k, const ExactMacro& m, const doubl
   const double inv_t = cell_rcp(m.tau);
   const double pref = cell_fma(-0.5, inv_t, 1.0);  // 1 - 1 / (2 tau)
   const double na = rho - cell_mul<17>(k.c_a0, p, ok), nb = psi - cell_mul<18>(k.c_b0, mu, ok);
-  ok = ok & cell_in_range<800>(mu) & cell_in_range<800>(na) & cell_in_range<800>(nb) & cell_in_range<100>(ux) &
-       cell_in_range<100>(uy) & cell_in_range<100>(inv_t);
+  ok = ok & cell_in_range<800>(mu) & cell_in_range<800>(na) & cell_in_range<800>(nb) & cell_in_range<400>(ux) &
+       cell_in_range<400>(uy) & cell_in_range<100>(inv_t);
   const double A0 = cell_div_const(na, k.w0, k.yw0), A = cell_scale<40, 3, 0>(p);
   const double B0 = cell_div_const(nb, k.w0, k.yw0), B = cell_mul<19>(k.c_b18, mu, ok);
   // forcing prefactor of w_1; 4 P and P / 4 are those of w_0 and w_5

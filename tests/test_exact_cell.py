@@ -80,6 +80,27 @@ def test_cell_equals_the_reference_order(cells, spread, eta):
     assert np.array_equal(g, st.g.reshape(9, -1))
 
 
+def test_rounding_noise_is_in_range(cells):
+    """Far from the interface u and g are products of rounding errors (1e-36 and
+    below): such cells are taken, with the same bits."""
+    H, W = 8, 160
+    prm = OracleParams(H=H, W=W, variant="periodic", tau=0.789, eta_n=1 / 30, M=4.0, a=-0.0125, kappa=0.0125, gamma=7.0,
+                       psi_wall=-0.5, inlet_ux=np.full(H, 0.003), outlet_coef=2 / 3)
+    st = OracleState(prm, np.zeros((H, W), bool), np.where(np.arange(W) < 20, 1.0, -1.0) * np.ones((H, 1)))
+    small = 0
+    for _ in range(40):
+        st.step()
+        f, g = (np.ascontiguousarray(v.reshape(9, -1)).copy() for v in (st.f, st.g))
+        small += int(((st.g != 0) & (abs(st.g) < 2.0 ** -100)).sum() + ((st.uy != 0) & (abs(st.uy) < 2.0 ** -100)).sum())
+        assert run(cells, st, f, g).all()
+        want = OracleState(prm, st.solid, st.psi.copy())
+        want.f, want.g = st.f.copy(), st.g.copy()
+        want.macros()
+        want.collide()
+        assert np.array_equal(f, want.f.reshape(9, -1)) and np.array_equal(g, want.g.reshape(9, -1))
+    assert small > 0
+
+
 def test_values_out_of_range_are_refused_untouched(cells):
     st = oracle_state(8, 64, 5, 1e-3)
     f, g = (np.ascontiguousarray(v.reshape(9, -1)).copy() for v in (st.f, st.g))
