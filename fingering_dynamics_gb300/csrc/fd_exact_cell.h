@@ -25,7 +25,7 @@
 // the reference's own operand order.  rho and 1 / tau stay within 2^+-100, psi, g
 // and u within 2^+-400, so that their squares stay within 2^+-800: away from the
 // interface u and g are products of rounding errors, 1e-36 and below, and with
-// 2^+-100 for them too a fifth of such cells were evaluated twice (a channel of
+// 2^+-100 for them too whole columns there were evaluated twice (a channel of
 // 194 x 2372 ahead of the front: 311 -> 242 us per iteration over the first twenty).
 #pragma once
 

@@ -25,11 +25,12 @@
 // What it replaced: boxes of 8 channels (16-byte pieces, four to eight times as
 // many), the weights streamed anew for every tile, two descriptors built per MMA
 // by the thread that also issued the boxes.  Measured at batch 32, us, before ->
-// here: 16 -> 32 (256 x 512, GELU) 271 -> 169, 32 -> 32 354 -> 191, 96 -> 32 855 ->
-// 340, 32 -> 96 (no activation) 924 -> 302, 64 -> 64 (128 x 256) 250 -> 126, 192 ->
-// 64 507 -> 204, 128 -> 128 (64 x 128) 207 -> 83, 384 -> 128 397 -> 160 (1448
-// TFLOP/s).  The thin layers with GELU are bound by the epilogue's tanhf and the
-// writes of z and y (537 MB, 79 us), the wide ones by the tensor pipe.
+// here: 16 -> 32 (256 x 512, GELU) 271 -> 167, 32 -> 32 354 -> 181, 96 -> 32 855 ->
+// 338, 32 -> 96 (no activation) 924 -> 208, 64 -> 64 (128 x 256) 250 -> 96, 192 -> 64
+// 507 -> 200, 128 -> 128 (64 x 128) 207 -> 68, 384 -> 128 397 -> 151 (1538 TFLOP/s).
+// The thin layers are bound by the MMAs, which take some 55 clocks however few
+// columns they have (32 -> 16: 114 us, its bytes 59), with GELU also by the
+// epilogue's tanhf; the wide ones by the tensor pipe.
 #include "sg_tc.cuh"
 
 namespace sg {
@@ -38,9 +39,26 @@ namespace {
 constexpr int kCvEpiWarps = 8;
 constexpr int kCvThreads = 32 * (kCvEpiWarps + 2);
 
+// 32 bytes of one pixel: one store of a whole sector where the tensors are 32-byte
+// aligned (`wide`), else two.  Two stores of half a sector each bound the layers
+// that write much: at batch 32, us, two -> one: 64 -> 64 (128 x 256, GELU) 127 -> 96,
+// 32 -> 64 113 -> 87, 32 -> 96 (256 x 512) 300 -> 208, 128 -> 128 (64 x 128) 84 -> 68.
+// (12 or 16 epilogue warps instead of 8 then gain 3-8% on the two thinnest layers and
+// lose 2-4% on the others.)
+__device__ __forceinline__ void cv_store32(bf16* p, const uint32_t (&w)[8], bool wide) {
+  if (wide) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+                 "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+  } else {
+    reinterpret_cast<uint4*>(p)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    reinterpret_cast<uint4*>(p)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+  }
+}
+
 // Bias, activation and stores of 16 output channels of one pixel (element offset o).
-__device__ __forceinline__ void cv_store16(const float (&v)[16], const float* sbias, int act, bf16* __restrict__ z,
-                                           bf16* __restrict__ y, size_t o) {
+__device__ __forceinline__ void cv_store16(const float (&v)[16], const float* sbias, int act, bool wide,
+                                           bf16* __restrict__ z, bf16* __restrict__ y, size_t o) {
   uint32_t zw[8], yw[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
@@ -54,14 +72,8 @@ __device__ __forceinline__ void cv_store16(const float (&v)[16], const float* sb
     const __nv_bfloat162 yp = __floats2bfloat162_rn(t0, t1);
     yw[k] = *reinterpret_cast<const uint32_t*>(&yp);
   }
-  if (z) {
-    reinterpret_cast<uint4*>(z + o)[0] = make_uint4(zw[0], zw[1], zw[2], zw[3]);
-    reinterpret_cast<uint4*>(z + o)[1] = make_uint4(zw[4], zw[5], zw[6], zw[7]);
-  }
-  if (y) {
-    reinterpret_cast<uint4*>(y + o)[0] = make_uint4(yw[0], yw[1], yw[2], yw[3]);
-    reinterpret_cast<uint4*>(y + o)[1] = make_uint4(yw[4], yw[5], yw[6], yw[7]);
-  }
+  if (z) cv_store32(z + o, zw, wide);
+  if (y) cv_store32(y + o, yw, wide);
 }
 
 // FLAT: the tile of k_conv3x3_rows at widths that are not a multiple of 128 and few
@@ -236,6 +248,7 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_rows(const __grid_con
     // epilogue: warp w reads TMEM lanes 32 q .. 32 q + 31 (pixels x0 + 32 q + lane of each row, q = w % 4) of every
     // second group of 16 columns (w / 4)
     const int q = warp & 3, h = warp >> 2;
+    const bool wide = ((uintptr_t)z | (uintptr_t)y) % 32 == 0;
     const int m = q * 32 + lane, my = FLAT ? m / pitch : 0, mx = m - my * pitch;
     for (int j = 0; j < mine; ++j) {
       const int b = j & 1;
@@ -250,7 +263,7 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_rows(const __grid_con
         float v[16];
         tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * R * BN + i * 16), v);
         const size_t o = (((size_t)n * sh.H + yy + r + my) * sh.W + x0 + mx) * sh.Cout + co0 + c0;
-        if (in) cv_store16(v, sbias + c0, sh.act, z, y, o);
+        if (in) cv_store16(v, sbias + c0, sh.act, wide, z, y, o);
       }
       // this warp's reads of buffer b are complete (tcgen05.wait::ld in tmem_ld16)
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -390,6 +403,7 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_narrow(const __grid_c
       mbar_wait_ok(&empty[i], (unsigned)((c - 1 - ((c - 1 - i) % S)) / S) & 1u, false);
   } else {
     const int q = warp & 3, h = warp >> 2;
+    const bool wide = ((uintptr_t)z | (uintptr_t)y) % 32 == 0;
     const int m = q * 32 + lane, my = m / bw, mx = m - my * bw;  // pixel of the tile
     for (int j = 0; j < mine; ++j) {
       const int b = j & 1;
@@ -404,7 +418,7 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_narrow(const __grid_c
         float v[16];
         tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + i * 16), v);
         if (in)
-          cv_store16(v, sbias + i * 16, sh.act, z, y, (((size_t)n * sh.H + yy) * sh.W + xx) * sh.Cout + co0 + i * 16);
+          cv_store16(v, sbias + i * 16, sh.act, wide, z, y, (((size_t)n * sh.H + yy) * sh.W + xx) * sh.Cout + co0 + i * 16);
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();

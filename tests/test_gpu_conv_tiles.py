@@ -61,3 +61,23 @@ def test_narrow_convolution_is_exact(n, h, w, cin, cout, act):
                                                 (4, 40, 328, 32, 32, 1), (1, 3, 1000, 96, 160, 0)])
 def test_any_width_convolution_is_exact(n, h, w, cin, cout, act):
     _check("sg_conv3x3_tc", n, h, w, cin, cout, act)
+
+
+@pytest.mark.parametrize("fn,w", [("sg_conv3x3_tma", 128), ("sg_conv3x3_tc", 40)])
+def test_outputs_that_are_16_byte_aligned_only(fn, w):
+    """z and y at 16 bytes from a 32-byte boundary take two stores per sector."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from fingering_dynamics_gb300 import _lib as L
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn((1, 4, w, 32), generator=g, device="cuda").to(torch.bfloat16)
+    wt = torch.randn((48, 3, 3, 32), generator=g, device="cuda").to(torch.bfloat16)
+    b = torch.randn(48, generator=g, device="cuda")
+    p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    out = []
+    for off in (0, 8):
+        z, y = (torch.zeros(4 * w * 48 + 16, dtype=torch.bfloat16, device="cuda")[off:off + 4 * w * 48] for _ in range(2))
+        L.call(fn, p(x), 1, 4, w, 32, p(wt), p(b), 48, 1, p(z), p(y), None)
+        out.append((z, y))
+    torch.cuda.synchronize()
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
