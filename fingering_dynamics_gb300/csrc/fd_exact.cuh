@@ -22,10 +22,9 @@
 // thread per pair of cells in the reference's operand order (solid lanes idle,
 // twelve divisions, the products by 0 and 1 evaluated); 1.05 ms with full warps
 // and the rewritings of fd_exact_cell.h (369 FP64 instructions per 32 fluid
-// cells, the pipe 84% busy, one issue slot in ten used); 0.87 ms with the
-// products in integer arithmetic (250 FP64 instructions).  Five CTAs an SM (96
-// registers, some spilled) beat four by 6% on 400 x 400: warps in flight hide
-// the pipe's latency.
+// cells, the pipe 84% busy, one issue slot in ten used); 0.89 ms with the
+// products in integer arithmetic (250 FP64 instructions), 0.82 with those in
+// calls and a thread per cell of a tile of 8 rows.
 //
 // Cells whose values leave the range that exact_cell() takes (a diverging run),
 // and the body-force variant, are evaluated in the reference's operand order by
@@ -38,9 +37,10 @@
 namespace fd {
 
 constexpr int kExactTX = 32;
-#ifndef FD_EXACT_MINB
-#define FD_EXACT_MINB 5
-#endif
+// CTAs per SM that the registers are cut for: 96 registers at 128 threads (tiles of
+// 4 rows), 80 at 256 (8 rows; 128 threads x 5 845 us per iteration of 1024 x 2048,
+// 128 x 4 831, 192 x 4 852, 256 x 2 903, 256 x 3 819)
+constexpr int exact_min_ctas(int nt) { return nt == 128 ? 5 : 3; }
 
 struct ExactArgs {
   FusedArgs<double> a;
@@ -108,7 +108,7 @@ __device__ __noinline__ void exact_slow_cell(const FusedArgs<double>& a, int x, 
 }
 
 template <int TY, int NT>
-__global__ void __launch_bounds__(NT, FD_EXACT_MINB) k_exact_step(const __grid_constant__ ExactArgs ea) {
+__global__ void __launch_bounds__(NT, exact_min_ctas(NT)) k_exact_step(const __grid_constant__ ExactArgs ea) {
   constexpr int CW = 32 / TY, CHUNKS = kExactTX / CW, PW = kExactTX + 2;
   static_assert(TY * CW == 32 && CHUNKS * CW == kExactTX, "a group of 32 cells is CW columns of the tile");
   __shared__ double psi[(TY + 2) * PW];
@@ -230,13 +230,10 @@ __global__ void __launch_bounds__(NT, FD_EXACT_MINB) k_exact_step(const __grid_c
   }
 }
 
-#ifndef FD_EXACT_NT
-#define FD_EXACT_NT 128
-#endif
-
 template <int TY>
 int launch_exact(ExactArgs& ea, const fd_params& p, double* pa, double* pb, double* sa, double* sb, int nsteps,
                  cudaStream_t st) {
+  constexpr int NT = 32 * TY;  // one cell a thread
   ea.ntx = (p.W + kExactTX - 1) / kExactTX;
   const unsigned blocks = (unsigned)ea.ntx * (unsigned)((p.H + TY - 1) / TY);
   for (int s = 0; s < nsteps; ++s) {
@@ -245,7 +242,7 @@ int launch_exact(ExactArgs& ea, const fd_params& p, double* pa, double* pb, doub
     ea.a.dst = even ? pb : pa;
     ea.a.side_in = even ? sa : sb;
     ea.a.side_out = even ? sb : sa;
-    k_exact_step<TY, FD_EXACT_NT><<<blocks, FD_EXACT_NT, 0, st>>>(ea);
+    k_exact_step<TY, NT><<<blocks, NT, 0, st>>>(ea);
   }
   return cudaGetLastError() == cudaSuccess ? FD_OK : FD_ERR_CUDA;
 }

@@ -18,12 +18,12 @@ int fused_f64(const fd_params& p, const uint16_t* mask, const double* inlet_ux, 
   const Coef<double>& c = ea.a.c;
   ea.k = make_exact_const(c.w[0], c.w[1], c.a, c.kappa, c.eta_n, c.eta_n_M, c.c_a0, c.c_b0, c.c_b18, c.one_third,
                           c.tau_inv);
-  // Tiles of 8 rows on large lattices (fewer psi cells around the tiles), of 4
-  // where 8-row tiles would not give every SM about eight CTAs (four are
-  // resident): 1024 x 2048 11.56 vs 11.92 ms for ten iterations, 400 x 400
-  // (650 tiles of 8 rows) 3.52 vs 3.16 ms for 25.
+  // Tiles of 8 rows, one cell a thread, where they give every SM five CTAs or more
+  // (three are resident); below, tiles of 4 rows.  us per iteration, 8 / 4 rows:
+  // 400 x 400 (650 tiles of 8 rows) 105 / 97, 1764 x 128 (884) 139 / 150, 512 x 512
+  // 140 / 139, 512 x 1024 242 / 253, 1024 x 2048 819 / 895.
   const long long tiles = (long long)((p.W + kExactTX - 1) / kExactTX) * ((p.H + 7) / 8);
-  if (tiles < 8 * 152) return launch_exact<4>(ea, p, (double*)pa, (double*)pb, (double*)sa, (double*)sb, nsteps, st);
+  if (tiles < 5 * 152) return launch_exact<4>(ea, p, (double*)pa, (double*)pb, (double*)sa, (double*)sb, nsteps, st);
   return launch_exact<8>(ea, p, (double*)pa, (double*)pb, (double*)sa, (double*)sb, nsteps, st);
 }
 }  // namespace fd
