@@ -1,11 +1,11 @@
 """Learned surrogate: a convolutional U-Net that advances (psi, u_x, u_y) by a
 fixed number of lattice steps (a "jump") given the solid mask, trained on
 trajectories of the batched LBM with this package's own CUDA kernels
-(include/fdsurrogate.h: tensor-core implicit-GEMM convolutions, forward and
-data gradient on tcgen05 with the accumulator in tensor memory or on
-warp-level MMA, whichever is faster for the shape, weight gradient on
-warp-level MMA, and the training elementwise kernels), and a rollout
-driver that uses the plain LBM as its judge and fallback.
+(include/fdsurrogate.h: tensor-core implicit-GEMM convolutions, forward,
+data gradient and weight gradient on tcgen05 with the accumulator in tensor
+memory or on warp-level MMA, whichever is faster for the shape, and the
+training elementwise kernels), and a rollout driver that uses the plain LBM as
+its judge and fallback.
 
 The reference has no learned component.  Network (widths c1..c4, 3x3 convs,
 GELU, 2x2 mean pooling, nearest upsampling, skip concatenation):
