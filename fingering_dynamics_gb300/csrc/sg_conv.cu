@@ -525,7 +525,8 @@ int rows_n(const CvCall& c) {
 // fewest tiles.
 inline void tile_box(int H, int W, int gap, int& bw, int& rows) {
   long long best = 0;
-  for (int k = (W + kTcBM - 1) / kTcBM; k <= 16 && k <= W; ++k) {
+  const int least = (W + kTcBM - 1) / kTcBM;
+  for (int k = least; k <= std::max(least, 16) && k <= W; ++k) {
     const int w = (W + k - 1) / k, r = std::min((kTcBM + gap) / (w + gap), 254);
     const long long tiles = (long long)((W + w - 1) / w) * ((H + r - 1) / r);
     if (best == 0 || tiles < best) {

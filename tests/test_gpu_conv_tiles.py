@@ -58,7 +58,8 @@ def test_narrow_convolution_is_exact(n, h, w, cin, cout, act):
                                                 (3, 7, 25, 96, 32, 1), (1, 50, 41, 64, 128, 1), (2, 21, 62, 48, 32, 1),
                                                 (1, 9, 63, 32, 64, 0), (2, 5, 100, 96, 64, 1), (1, 6, 126, 32, 32, 1),
                                                 (1, 6, 127, 128, 32, 0), (2, 4, 129, 16, 32, 1), (1, 11, 130, 64, 16, 1),
-                                                (4, 40, 328, 32, 32, 1), (1, 3, 1000, 96, 160, 0)])
+                                                (4, 40, 328, 32, 32, 1), (1, 3, 1000, 96, 160, 0),
+                                                (1, 2, 2100, 32, 16, 1), (1, 3, 2184, 64, 32, 0)])
 def test_any_width_convolution_is_exact(n, h, w, cin, cout, act):
     _check("sg_conv3x3_tc", n, h, w, cin, cout, act)
 
