@@ -145,6 +145,7 @@ SIGNATURES = {
     "sg_masked_mse_scaled": [_VP, _VP, _VP, _SZ, _I, _VP, _VP, _VP, _VP],
     "sg_add_prediction": [_VP, _VP, _SZ, _I, _VP, _VP],
     "sg_run": [_VP, _I, _VP],
+    "sg_frame": [_VP, _VP, _VP, _VP, _SZ, _I, _FL, _VP, _VP],
     "sg_to_bf16": [_VP, _SZ, _VP, _VP],
 }
 _RET = {"fd_last_error": C.c_char_p, "fd_packed_bytes": C.c_size_t, "fd_diag_scratch_bytes": C.c_size_t,

@@ -775,6 +775,22 @@ __global__ void k_masked_mse(const bf16* __restrict__ x, const bf16* __restrict_
 }
 
 // y = x with its first three channels replaced by bf16(x + out)
+// A frame of the network (16 channels: psi, u_x / U, u_y / U, solid, zeros) from
+// the fields, one cell a thread, one 32-byte store; as tensor operations it was ten
+// passes of a few microseconds each.
+template <typename T>
+__global__ void k_frame(const T* __restrict__ psi, const T* __restrict__ ux, const T* __restrict__ uy,
+                        const unsigned char* __restrict__ solid, size_t n, float inv_u, bf16* __restrict__ out) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const bool s = solid[i] != 0;
+  const __nv_bfloat162 a = __floats2bfloat162_rn((float)psi[i], (s ? 0.0f : (float)ux[i]) * inv_u);
+  const __nv_bfloat162 b = __floats2bfloat162_rn((s ? 0.0f : (float)uy[i]) * inv_u, s ? 1.0f : 0.0f);
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %3, %3, %3, %3, %3};" ::"l"(out + 16 * i),
+               "r"(*reinterpret_cast<const uint32_t*>(&a)), "r"(*reinterpret_cast<const uint32_t*>(&b)), "r"(0u)
+               : "memory");
+}
+
 __global__ void k_add_prediction(const bf16* __restrict__ x, const bf16* __restrict__ out, size_t P, int C,
                                  bf16* __restrict__ y) {
   const int cg = C / 8;
@@ -1076,6 +1092,20 @@ int sg_add_prediction(const void* x, const void* out, size_t P, int C, void* y, 
   fd::launch_pdl(k_add_prediction, ew_blocks(P * (C / 8)), kEw, 0, as_stream(stream), t_op_follows, (const bf16*)x,
                  (const bf16*)out, P, C, (bf16*)y);
   return check_launch("sg_add_prediction");
+}
+
+int sg_frame(const void* psi, const void* ux, const void* uy, const void* solid, size_t n, int f64, float inv_u,
+             void* out, void* stream) {
+  FD_REQUIRE(psi && ux && uy && solid && out && (uintptr_t)out % 32 == 0, FD_ERR_ARG, "sg_frame: bad arguments");
+  if (n == 0) return FD_OK;
+  cudaStream_t s = as_stream(stream);
+  if (f64)
+    k_frame<double><<<ew_blocks(n), kEw, 0, s>>>((const double*)psi, (const double*)ux, (const double*)uy,
+                                                 (const unsigned char*)solid, n, inv_u, (bf16*)out);
+  else
+    k_frame<float><<<ew_blocks(n), kEw, 0, s>>>((const float*)psi, (const float*)ux, (const float*)uy,
+                                                (const unsigned char*)solid, n, inv_u, (bf16*)out);
+  return check_launch("sg_frame");
 }
 
 int sg_to_bf16(const float* src, size_t n, void* dst, void* stream) {

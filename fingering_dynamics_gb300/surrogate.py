@@ -60,6 +60,15 @@ def _s():
 def frame_from_fields(psi, ux, uy, solid) -> torch.Tensor:
     """(H, W) device tensors -> one frame (H, W, 16) bfloat16."""
     H, W = psi.shape
+    if (psi.is_cuda and psi.device.index == torch.cuda.current_device() and solid.dtype == torch.bool
+            and psi.dtype in (torch.float32, torch.float64)
+            and all(type(t) is torch.Tensor and t.dtype == psi.dtype and not t.requires_grad for t in (psi, ux, uy))
+            and all(t.shape == psi.shape and t.device == psi.device and t.is_contiguous() for t in (psi, ux, uy, solid))):
+        out = torch.empty((H, W, FRAME_CHANNELS), dtype=torch.bfloat16, device=psi.device)
+        # the reciprocal that the division of a tensor by a number multiplies with
+        L.call("sg_frame", _p(psi), _p(ux), _p(uy), _p(solid), H * W, int(psi.dtype == torch.float64),
+               float(np.float32(1) / np.float32(VELOCITY_SCALE)), _p(out), _s())
+        return out
     fr = torch.zeros((H, W, FRAME_CHANNELS), dtype=torch.float32, device=psi.device)
     fl = ~solid
     fr[..., 0] = psi.float()

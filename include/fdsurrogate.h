@@ -171,6 +171,12 @@ typedef struct sg_op {
 } sg_op;
 int sg_run(const sg_op* ops, int count, void* stream);
 
+/* The network's frame of n cells: 16 bfloat16 channels psi, u_x inv_u, u_y inv_u
+ * (0 on solid cells), solid, zeros, from FP32 (f64 = 0) or FP64 fields and a byte
+ * per cell.  out: 32-byte aligned. */
+int sg_frame(const void* psi, const void* ux, const void* uy, const void* solid, size_t n, int f64, float inv_u,
+             void* out, void* stream);
+
 /* FP32 -> bfloat16 (round to nearest even), n elements. */
 int sg_to_bf16(const float* src, size_t n, void* dst, void* stream);
 

@@ -132,3 +132,20 @@ def test_a_list_equals_its_operations(n, h, w):
     net._run_words = lambda words: [run(words[k:k + 16]) for k in range(0, len(words), 16)]
     for x, y in zip(xs, listed):
         assert torch.equal(net.predict(x), y)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("h,w", [(1, 1), (3, 40), (33, 257)])
+def test_frame_equals_the_tensor_operations(dtype, h, w):
+    """sg_frame against the tensor operations (which strided fields still take), with infinities and NaN."""
+    from fingering_dynamics_gb300.surrogate import frame_from_fields
+    g = torch.Generator(device="cuda").manual_seed(h)
+    psi, ux, uy = (torch.randn((h, 2 * w), generator=g, device="cuda", dtype=getattr(torch, dtype)) * s
+                   for s in (1.0, 3e-2, 1e-9))
+    if h > 1:
+        ux[0, 0], uy[1, 2], psi[2, 4], ux[1, 0] = float("inf"), float("-inf"), float("nan"), 1e-40
+    solid = torch.rand((h, 2 * w), generator=g, device="cuda") < 0.3
+    want = frame_from_fields(psi[:, ::2], ux[:, ::2], uy[:, ::2], solid[:, ::2])
+    got = frame_from_fields(*(t[:, ::2].contiguous() for t in (psi, ux, uy, solid)))
+    assert got.shape == want.shape and torch.equal(torch.isnan(got), torch.isnan(want))
+    assert torch.equal(torch.nan_to_num(got).view(torch.int16), torch.nan_to_num(want).view(torch.int16))
