@@ -100,15 +100,15 @@ class UNet:
         memory), "tma" (the same as a persistent kernel fed by tensor-map
         boxes; images whose width is a multiple of 128, the others fall back to
         "tcgen05"), "tma_ws" (the same kernel),
-        "mma" (warp-level tensor-core instructions) or "auto" (all
-        that take the shape timed once per convolution shape at first use, the
-        fastest kept).  The weight gradient runs on the tcgen05 kernel at widths
-        that are multiples of 128 for every choice but "mma" ("auto": the faster
-        of the two per shape), else on the warp-level kernel."""
+        "mma" (warp-level tensor-core instructions) or "auto" ("tma", by the rule
+        of _run_conv, so that a network's outputs do not depend on a
+        measurement).  The weight gradient runs on the tcgen05 kernel at widths
+        that are multiples of 128 for every choice but "mma", else on the
+        warp-level kernel."""
         if conv not in ("tcgen05", "tma", "tma_ws", "mma", "auto"):
             raise ValueError("conv must be 'tcgen05', 'tma', 'tma_ws', 'mma' or 'auto'")
         self.conv = conv
-        self.conv_choice = {}  # (N, H, W, Cin, Cout) -> kernel name, filled by "auto"
+        self.conv_choice = {}  # (N, H, W, Cin, Cout) -> kernel name, filled by "auto" where it is not set already
         self.widths = tuple(widths)
         self.shapes = layer_shapes(self.widths)
         self.device = torch.device(device)
@@ -196,7 +196,6 @@ class UNet:
 
     _KERNELS = {"mma": "sg_conv3x3", "tcgen05": "sg_conv3x3_tc", "tma": "sg_conv3x3_tma",
                 "tma_ws": "sg_conv3x3_tma_ws"}
-    _TIMED = ("mma", "tcgen05", "tma")  # "auto" times these ("tma_ws" names the kernel of "tma")
     # operations of a pass (include/fdsurrogate.h sg_op_kind)
     _OP = {"sg_conv3x3": 0, "sg_conv3x3_tc": 1, "sg_conv3x3_tma": 2, "sg_conv3x3_tma_ws": 2, "sg_conv3x3_wgrad": 3,
            "sg_conv3x3_wgrad_tc": 4, "sg_pool2": 5, "sg_up2_concat": 6, "sg_gelu_bias_bwd": 7, "sg_bias_grad": 8,
@@ -232,52 +231,34 @@ class UNet:
         multiples of 128, channel counts that are multiples of 16)."""
         return not kernel.startswith("tma") or (w % 128 == 0 and ci % 16 == 0 and co % 16 == 0)
 
-    def _fastest(self, key, fns, ints, tensors):
-        """The fastest of the kernels, timed once per shape on the real operands
-        (after the pass's pending operations) in a list, as a pass runs them:
-        calls of their own are bound by Python on a batch of one.  Kept in
-        conv_choice."""
-        if key not in self.conv_choice:
-            self._run_ops()
-            best = None
-            for fn in fns:
-                words = self._words(fn, ints, tensors)
-                self._run_words(words)
-                e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-                e0.record()
-                self._run_words(words * 4)
-                e1.record()
-                e1.synchronize()
-                t = e0.elapsed_time(e1)
-                if best is None or t < best[0]:
-                    best = (t, fn)
-            self.conv_choice[key] = best[1]
-        return self.conv_choice[key]
-
+    # Rule of "auto": sg_conv3x3_tma at widths that are multiples of 128, sg_conv3x3_tc at
+    # the others.  A stopwatch chose before, and as the kernels add the taps in different
+    # orders two runs of one program could differ in the last bits.  The rule's kernel was
+    # the fastest on each of the network's layers at ten batch shapes (1 x 64 x 64 to 32 x
+    # 256 x 512) and on 150 random shapes; the closest, us, rule / next: 1 x 64 x 128, 16 ->
+    # 32 4.7 / 6.8, 2 x 34 x 66, 64 -> 128 6.5 / 10.9; one image of 256 x 512: 32 -> 32 11.1 /
+    # 24.4, 384 -> 128 17.5 / 41.7; 32 of them: 32 -> 32 177 / 580, 384 -> 128 150 / 539.
     def _run_conv(self, x, N, h, w, ci, wt, bias, co, act, z, y):
         """One 3x3 convolution with the kernel chosen for its shape."""
-        if self.conv != "auto":
-            fn = self._KERNELS[self.conv if self._takes(self.conv, w, ci, co) else "tcgen05"]
-        else:
-            fns = [self._KERNELS[k] for k in self._TIMED if self._takes(k, w, ci, co)]
-            fn = self._fastest((N, h, w, ci, co), fns, (N, h, w, ci, co, act), (x, wt, bias, z, y))
+        kernel = "tma" if self.conv == "auto" else self.conv
+        fn = self._KERNELS[kernel if self._takes(kernel, w, ci, co) else "tcgen05"]
+        if self.conv == "auto":
+            fn = self.conv_choice.setdefault((N, h, w, ci, co), fn)
         self._op(fn, (N, h, w, ci, co, act), (x, wt, bias, z, y))
 
     _WGRAD = {"mma": "sg_conv3x3_wgrad", "tcgen05": "sg_conv3x3_wgrad_tc"}
 
+    # At widths that both take, sg_conv3x3_wgrad_tc was within 2% of the faster on 98 of 100 random
+    # shapes and on all layers but two of a batch of one (64 chunks of 128 pixels): us, it /
+    # warp-level, 64 -> 128 22.6 / 21.5, 128 -> 128 27.7 / 25.6, 384 -> 128 33.7 / 46.4; 32
+    # images of 256 x 512: 32 -> 32 131 / 672, 384 -> 128 146 / 985.
     def _run_wgrad(self, inp, dz, N, h, w, ci, co, gw, part):
         """Weight gradient of one layer: the tcgen05 kernel (widths that are
-        multiples of 128) or the warp-level one; with conv="auto" both are timed
-        once per shape and the faster kept (their FP32 sums differ in the last
-        bits only)."""
-        ok_tc = w % 128 == 0
-        if self.conv == "mma" or not ok_tc:
-            fn = self._WGRAD["mma"]
-        elif self.conv != "auto":
-            fn = self._WGRAD["tcgen05"]
-        else:
-            fn = self._fastest(("wgrad", N, h, w, ci, co), list(self._WGRAD.values()),
-                               (N, h, w, ci, co, part.numel()), (inp, dz, gw, part))
+        multiples of 128) or the warp-level one (their FP32 sums differ in the
+        last bits only)."""
+        fn = self._WGRAD["mma" if self.conv == "mma" or w % 128 != 0 else "tcgen05"]
+        if self.conv == "auto" and w % 128 == 0:
+            fn = self.conv_choice.setdefault(("wgrad", N, h, w, ci, co), fn)
         self._op(fn, (N, h, w, ci, co, part.numel()), (inp, dz, gw, part))
 
     def _conv(self, name, x, B, act=True, keep=True):

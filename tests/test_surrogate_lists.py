@@ -1,0 +1,50 @@
+"""The lists of operations that a network's passes queue, with the launch itself
+replaced (no GPU is needed)."""
+import pytest
+
+torch = pytest.importorskip("torch")
+
+FLIP, WORDS = 9, 16
+
+
+@pytest.fixture
+def net(monkeypatch):
+    from fingering_dynamics_gb300 import build
+    from fingering_dynamics_gb300 import surrogate as sg
+    build.build()
+    net = sg.UNet((16, 16, 32, 32), seed=1, device="cpu")
+    net.ran = []
+    net._run_words = lambda words: net.ran.append([words[k] for k in range(0, len(words), WORDS)])
+    monkeypatch.setattr(torch.cuda, "Event", _no_stopwatch)
+    return net
+
+
+def _no_stopwatch(*a, **k):
+    raise AssertionError("a kernel was chosen by its time")
+
+
+def _frames(n, h, w):
+    return torch.zeros((n, h, w, 16), dtype=torch.bfloat16)
+
+
+@pytest.mark.parametrize("h,w", [(8, 128), (16, 1024), (64, 8), (8, 200)])
+def test_auto_chooses_by_shape(net, h, w):
+    """conv="auto": the kernel of every convolution follows from its shape alone."""
+    x = _frames(1, h, w)
+    net.forward(x)
+    net.backward(torch.zeros_like(x))
+    assert len(net.ran) == 2  # one list a pass
+    for key, fn in net.conv_choice.items():
+        wide = key[-3] % 128 == 0
+        if key[0] == "wgrad":
+            assert wide and fn == "sg_conv3x3_wgrad_tc"
+        else:
+            assert fn == ("sg_conv3x3_tma" if wide else "sg_conv3x3_tc")
+    assert len([k for k in net.conv_choice if k[0] != "wgrad"]) >= len(set(net.shapes.values()))
+
+
+def test_a_choice_that_the_caller_made_stands(net):
+    x = _frames(1, 8, 128)
+    net.conv_choice[(1, 8, 128, 16, 16)] = "sg_conv3x3"
+    net.predict(x)
+    assert net.ran[0][:2] == [0, 0]  # enc1a, enc1b
