@@ -136,8 +136,8 @@ class UNet:
         self.steps = 0
         self._buf = {}
         self._ops = []        # operations collected for the next sg_run
-        self._x, self._kept = None, False
-        self._flipped = False
+        self._x, self._kept = None, False  # the last pass's frames; whether its pre-activations are in the buffers
+        self._flipped = False  # whether wt16 holds the flipped w16
 
     @property
     def n_params(self) -> int:
@@ -277,7 +277,7 @@ class UNet:
         c1, c2, c3, c4 = self.widths
         lv = B["lv"]
         self._ops.clear()  # what a pass that raised left behind
-        self._x, self._kept = x, keep
+        self._x, self._kept = x, False
         e1 = self._conv("enc1b", self._conv("enc1a", x, B, keep=keep), B, keep=keep)
         self._op("sg_pool2", (N, H, W, c1), (e1, B["p1"]))
         e2 = self._conv("enc2b", self._conv("enc2a", B["p1"], B, keep=keep), B, keep=keep)
@@ -298,6 +298,7 @@ class UNet:
         prediction is x[..., :3] + out[..., :3])."""
         out = self._pass(x, True)
         self._run_ops()
+        self._kept = True
         return out
 
     def predict(self, x: torch.Tensor) -> torch.Tensor:
@@ -340,14 +341,15 @@ class UNet:
 
     def backward(self, dout: torch.Tensor):
         """Gradients (self.gw, self.gb) of the loss whose gradient w.r.t. the
-        output of the last forward() is dout."""
+        output of the last forward() is dout.  After a predict(), which stores no
+        pre-activations, the forward pass runs again here, on the frames that
+        predict() was given: they must still hold what they held."""
         self._ops.clear()
         if not self._kept:  # the last pass was predict()'s, which keeps no pre-activations
             self._pass(self._x, True)
         if not self._flipped:
             for name, (ci, co) in self.shapes.items():
                 self._op("sg_flip_weights", (ci, co), (self.w16[name], self.wt16[name]))
-            self._flipped = True
         x = self._x
         N, H, W, _ = x.shape
         B = self._buffers(N, H, W)
@@ -369,6 +371,7 @@ class UNet:
         de1 = self._block_back("enc1b", y("enc1a"), dp1, B, source=self._POOL, skip=du1, cy=c2 + c1, coff=c2)
         self._block_back("enc1a", x, de1, B, need_dx=False)
         self._run_ops()
+        self._kept = self._flipped = True  # only now: a list that was not run leaves neither behind
 
     def loss_grad(self, x: torch.Tensor, xn: torch.Tensor) -> torch.Tensor:
         """Forward, masked MSE of the prediction against xn, backward.
@@ -392,8 +395,8 @@ class UNet:
                                                        (self.b, None, self.gb, self.mb, self.vb, 0.0))):
                 items[2 * k + j] = L.sg_adamw_item(w[n].data_ptr(), None if w16 is None else w16[n].data_ptr(),
                                                    g[n].data_ptr(), m[n].data_ptr(), v[n].data_ptr(), w[n].numel(), wd)
-        L.call("sg_adamw_list", items, len(items), lr, beta1, beta2, eps, self.steps, _s())
         self._flipped = False
+        L.call("sg_adamw_list", items, len(items), lr, beta1, beta2, eps, self.steps, _s())
 
 
 # ----------------------------------------------------------------------------

@@ -48,3 +48,35 @@ def test_a_choice_that_the_caller_made_stands(net):
     net.conv_choice[(1, 8, 128, 16, 16)] = "sg_conv3x3"
     net.predict(x)
     assert net.ran[0][:2] == [0, 0]  # enc1a, enc1b
+
+
+def test_backward_after_one_that_raised_flips_the_weights(net):
+    x = _frames(1, 8, 128)
+    net.forward(x)
+    with pytest.raises(AttributeError):
+        net.backward(x.float().numpy())  # no tensor
+    net.forward(x)
+    net.backward(torch.zeros_like(x))
+    assert net.ran[-1].count(FLIP) == len(net.shapes)
+    net.backward(torch.zeros_like(x))
+    assert FLIP not in net.ran[-1]  # the weights have not changed
+
+
+@pytest.mark.parametrize("call", ["forward", "predict", "backward"])
+def test_a_list_that_was_not_run_leaves_nothing_behind(net, call):
+    """The launch of a pass fails once: the retry queues the flips and, if no pass
+    has stored the pre-activations, the forward pass."""
+    x, dout, run = _frames(1, 8, 128), _frames(1, 8, 128), net._run_words
+    net.forward(x)
+    forward = net.ran[-1]
+
+    def fails(words):
+        net._run_words = run
+        raise RuntimeError("launch")
+    net._run_words = fails
+    with pytest.raises(RuntimeError):
+        {"forward": net.forward, "predict": net.predict, "backward": net.backward}[call](x if call != "backward" else dout)
+    net.backward(dout)
+    kinds = net.ran[-1]
+    assert kinds.count(FLIP) == len(net.shapes)
+    assert (kinds[:len(forward)] == forward) == (call != "backward")
