@@ -256,13 +256,16 @@ class Lattice:
     def peek(self):
         """Fields of the next iteration (psi, rho, ux, uy, ... in the field
         tensors) without leaving fused mode: the pending packed state is
-        finished into a reference-layout buffer, which the fused state does
-        not use.  The state itself is not touched, so a
+        unpacked into ``f`` and ``g`` (its post-collision populations) and
+        finished into the other reference-layout buffer, neither of which the
+        fused state uses.  The state itself is not touched, so a
         lattice that is a member of an ensemble can be read between batched
         steps."""
         self._require("fused")
         if self.storage is None:
             raise ValueError("peek needs packed storage (dtype f32, f16 or bf16)")
+        L.call("fd_unpack", C.byref(self.prm), C.byref(self.storage), _ptr(self.ppop[self.pcur]), self.fd_dtype,
+               _ptr(self.pop[self.cur]), self._stream())
         self._finish_fused()
 
     def restart_from_fields(self, psi, ux, uy, rho=None, iteration: int | None = None,
