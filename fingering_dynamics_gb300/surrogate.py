@@ -57,12 +57,23 @@ def _s():
     return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
+def _plain(*tensors) -> bool:
+    """Whether the tensors' values are all there is to them, so that a kernel may
+    stand in for tensor operations: no gradient in either mode, no transform, no
+    subclass, and nothing that records the operations."""
+    if torch.compiler.is_compiling() or torch.jit.is_tracing() or torch._C._len_torch_dispatch_stack():
+        return False
+    return all(type(t) is torch.Tensor and not t.requires_grad
+               and not torch._C._functorch.is_functorch_wrapped_tensor(t)
+               and torch.autograd.forward_ad.unpack_dual(t).tangent is None for t in tensors)
+
+
 def frame_from_fields(psi, ux, uy, solid) -> torch.Tensor:
     """(H, W) device tensors -> one frame (H, W, 16) bfloat16."""
     H, W = psi.shape
     if (psi.is_cuda and psi.device.index == torch.cuda.current_device() and solid.dtype == torch.bool
-            and psi.dtype in (torch.float32, torch.float64)
-            and all(type(t) is torch.Tensor and t.dtype == psi.dtype and not t.requires_grad for t in (psi, ux, uy))
+            and psi.dtype in (torch.float32, torch.float64) and psi.numel() > 0 and _plain(psi, ux, uy, solid)
+            and all(t.dtype == psi.dtype for t in (psi, ux, uy))
             and all(t.shape == psi.shape and t.device == psi.device and t.is_contiguous() for t in (psi, ux, uy, solid))):
         out = torch.empty((H, W, FRAME_CHANNELS), dtype=torch.bfloat16, device=psi.device)
         # the reciprocal that the division of a tensor by a number multiplies with

@@ -80,3 +80,29 @@ def test_a_list_that_was_not_run_leaves_nothing_behind(net, call):
     kinds = net.ran[-1]
     assert kinds.count(FLIP) == len(net.shapes)
     assert (kinds[:len(forward)] == forward) == (call != "backward")
+
+
+def test_plain_tensors_only():
+    """What is not just its values keeps the tensor operations."""
+    import torch.autograd.forward_ad as fwd
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from fingering_dynamics_gb300.surrogate import _plain
+    x = torch.ones(3)
+    assert _plain(x, x > 0)
+    assert not _plain(x, torch.ones(3, requires_grad=True))
+    assert not _plain(torch.nn.Parameter(x, requires_grad=False))
+    seen = []
+    with fwd.dual_level():
+        seen.append(_plain(fwd.make_dual(x, x)))
+        assert _plain(x)
+
+    def look(t):
+        seen.append(_plain(t))
+        return t.sum()
+    torch.func.grad(look)(x)
+    torch.func.vmap(look)(x[None])
+    torch.jit.trace(look, x, check_trace=False)  # its check runs the function eagerly
+    with TorchDispatchMode():
+        seen.append(_plain(x))
+    assert len(seen) >= 5 and not any(seen)
+    assert _plain(x)
