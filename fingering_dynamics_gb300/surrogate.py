@@ -315,7 +315,7 @@ class UNet:
     def predict(self, x: torch.Tensor) -> torch.Tensor:
         """Frames one jump later: x[..., :3] + out[..., :3], other channels of x."""
         out = self._pass(x, False)
-        if x.is_contiguous() and x.dtype == torch.bfloat16 and x.shape[-1] == out.shape[-1]:
+        if x.is_contiguous() and x.dtype == torch.bfloat16 and x.shape[-1] == out.shape[-1] and _plain(x):
             y = torch.empty_like(x)
             self._op("sg_add_prediction", (x.numel() // x.shape[-1], x.shape[-1]), (x, out, y))
             self._run_ops()

@@ -1,4 +1,4 @@
-"""frame_from_fields on tensors that are more than their values, and on
+"""frame_from_fields and predict on tensors that are more than their values, and on
 empty fields: the tensor operations' results."""
 import pytest
 
@@ -32,3 +32,12 @@ def test_empty_fields_give_an_empty_frame(h, w):
     from fingering_dynamics_gb300.surrogate import frame_from_fields
     a = torch.zeros((h, w), device="cuda")
     assert frame_from_fields(a, a, a, a > 0).shape == (h, w, 16)
+
+
+def test_a_prediction_stays_attached_to_its_frames():
+    from fingering_dynamics_gb300.surrogate import UNet
+    net = UNet((16, 16, 32, 32), seed=1)
+    x = torch.randn((1, 8, 16, 16), device="cuda").to(torch.bfloat16)
+    y = net.predict(x)
+    z = net.predict(x.clone().requires_grad_())
+    assert z.requires_grad and not y.requires_grad and torch.equal(y, z.detach())
