@@ -19,6 +19,7 @@ FD_F64, FD_F32, FD_F16, FD_BF16 = 0, 1, 2, 3
 FD_VARIANT_PERIODIC, FD_VARIANT_WALLS, FD_VARIANT_PERIODIC_XY = 0, 1, 2
 FD_INIT_MU, FD_INIT_UY, FD_INIT_VELOCITY, FD_OUTLET_PRESSURE = 1, 2, 4, 8
 FD_ROUND_NEAREST, FD_ROUND_STOCHASTIC = 0, 1
+FD_BATCH_AUTO, FD_BATCH_STAGED, FD_BATCH_TILE = 0, 1, 2
 ROUNDING = {"nearest": FD_ROUND_NEAREST, "stochastic": FD_ROUND_STOCHASTIC}
 TERMS = {"large_F": 0, "feq": 1, "geq": 2, "F": 3, "G": 4}
 FIELDS = {"rho": 0, "npx": 1, "npy": 2, "np2": 3, "mu": 4, "mu_plain": 5, "ux": 6, "uy": 7, "p": 8, "mix_tau": 9, "psi": 10}
@@ -109,6 +110,8 @@ SIGNATURES = {
     "fd_diag_scratch_bytes": [],
     "fd_batch_create": [C.POINTER(fd_instance), _I, _S, _I, _I, C.POINTER(C.c_void_p)],
     "fd_batch_configure": [_VP, _I, _I],
+    "fd_batch_set_kernel": [_VP, _I],
+    "fd_batch_kernel": [_VP],
     "fd_batch_step": [_VP, _I, _I, _VP],
     "fd_batch_parity": [_VP],
     "fd_batch_member_status": [_VP, C.POINTER(C.c_uint32), _I],

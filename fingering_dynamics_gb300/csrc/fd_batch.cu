@@ -22,6 +22,7 @@ struct fd_batch {
   int ntiles = 0;  // tiles of the shape asked for (fd_batch_tiles)
   int nwork = 0;   // tiles of the table, whose strips may be shorter (fd_batch_plan.h)
   int grid = 0;
+  int kernel = FD_BATCH_AUTO;
   int2* d_cells = nullptr;  // (member, tile) of the tile kernel; ncells 0: the staged kernel
   int ncells = 0;
   cudaGraph_t graph = nullptr;
@@ -112,8 +113,8 @@ __global__ void __launch_bounds__(32 * TY, MINB)
 }
 
 // The table of the tile kernel, if the batch takes it: its live members are
-// few cells, and the strips are the default ones (another shape asks for the
-// staged kernel).
+// few cells, the strips are the default ones (another shape asks for the
+// staged kernel), and the caller has not asked for the staged kernel.
 int prepare_cells(fd_batch* b, const std::vector<unsigned>& flagged) {
   cudaFree(b->d_cells);
   b->d_cells = nullptr;
@@ -125,7 +126,9 @@ int prepare_cells(fd_batch* b, const std::vector<unsigned>& flagged) {
     live += (long long)b->inst[i].prm.H * b->inst[i].prm.W;
     lowest = std::min(lowest, b->inst[i].prm.H);
   }
-  if (live == 0 || lowest < 3 || live > tile_batch_cells(b->st.dtype) || b->rows != 32 || b->band != 128) return FD_OK;
+  if (b->kernel == FD_BATCH_STAGED || live == 0 || lowest < 3 || live > tile_batch_cells(b->st.dtype) || b->rows != 32 ||
+      b->band != 128)
+    return FD_OK;
   std::vector<int2> cells;
   for (int i = 0; i < b->n; ++i) {
     if (flagged[(size_t)i] != 0u) continue;
@@ -342,6 +345,16 @@ int fd_batch_configure(fd_batch* b, int rows_per_strip, int band_width) {
   b->rows = rows_per_strip;
   return prepare_any(b);
 }
+
+int fd_batch_set_kernel(fd_batch* b, int kernel) {
+  FD_REQUIRE(b != nullptr, FD_ERR_ARG, "fd_batch_set_kernel: NULL batch");
+  FD_REQUIRE(kernel == FD_BATCH_AUTO || kernel == FD_BATCH_STAGED, FD_ERR_ARG, "fd_batch_set_kernel: kernel %d", kernel);
+  drop_graph(b);
+  b->kernel = kernel;
+  return prepare_any(b);
+}
+
+int fd_batch_kernel(const fd_batch* b) { return !b ? -1 : (b->ncells > 0 ? FD_BATCH_TILE : FD_BATCH_STAGED); }
 
 int fd_batch_step(fd_batch* b, int nsteps, int use_graph, void* stream) {
   FD_REQUIRE(b != nullptr && nsteps >= 0, FD_ERR_ARG, "fd_batch_step: bad arguments");

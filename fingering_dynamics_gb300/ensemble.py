@@ -3,8 +3,9 @@
 Each member is a :class:`~fingering_dynamics_gb300.lattice.Lattice` in fused
 mode with packed storage; :class:`Ensemble` hands their buffers to the C
 batch (``fd_batch_*``), which advances every member one iteration per
-persistent launch over a tile table and replays the iteration loop from a CUDA
-graph.  :meth:`Ensemble.autotune` picks the tile shape (band width and rows
+launch: a persistent one over a tile table, the iteration loop replayed from a CUDA
+graph, or for a batch of few cells one of a thread per cell.
+:meth:`Ensemble.autotune` picks the tile shape (band width and rows
 per strip) by timing the candidates on the ensemble itself.
 """
 from __future__ import annotations
@@ -182,6 +183,18 @@ class Ensemble:
         L.call("fd_batch_configure", self._batch, int(rows_per_strip), int(band_width))
         self.config = (int(band_width), int(rows_per_strip))
 
+    @property
+    def kernel(self) -> str:
+        """The kernel that steps the batch: "staged" or "tile" (one thread per cell)."""
+        return "tile" if L.lib().fd_batch_kernel(self._batch) == L.FD_BATCH_TILE else "staged"
+
+    def use_kernel(self, kernel: str):
+        """"auto" (as built: the tile kernel for a batch of few cells in the default
+        shape) or "staged" (in every shape).  The results are the same bits."""
+        if kernel not in ("auto", "staged"):
+            raise ValueError("kernel must be 'auto' or 'staged'")
+        L.call("fd_batch_set_kernel", self._batch, L.FD_BATCH_STAGED if kernel == "staged" else L.FD_BATCH_AUTO)
+
     def step(self, n: int, use_graph: bool = True):
         """Advance every member n iterations."""
         if n <= 0:
@@ -244,7 +257,9 @@ class Ensemble:
     def autotune(self, candidates=None, steps: int = 20) -> dict:
         """Time every (band width, rows per strip) candidate on this ensemble
         and keep the fastest; returns {candidate: MLUPS}.  Default candidates:
-        a fixed set plus the shapes that fill whole rounds of the grid."""
+        a fixed set plus the shapes that fill whole rounds of the grid.  The entry
+        (128, 32) of a batch of few cells is the tile kernel's, unless
+        use_kernel("staged") was called before."""
         if candidates is None:
             candidates = sorted(set(DEFAULT_CANDIDATES) | set(self.wave_candidates()))
         res = {}

@@ -361,11 +361,14 @@ typedef struct fd_instance {
 typedef struct fd_batch fd_batch;
 
 /* Build a batch over n members sharing one packed storage type (unscaled).
- * Every iteration is one persistent launch of the staged kernel over a table
+ * Every iteration is one launch.  The staged kernel's is persistent, over a table
  * of (member, band, strip) tiles: bands of band_width cells (64, 128, 256) and
  * strips of at most rows_per_strip rows (a member's strips are of equal
  * height within one row; they are cut shorter where that fills the persistent
- * grid's rounds better).  Allocates the (small) device tables. */
+ * grid's rounds better).  In the shape band_width 128, rows_per_strip 32 a batch of
+ * few cells (4 million in FP32, 1.5 million in 16 bits) runs the kernel of one
+ * thread per cell, unless fd_batch_set_kernel asks for the staged one; the results
+ * are the same bits.  Allocates the (small) device tables. */
 int fd_batch_create(const fd_instance* inst, int n, const fd_storage* st, int rows_per_strip, int band_width,
                     fd_batch** out);
 
@@ -375,9 +378,18 @@ int fd_batch_create(const fd_instance* inst, int n, const fd_storage* st, int ro
  * grid; a member whose flag was cleared is taken back by the next call. */
 int fd_batch_configure(fd_batch* b, int rows_per_strip, int band_width);
 
+/* Which kernel steps the batch: FD_BATCH_AUTO chooses as fd_batch_create says,
+ * FD_BATCH_STAGED is the staged kernel in every shape, also fd_batch_configure's
+ * later ones (drops a captured graph and builds the tables as that does).
+ * fd_batch_kernel returns the one that runs, FD_BATCH_STAGED or FD_BATCH_TILE. */
+enum { FD_BATCH_AUTO = 0, FD_BATCH_STAGED = 1, FD_BATCH_TILE = 2 };
+int fd_batch_set_kernel(fd_batch* b, int kernel);
+int fd_batch_kernel(const fd_batch* b);
+
 /* Advance every member nsteps iterations on `stream`.  use_graph != 0 replays
  * a captured two-iteration CUDA graph (needs a non-default stream; the graph
- * is captured on first use). */
+ * is captured on first use); the kernel of one thread per cell is launched
+ * programmatically in either case. */
 int fd_batch_step(fd_batch* b, int nsteps, int use_graph, void* stream);
 
 /* 0 if the members' states are in pop_a / side_a, 1 if in pop_b / side_b. */
@@ -393,11 +405,12 @@ int fd_batch_parity(const fd_batch* b);
  * Returns FD_ERR_NONFINITE if any member is flagged, FD_OK otherwise. */
 int fd_batch_member_status(fd_batch* b, uint32_t* out, int clear);
 
-/* Number of tiles per iteration in strips as tall as rows_per_strip allows. */
+/* Number of the staged kernel's tiles per iteration in strips as tall as
+ * rows_per_strip allows. */
 int fd_batch_tiles(const fd_batch* b);
 
-/* CTAs of the persistent launch (resident CTAs per SM x SMs, at most the tile
- * count).  The CTAs take tiles from a counter, tallest strips first; a tile
+/* CTAs of the staged kernel's persistent launch (resident CTAs per SM x SMs, at most
+ * the tile count), whichever kernel runs.  The CTAs take tiles from a counter, tallest strips first; a tile
  * count just under a whole number of rounds of the grid avoids a last round in
  * which a few CTAs run while the rest wait. */
 int fd_batch_grid(const fd_batch* b);
