@@ -22,6 +22,7 @@ struct fd_batch {
   int ntiles = 0;  // tiles of the shape asked for (fd_batch_tiles)
   int nwork = 0;   // tiles of the table, whose strips may be shorter (fd_batch_plan.h)
   int grid = 0;
+  int sms = 1;
   int kernel = FD_BATCH_AUTO;
   int2* d_cells = nullptr;  // (member, tile) of the tile kernel; ncells 0: the staged kernel
   int ncells = 0;
@@ -75,7 +76,7 @@ DevArgs<SF> instance_args(const fd_instance& in, const fd_storage& st, int rows,
 // 22.6, 8 31.9 / 35.3, 12 50.4 / 50.4, 32 125 / 116.
 constexpr long long tile_batch_cells(int dtype) { return dtype == FD_F32 ? 4000000 : 1500000; }
 
-constexpr int kTileBatchFew = 2432;  // tiles: two rounds of 8 CTAs on each of 152 SMs
+constexpr int kTileBatchFew = 16;  // tiles per SM: two rounds of 8 CTAs
 
 // The tile kernel over a batch: a CTA copies its member's arguments to shared
 // memory while the previous iteration drains.
@@ -151,7 +152,7 @@ void launch_cells(const fd_batch* b, int parity, bool early, cudaStream_t st) {
   };
   // registers for 8 or 9 CTAs per SM (launch_tile); FP32, lattices of 256 x 512: one 6.7 / 7.3 us, four 18.4 /
   // 17.4, eight 39.5 / 37.8, 24 109 / 103; 10 is slower than 9 (40.4 for eight)
-  if (b->ncells <= kTileBatchFew) go(k_tile_step_batch<SF, STOCH, FD_TILE_TY, 8>);
+  if (b->ncells <= kTileBatchFew * b->sms) go(k_tile_step_batch<SF, STOCH, FD_TILE_TY, 8>);
   else go(k_tile_step_batch<SF, STOCH, FD_TILE_TY, 9>);
 }
 
@@ -161,11 +162,10 @@ int prepare(fd_batch* b) {
   auto kern = k_fused_tma_batch<SF, NT, tma_ring_depth<SF>(), false, STOCH>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, M::ALLOC) != cudaSuccess)
     return check_launch("fd_batch: shared-memory attribute");
-  int per_sm = 1, dev = 0, sms = 1;
+  int per_sm = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, M::ALLOC);
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  b->grid = per_sm * sms;
+  b->sms = sm_count();
+  b->grid = per_sm * b->sms;
   std::vector<BatchInst<SF>> hi(b->n);
   BatchShape shape;
   b->ntiles = 0;

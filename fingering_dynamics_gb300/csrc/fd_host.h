@@ -42,6 +42,14 @@ inline int check_params(const fd_params* p) {
   return FD_OK;
 }
 
+// SMs of the current device
+inline int sm_count() {
+  int dev = 0, sms = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 // Raise a kernel's dynamic shared-memory limit to `bytes` once per device

@@ -577,12 +577,6 @@ int flat_n(const CvCall& c) {
   return launch_rows<16, 1, CH, true>(c, bw, rows);
 }
 
-void set_sms(CvCall& c) {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&c.sms, cudaDevAttrMultiProcessorCount, dev);
-}
-
 int conv_rows(const void* x, int N, int H, int W, int Cin, const void* w, const float* bias, int Cout, int act, void* z,
               void* y, void* stream, const char* what) {
   FD_REQUIRE(x && w && (z || y) && N > 0 && H > 0 && W > 0, FD_ERR_ARG, "%s: bad arguments", what);
@@ -591,8 +585,8 @@ int conv_rows(const void* x, int N, int H, int W, int Cin, const void* w, const 
   FD_REQUIRE(act == SG_ACT_NONE || act == SG_ACT_GELU, FD_ERR_ARG, "%s: activation %d", what, act);
   FD_REQUIRE(((uintptr_t)x | (uintptr_t)w | (uintptr_t)z | (uintptr_t)y) % 16 == 0, FD_ERR_ARG,
              "%s: tensors must be 16-byte aligned", what);
-  CvCall c{(const bf16*)x, N, H, W, Cin, (const bf16*)w, bias, Cout, act, (bf16*)z, (bf16*)y, fd::as_stream(stream), 1};
-  set_sms(c);
+  CvCall c{(const bf16*)x, N, H, W, Cin, (const bf16*)w, bias, Cout, act, (bf16*)z, (bf16*)y, fd::as_stream(stream),
+           fd::sm_count()};
   return Cin % 32 == 0 ? rows_n<32>(c) : rows_n<16>(c);
 }
 
@@ -603,8 +597,7 @@ int conv_error_word(unsigned* out, bool clear) { return tc_error_word(out, clear
 // sg_conv3x3_tc on widths that are not a multiple of 128 (arguments checked by the caller).
 int conv_narrow(const void* x, int N, int H, int W, int Cin, const void* w, const float* bias, int Cout, int act, void* z,
                 void* y, cudaStream_t s) {
-  CvCall c{(const bf16*)x, N, H, W, Cin, (const bf16*)w, bias, Cout, act, (bf16*)z, (bf16*)y, s, 1};
-  set_sms(c);
+  CvCall c{(const bf16*)x, N, H, W, Cin, (const bf16*)w, bias, Cout, act, (bf16*)z, (bf16*)y, s, fd::sm_count()};
   if (Cin % 64 == 0) return narrow_n<64>(c);
   return Cin % 32 == 0 ? flat_n<32>(c) : flat_n<16>(c);
 }
