@@ -254,6 +254,15 @@ struct ExactMacro {
   bool ok;  // every value in range
 };
 
+// The stored fields of a cell, for exact_collide (which checks the others): the
+// ranges of exact_macros.
+FD_CELL ExactMacro exact_stored(double rho, double ux, double uy, double p, double mu, double tau, double psi, double gx,
+                                double gy) {
+  return ExactMacro{rho, ux, uy, p, mu, tau, psi, gx, gy,
+                    cell_in_range<100>(rho) && cell_in_range<400>(psi) && cell_in_range<800>(p) && cell_in_range<800>(gx) &&
+                        cell_in_range<800>(gy)};
+}
+
 FD_CELL ExactMacro exact_macros(const ExactConst& k, double rho, double psi, const ExactStencil& st,
                                 const double (&f)[9]) {
   ExactMacro m;

@@ -229,9 +229,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_collide_f64(Shape s, Coef<double>
   double f[9], fn[9], gn[9];
 #pragma unroll
   for (int i = 0; i < 9; ++i) f[i] = F.f[i * s.P + q];
-  const ExactMacro em{m.rho, m.ux, m.uy, m.p, m.mu, m.tau_mix, m.psi, m.gx, m.gy,
-                      cell_in_range<100>(m.rho) && cell_in_range<100>(m.psi) && cell_in_range<100>(m.p) &&
-                          cell_in_range<800>(m.gx) && cell_in_range<800>(m.gy)};
+  const ExactMacro em = exact_stored(m.rho, m.ux, m.uy, m.p, m.mu, m.tau_mix, m.psi, m.gx, m.gy);
   auto load_g = [&](int i) { return F.g[i * s.P + q]; };
   auto store = [&](int i, double a, double bb) {
     fn[i] = a;
