@@ -31,11 +31,13 @@
 // The thin layers are bound by the MMAs, which take some 55 clocks however few
 // columns they have (32 -> 16: 114 us, its bytes 59), with GELU also by the
 // epilogue's tanhf; the wide ones by the tensor pipe.
+#include "sg_conv_plan.h"
 #include "sg_tc.cuh"
 
 namespace sg {
 namespace {
 
+static_assert(kConvPixels == kTcBM, "operand rows");
 constexpr int kCvEpiWarps = 8;
 constexpr int kCvThreads = 32 * (kCvEpiWarps + 2);
 
@@ -479,11 +481,9 @@ int launch_rows(const CvCall& c, int bw = kTcBM, int rows = R) {
     return fd::check_launch("sg_conv3x3_tma: shared-memory attribute");
   constexpr int kRoom = 227 * 1024 - C::TAIL;
   CvShape sh{c.N, c.H, c.W, c.Cin, c.Cout, c.act, c.Cin / CH, 0, 0, bw, rows};
-  // the weights stay where two stages of the ring fit beside them (or all the chunks there are)
-  const int need = sh.nk < 2 ? 1 : 2;
-  sh.resident = sh.nk * C::B_BYTES + need * C::A_BYTES <= kRoom;
-  const int stage = C::A_BYTES + (sh.resident ? 0 : C::B_BYTES);
-  sh.S = std::min<int>(C::S_MAX, (kRoom - (sh.resident ? sh.nk * C::B_BYTES : 0)) / stage);
+  const ConvRing ring = conv_ring(sh.nk, C::A_BYTES, C::B_BYTES, kRoom, C::S_MAX);
+  sh.resident = ring.resident;
+  sh.S = ring.stages;
   if (sh.S < 1) {
     fd::set_error("sg_conv3x3_tma: no stage fits");
     return FD_ERR_SHAPE;
@@ -518,23 +518,6 @@ int rows_n(const CvCall& c) {
   if (c.Cout % 64 == 0) return rows_r<64, CH>(c);
   if (c.Cout % 32 == 0) return rows_r<32, CH>(c);
   return rows_r<16, CH>(c);
-}
-
-// The tile of a width: W in equal parts (the last may be shorter), as many rows as
-// fit 128 operand rows at a pitch of the part plus `gap`; the parts that give the
-// fewest tiles.
-inline void tile_box(int H, int W, int gap, int& bw, int& rows) {
-  long long best = 0;
-  const int least = (W + kTcBM - 1) / kTcBM;
-  for (int k = least; k <= std::max(least, 16) && k <= W; ++k) {
-    const int w = (W + k - 1) / k, r = std::min((kTcBM + gap) / (w + gap), 254);
-    const long long tiles = (long long)((W + w - 1) / w) * ((H + r - 1) / r);
-    if (best == 0 || tiles < best) {
-      best = tiles;
-      bw = w;
-      rows = r;
-    }
-  }
 }
 
 template <int BN, int BK>
