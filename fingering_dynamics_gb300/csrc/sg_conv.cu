@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_rows(const __grid_con
     const uint64_t a0 = smem_desc_sw<C::ROW>(smem_u32(smem), 16, 8 * C::ROW);
     const uint64_t w0 = smem_desc_sw<C::ROW>(smem_u32(sh.resident ? wres : smem + C::A_BYTES), 16, 8 * C::ROW);
     bool ok = mine > 0 && (!sh.resident || mbar_wait_ok(wfull, 0u, true));
-    int c = 0;
+    int c = 0, tiles = 0;  // chunks and whole tiles issued
     for (int j = 0; j < mine && ok; ++j) {
       const int b = j & 1;
       if (j >= 2) ok = mbar_wait_ok(&acce[b], (unsigned)((j - 2) >> 1) & 1u, true);  // tile j - 2 has been read
@@ -240,12 +240,15 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_rows(const __grid_con
           tc_commit(&empty[st]);
           if (kc == nk - 1) tc_commit(&accf[b]);  // tile j's accumulators are complete
         }
+        if (kc == nk - 1) tiles = j + 1;
         __syncwarp();
       }
     }
-    // the MMAs issued have completed before tensor and shared memory are given up
+    // the MMAs issued have completed and their commits have arrived before tensor and shared memory are given up
     for (int i = 0; i < S && i < c; ++i)
       mbar_wait_ok(&empty[i], (unsigned)((c - 1 - ((c - 1 - i) % S)) / S) & 1u, false);
+    if (!ok)  // else the epilogue warps wait for every tile
+      for (int j = tiles > 2 ? tiles - 2 : 0; j < tiles; ++j) mbar_wait_ok(&accf[j & 1], (unsigned)(j >> 1) & 1u, false);
   } else {
     // epilogue: warp w reads TMEM lanes 32 q .. 32 q + 31 (pixels x0 + 32 q + lane of each row, q = w % 4) of every
     // second group of 16 columns (w / 4)
@@ -380,7 +383,7 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_narrow(const __grid_c
     const uint64_t a0 = smem_desc_sw<C::ROW>(smem_u32(smem), 16, 8 * C::ROW);
     const uint64_t w0 = smem_desc_sw<C::ROW>(smem_u32(smem + C::A_BYTES), 16, 8 * C::ROW);
     bool ok = true;
-    int c = 0;
+    int c = 0, tiles = 0;
     for (int j = 0; j < mine && ok; ++j) {
       const int b = j & 1;
       if (j >= 2) ok = mbar_wait_ok(&acce[b], (unsigned)((j - 2) >> 1) & 1u, true);
@@ -398,11 +401,14 @@ __global__ void __launch_bounds__(kCvThreads, 1) k_conv3x3_narrow(const __grid_c
           tc_commit(&empty[st]);
           if (k == nst - 1) tc_commit(&accf[b]);
         }
+        if (k == nst - 1) tiles = j + 1;
         __syncwarp();
       }
     }
     for (int i = 0; i < S && i < c; ++i)
       mbar_wait_ok(&empty[i], (unsigned)((c - 1 - ((c - 1 - i) % S)) / S) & 1u, false);
+    if (!ok)  // else the epilogue warps wait for every tile
+      for (int j = tiles > 2 ? tiles - 2 : 0; j < tiles; ++j) mbar_wait_ok(&accf[j & 1], (unsigned)(j >> 1) & 1u, false);
   } else {
     const int q = warp & 3, h = warp >> 2;
     const bool wide = ((uintptr_t)z | (uintptr_t)y) % 32 == 0;
