@@ -14,7 +14,9 @@
 #pragma once
 
 #include <algorithm>
+#include <functional>
 #include <queue>
+#include <utility>
 #include <vector>
 
 namespace fd {
@@ -61,8 +63,9 @@ inline std::vector<int> plan_strips(const BatchShape& s, int rows, int grid) {
     base[i] = (s.height[i] + rows - 1) / rows;
     tiles += (long long)base[i] * s.bands[i];
   }
+  if (grid < 1 || tiles == 0) return base;
   const long long first = (tiles + grid - 1) / grid;
-  if (grid < 1 || tiles == 0 || first > kMaxPlanRounds) return base;
+  if (first > kMaxPlanRounds) return base;
   std::vector<int> best = base;
   long long best_end = batch_makespan(s, base, grid);
   for (long long rounds = first; rounds < first + 4; ++rounds) {
