@@ -735,7 +735,7 @@ def main():
     ap.add_argument("--train-steps", type=int, default=1000, help="surrogate: timed AdamW steps")
     ap.add_argument("--batch", type=int, default=32, help="surrogate: training batch")
     ap.add_argument("--conv", default="auto", choices=["auto", "mma", "tcgen05", "tma", "tma_ws"],
-                    help="surrogate: forward / data-gradient convolution kernel (auto: the faster per shape)")
+                    help="surrogate: forward / data-gradient convolution kernel (auto: by the image's width)")
     ap.add_argument("--save-net", default=None, help="surrogate: write the trained network's weights (.npz) here")
     ap.add_argument("--load-net", default=None,
                     help="accelerated: the trained network's weights (.npz, as written by --save-net)")

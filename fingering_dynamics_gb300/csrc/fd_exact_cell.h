@@ -191,13 +191,12 @@ FD_CELL ExactStencil exact_stencil(const ExactConst& k, double C, double E, doub
 // How many of a cell's products are formed in integer arithmetic (0: none, 58:
 // all), in the order of their numbers below.  An integer product is about 40
 // instructions, which the four schedulers issue in 10 clocks beside the FP64
-// pipe, against the pipe's 16.  Ten iterations of 1024 x 2048: 11.6 ms with
-// none, 10.7 with those of cell_relax (7), 10.2 with all; 25 of 400 x 400:
-// 3.16, 2.96, 2.57 ms.
+// pipe, against the pipe's 16.  Ten iterations of 1024 x 2048: 11.7 ms with
+// none, 10.0 with those of cell_relax (7), 8.4 with all; 25 of 400 x 400:
+// 3.33, 2.85, 2.45 ms.
 #ifndef FD_EXACT_INT_PRODUCTS
 #define FD_EXACT_INT_PRODUCTS 58
 #endif
-
 
 // The products outside cell_relax are calls of one function: 33 copies of it took
 // more instructions than the caches hold (2.8 stalls on a missing instruction per

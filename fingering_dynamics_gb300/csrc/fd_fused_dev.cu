@@ -60,7 +60,7 @@ int tile(const fd_params& p, const fd_storage& st, const DevCoef& c, const uint1
 }
 
 // Cells up to which the tile kernel is taken where the staged kernel could run.
-// Per step, tile / staged, us: FP32 64 x 128 3.4 / 30, 512 x 512 8.6 / 29, 1024 x
+// Per step, tile / staged, us: FP32 64 x 128 3.4 / 27.6, 512 x 512 8.3 / 28.7, 1024 x
 // 2048 64 / 72, 2048 x 2048 123 / 118; FP16 512 x 1024 13.0 / 26.9, 1024 x 1024
 // 24.4 / 34.0, 1024 x 2048 50.5 / 50.  The staged kernel's time does not fall with
 // the lattice (a strip is at least 16 rows, a microsecond or more each).

@@ -204,7 +204,8 @@ __global__ void k_collide(Shape s, Coef<T> c, const uint16_t* __restrict__ mask,
 // The same in FP64, which is bound by the FP64 pipe: a block's fluid cells are
 // taken by full warps, in the arithmetic of fd_exact_cell.h (the same bits).
 // Ten iterations of 1024 x 2048 at porosity 0.7, which run this kernel and
-// k_macros_f64 once each: 10.2 -> 9.1 ms (k_collide<double> alone took 1.3).
+// k_macros_f64 once each, took 10.2 ms before and 9.1 after (k_collide<double> alone
+// took 1.3); with what the fused step gained since they take 8.4.
 __global__ void __launch_bounds__(kBlock, 2) k_collide_f64(Shape s, Coef<double> c, ExactConst k,
                                                            const uint16_t* __restrict__ mask, Fields<double> F) {
   __shared__ uint16_t list[kBlock];

@@ -12,7 +12,7 @@
 // previous step drains, load their masks, and wait for it before they touch
 // the populations.
 //
-// Measured, us per step (the kernel before -> this one): FP32 64 x 128 26 -> 3.5
+// Measured, us per step (the kernel before -> this one): FP32 64 x 128 27.6 -> 3.4
 // and 380 x 380 15.7 -> 6.2, BF16 1021 x 1500 82 -> 41.4 (there it is bound by
 // instruction issue; 47.5 with 64-bit addresses).  Tiles of 4 rows: 8 rows lose 7-11% on FP32 from 1024 x 1024
 // up and gain on single sizes below (256 x 512 6.2 vs 7.0).

@@ -1,5 +1,6 @@
-// 3x3 convolution (forward and data gradient) of the learned surrogate at widths
-// that are multiples of 128, on tcgen05 (sg_conv3x3_tma, sg_conv3x3_tma_ws).
+// 3x3 convolution (forward and data gradient) of the learned surrogate on tcgen05: at
+// widths that are multiples of 128 (sg_conv3x3_tma, sg_conv3x3_tma_ws), described here,
+// and at the others (sg_conv3x3_tc): this kernel's FLAT form and k_conv3x3_narrow below.
 //
 // Implicit GEMM, M = pixels, N = output channels, K = 9 x input channels.  A
 // persistent CTA walks tiles of R image rows x 128 pixels x BN output channels
@@ -19,8 +20,8 @@
 // FP32 sums run in one order whatever the chunk and tile.
 //
 // In a list of operations (sg_run) the barriers, the tensor memory and the tensor
-// maps are set up while the previous kernel drains: a prediction of one image of
-// 256 x 512 (23 kernels of 4 to 20 us) 256 -> 210 us.
+// maps are set up while the previous kernel drains: it took a prediction of one image
+// of 256 x 512 (23 kernels of 4 to 20 us) from 256 to 210 us (195 now).
 //
 // What it replaced: boxes of 8 channels (16-byte pieces, four to eight times as
 // many), the weights streamed anew for every tile, two descriptors built per MMA

@@ -774,7 +774,6 @@ __global__ void k_masked_mse(const bf16* __restrict__ x, const bf16* __restrict_
   }
 }
 
-// y = x with its first three channels replaced by bf16(x + out)
 // A frame of the network (16 channels: psi, u_x / U, u_y / U, solid, zeros) from
 // the fields, one cell a thread, one 32-byte store; as tensor operations it was ten
 // passes of a few microseconds each.
@@ -791,6 +790,7 @@ __global__ void k_frame(const T* __restrict__ psi, const T* __restrict__ ux, con
                : "memory");
 }
 
+// y = x with its first three channels replaced by bf16(x + out)
 __global__ void k_add_prediction(const bf16* __restrict__ x, const bf16* __restrict__ out, size_t P, int C,
                                  bf16* __restrict__ y) {
   const int cg = C / 8;
@@ -830,7 +830,6 @@ __global__ void k_adamw(float* __restrict__ w, bf16* __restrict__ w16, const flo
 struct AdamwList {
   sg_adamw_item item[SG_ADAMW_MAX];
   unsigned first[SG_ADAMW_MAX + 1];  // first block of each tensor
-  int n;
 };
 __global__ void __launch_bounds__(kEw) k_adamw_list(const __grid_constant__ AdamwList L, float lr, float b1, float b2,
                                                     float eps, float c1, float c2) {
@@ -1016,7 +1015,6 @@ int sg_adamw_list(const sg_adamw_item* items, int count, float lr, float beta1, 
                   void* stream) {
   FD_REQUIRE(items && count > 0 && count <= SG_ADAMW_MAX && step >= 1, FD_ERR_ARG, "sg_adamw_list: bad arguments");
   AdamwList L;
-  L.n = count;
   L.first[0] = 0;
   for (int i = 0; i < count; ++i) {
     const sg_adamw_item& a = items[i];

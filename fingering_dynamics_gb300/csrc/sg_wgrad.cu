@@ -26,8 +26,8 @@ namespace {
 // chunk (its descriptors are a base and constants, in uniform registers: with
 // descriptors built per MMA by one thread the issue was the bound).  FP32 partials
 // go to partial[split][co][tap][ci] and are added in a fixed order, and the split
-// into pixel ranges depends on the shape alone, so the result does not depend on
-// scheduling.
+// into pixel ranges depends on the shape, the device's SM count and the room that
+// `partial` has, so on one device the result does not depend on scheduling.
 // Measured at batch 32, us, against boxes of 8 channels with output or input
 // channels alone on the rows (and against the warp-level kernel): 32 -> 32 (256 x
 // 512) 133 (1048; 678), 96 -> 32 336 (1232; 1988), 64 -> 64 (128 x 256) 84 (332;
@@ -234,11 +234,10 @@ int launch_wgrad_tc(const bf16* x, const bf16* dz, int N, int H, int W, int Cin,
   const long long nchunks = (long long)N * H * (W / kTcBM);
   const size_t n = (size_t)Cout * 9 * Cin;
   if (splits <= 0) {
-    // The pixel ranges fix the order of every sum, so their count is a function of the shape: about two CTAs per SM
-    // when 128 channels of the larger count and a block of the other make a tile, within the chunks and the buffer.
-    int dev = 0, sms = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // The pixel ranges fix the order of every sum, so their count is a function of the shape and the device: about two
+    // CTAs per SM when 128 channels of the larger count and a block of the other make a tile.  Below, it is cut to the
+    // chunks and to what the buffer holds (sg_wgrad_partial_floats holds it on 152 SMs).
+    const int sms = fd::sm_count();
     const int big = Cin > Cout ? Cin : Cout, small = Cin > Cout ? Cout : Cin;
     const int blk = small % 128 == 0 ? 128 : (small % 64 == 0 ? 64 : (small % 32 == 0 ? 32 : 16));
     const long long per = (long long)((big + 127) / 128) * (small / blk) * 3;
